@@ -189,6 +189,115 @@ __device__ __forceinline__ float dist_rec_val(const TriRec& r, float dx, float d
     return dist_rec_t<false>(r, pa_n(r, dx, dy, dz), nullptr);
 }
 
+// The triangle's nearest point to a point (pa_n of it, the triangle's centroid at e from
+// the same origin as the offsets): any point of the triangle to within 40u (d + 4e + 4r),
+// d the distance; it need not be the nearest to the last bit.
+__device__ __forceinline__ void nearest_point(const TriRec& r, const PaN& p, float ex, float ey,
+                                              float ez, float& qx, float& qy, float& qz) {
+    const float pu = dot3f(p.x, p.y, p.z, r.uu), pv = dot3f(p.x, p.y, p.z, r.vv);
+    const float qu1 = pu - r.bx, qu2 = pu - r.cx, qv2 = pv - r.cy;
+    const float t0 = __saturatef(pu * r.ib);
+    const float t1 = __saturatef(fmaf(qu1, r.e1x, pv * r.cy) * r.inv1);
+    const float t2 = __saturatef(-fmaf(qu2, r.cx, qv2 * r.cy) * r.inv2);
+    float cu = t0 * r.bx, cv = 0.f;
+    float d = fmaf(pu - cu, pu - cu, pv * pv);
+    const float u1 = fmaf(t1, r.e1x, r.bx), v1 = t1 * r.cy;
+    const float d1 = fmaf(pu - u1, pu - u1, (pv - v1) * (pv - v1));
+    if (d1 < d) { d = d1; cu = u1; cv = v1; }
+    const float u2 = fmaf(-t2, r.cx, r.cx), v2 = fmaf(-t2, r.cy, r.cy);
+    const float d2 = fmaf(pu - u2, pu - u2, (pv - v2) * (pv - v2));
+    if (d2 < d) { cu = u2; cv = v2; }
+    if (r.ok > 0.f && pv >= 0.f && fmaf(r.e1x, pv, -r.cy * qu1) >= 0.f &&
+        fmaf(r.cy, qu2, -r.cx * qv2) >= 0.f) {
+        cu = pu;
+        cv = pv;
+    }
+    qx = ex + r.o0[0] + fmaf(cu, r.uu[0], cv * r.vv[0]);
+    qy = ey + r.o0[1] + fmaf(cu, r.uu[1], cv * r.vv[1]);
+    qz = ez + r.o0[2] + fmaf(cu, r.uu[2], cv * r.vv[2]);
+}
+
+// sqrt to 2u (the pruning tests below carry wider margins).
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// ------------------------------------------------------------------ box tests
+// Which triangles can matter to some cell p of a box (half-widths hx, hy, hz and
+// half-diagonal r around the origin), given one point q of the surface: p is at most
+// b(p) = |p - q| + eps from the surface, so a triangle matters to p only when its lower
+// bound is <= b(p) (eps carries the FP32 distances' errors). A triangle with centroid c and
+// radius w lies in the ball of radius w around c and in its plane (unit normal n), that
+// is in a disc, whose distance from p is (n . (p - c))^2 + max(0, lat - w)^2 squared, lat
+// the in-plane distance of p from c. That is <= b^2 exactly when n . (p - c) <= b and
+//     |p - c|^2 - b^2 <= w^2 + 2 w s,    s^2 = b^2 - (n . (p - c))^2,
+// and the two quadratics leave |c|^2 - |q|^2 - 2 p . (c - q) on the left, linear in p: its
+// minimum over the box is exact, where a test against the box's sphere gives away twice
+// its radius along every direction. s^2 is bounded over the box by its value and gradient
+// at the origin (its second-order part |p|^2 - (n . p)^2 is at most r^2). n = 0 (a
+// degenerate triangle) leaves the ball test. Rounding: every term is formed from c, q, n and
+// the box with relative errors that sum to less than 40u (|c|^2 + |q|^2 + r^2), the
+// normal's own error nerr to less than 6 nerr (|c|^2 + r^2); `mul` and `add` widen both
+// sides by more. A comparison with a NaN keeps the triangle.
+struct BoxTest {
+    float qx, qy, qz, q2;
+    float hx, hy, hz, r2;
+    float e2;   // 2 eps (|q| + r) + eps^2, rounded up
+    float qr;   // |q| + r + eps, rounded up (s <= qr without a plane)
+    float add;  // absolute margin
+};
+__device__ __forceinline__ BoxTest box_test(float qx, float qy, float qz, float hx, float hy,
+                                            float hz, float r, float eps, float pos) {
+    BoxTest b;
+    b.qx = qx; b.qy = qy; b.qz = qz;
+    b.hx = hx; b.hy = hy; b.hz = hz;
+    b.q2 = fmaf(qx, qx, fmaf(qy, qy, qz * qz));
+    b.r2 = r * r;
+    b.qr = (sqrtf(b.q2) + r + eps) * (1.f + 8.f * kU32);
+    b.e2 = eps * (2.f * b.qr + eps) * (1.f + 8.f * kU32);
+    // pos: absolute error of the positions beyond their own rounding
+    b.add = fmaf(64.f * kU32, b.q2 + b.r2, 8.f * pos * (b.qr + pos)) + 1e-36f;
+    return b;
+}
+// The test without the plane (s <= qr): false when no cell of the box can be concerned.
+__device__ __forceinline__ bool box_ball(const BoxTest& b, float cx, float cy, float cz, float w,
+                                         float pos) {
+    const float c2 = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
+    const float g = fmaf(b.hx, fabsf(cx - b.qx), fmaf(b.hy, fabsf(cy - b.qy), b.hz * fabsf(cz - b.qz)));
+    const float lin = fmaf(-2.f, g, c2 - b.q2);
+    const float m = fmaf(64.f * kU32, c2, fmaf(8.f * pos, w, b.add));
+    const float rhs = fmaf(w * (1.f + 32.f * kU32), fmaf(2.f, b.qr, w), b.e2) + m;
+    return !(lin > rhs);
+}
+// The test with the plane; n.w bounds the error of the unit normal n.
+__device__ __forceinline__ bool box_disc(const BoxTest& b, float cx, float cy, float cz, float w,
+                                         const float4& n) {
+    const float c2 = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
+    const float g = fmaf(b.hx, fabsf(cx - b.qx), fmaf(b.hy, fabsf(cy - b.qy), b.hz * fabsf(cz - b.qz)));
+    const float lin = fmaf(-2.f, g, c2 - b.q2);
+    const float m = fmaf(64.f * kU32 + 8.f * n.w, c2 + b.r2, fmaf(8.f * n.w, b.q2, b.add));
+    const float nc = fmaf(n.x, cx, fmaf(n.y, cy, n.z * cz));
+    const float gs = fmaf(b.hx, fabsf(fmaf(nc, n.x, -b.qx)),
+                          fmaf(b.hy, fabsf(fmaf(nc, n.y, -b.qy)), b.hz * fabsf(fmaf(nc, n.z, -b.qz))));
+    const float s2 = fmaf(2.f, gs, fmaf(-nc, nc, b.q2 + b.r2)) + (b.e2 + m);
+    const float s = sqrt_approx(fmaxf(s2, 0.f));
+    const float rhs = fmaf(w * (1.f + 32.f * kU32), fmaf(2.f, s, w), b.e2) + m;
+    return !(s2 < 0.f) && !(lin > rhs);
+}
+
+// One cell's test against a disc: d the cell's offset from the centroid (squared length
+// d2), pn its plane distance from the triangle, b its bound with the plane test's margin
+// (plane_reach), w the triangle's radius or more (reach_term: w (1 + 20u) + 17u r). The
+// offset's rounding moves d2 by at most 24u (b^2 + w^2) + 4u r (b + w), the right side's
+// own by 8u (b^2 + w^2); b^2 exceeds the cell's bound squared by 136u b (b + 4e + 4r), w^2
+// the radius squared by 40u w^2 + 34u w r.
+__device__ __forceinline__ bool cell_disc(float d2, float pn, float b, float w) {
+    const float s = sqrt_approx(fmaxf((b - fabsf(pn)) * (b + fabsf(pn)), 0.f));
+    return fabsf(pn) <= b && !(d2 > fmaf(w, fmaf(2.f, s, w), b * b) * (1.f + 16.f * kU32));
+}
+
 // ------------------------------------------------------------------ outputs
 struct Out {
     const uint8_t* occ;

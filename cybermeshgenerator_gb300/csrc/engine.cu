@@ -244,6 +244,7 @@ struct Batch::Impl {
     int* large_list = nullptr;
     unsigned* emax_bits = nullptr;
     float* bound = nullptr;
+    int* bound_tri = nullptr;  // the triangle that gave the bound
     int* cand_cnt = nullptr;
     int64_t* cand_off = nullptr;
     float* brick_emax = nullptr;
@@ -348,6 +349,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
             impl_->large_list = carve<int>(A, ntris_);
             impl_->emax_bits = carve<unsigned>(A, 3 * nseg);  // emax, scale, emax_all
             impl_->bound = carve<float>(A, nbrick_);
+            impl_->bound_tri = carve<int>(A, nbrick_);
             impl_->cand_cnt = carve<int>(A, nbrick_);
             impl_->cand_off = carve<int64_t>(A, nbrick_ + 1);
             impl_->brick_emax = carve<float>(A, nbrick_);
@@ -565,7 +567,7 @@ void Batch::run_impl(bool sizing) {
         launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.bin_list, dsegs_, nseg,
                         I.large_cnt + nseg, I.large_list, ss);
         launch_brick_walk(false, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
-                          I.bin_list, I.large_list, I.bound, I.cand_cnt, nullptr, nullptr, nullptr,
+                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, nullptr, nullptr, nullptr,
                           stats_, opts_.walk_warps, ss);
         exclusive_scan(I.cand_cnt, I.cand_off, nbrick_, tmp, ss);
     };
@@ -588,7 +590,7 @@ void Batch::run_impl(bool sizing) {
     };
     auto prep_tail = [&]() {
         launch_brick_walk(true, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
-                          I.bin_list, I.large_list, I.bound, I.cand_cnt, I.cand_off, I.cand,
+                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, I.cand_off, I.cand,
                           I.brick_emax, stats_, opts_.walk_warps, ss);
         if (opts_.brick == 16) launch_sub_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);
         else launch_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);

@@ -47,7 +47,7 @@ void launch_seg_finish(MeshSeg* segs, int nseg, const int64_t* large_off, const 
 void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
                        const int64_t* bin_off, const int* bin_list, const int* large_list,
-                       float* bound, int* cand_cnt, const int64_t* cand_off, int* cand,
+                       float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
                        float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st);
 // Warps per brick the walk uses: walk_warps when it is 1, 2 or 4, else by the brick
 // count (4 while 4-warp bricks fit about twice in the GPU, 2 up to twice that, then 1).

@@ -397,7 +397,7 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
              const float4* __restrict__ tlo, const float4* __restrict__ thi,
              const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
              const int* __restrict__ large_list, float* __restrict__ bound,
-             int* __restrict__ cand_cnt, const int64_t* __restrict__ cand_off,
+             int* __restrict__ bound_tri, int* __restrict__ cand_cnt, const int64_t* __restrict__ cand_off,
              int* __restrict__ cand, float* __restrict__ brick_emax,
              Stats* __restrict__ st) {
     constexpr int kWarps = kWalkThreads / 32;
@@ -451,9 +451,11 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
         g1 = static_cast<int>(static_cast<int64_t>(ng) * (sub + 1) / W);
     };
     float U;
+    int ut = INT_MAX;  // the binned triangle whose sphere gives the smallest bound
     if (!FILL) {
         // ---- upper bound on the distance from the brick centre to the surface
         U = FLT_MAX;
+        float ub = FLT_MAX;
         for (int64_t e = s.large_begin + 32 * sub + lane; e < s.large_end; e += 32 * W)
             U = fminf(U, large_upper(soup, large_list[e], s.g.corner, q.cx, q.cy, q.cz, tol));
         for (int r = 0; r <= rmax; ++r) {
@@ -476,7 +478,9 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
                         float4 ti = tinfo[t[j]];
                         float dx2 = ti.x - q.cx, dy2 = ti.y - q.cy, dz2 = ti.z - q.cz;
                         float d = sqrtf(dx2 * dx2 + dy2 * dy2 + dz2 * dz2) * (1.f + 4.f * kU32);
-                        U = fminf(U, d + ti.w + tol);
+                        const float v = d + ti.w + tol;
+                        U = fminf(U, v);
+                        if (v < ub) { ub = v; ut = t[j]; }
                     }
                 });
             }
@@ -486,15 +490,44 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
             }
         }
         U = brick_min(U);
-        if (sub == 0 && lane == 0) bound[gb] = U;
+        {
+            // the lowest index among the triangles at the smallest bound (exact in FP32)
+            const float m = brick_min(ub);
+            const int cand_t = ub == m ? ut : INT_MAX;
+            ut = __reduce_min_sync(0xffffffffu, cand_t);
+            if (W > 1) {
+                if (lane == 0) s_i[wid] = ut;
+                brick_sync();
+#pragma unroll
+                for (int w = 0; w < W; ++w) ut = min(ut, s_i[first + w]);
+                brick_sync();
+            }
+        }
+        if (sub == 0 && lane == 0) {
+            bound[gb] = U;
+            bound_tri[gb] = ut;
+        }
     } else {
         U = bound[gb];
+        ut = bound_tri[gb];
     }
     // ---- candidates: lower bound <= U + 2 r_B (+ margins). The relative margin (4e-5,
     // about 670 u) covers four stated FP32 errors 48u (d + 2e + 2r) beyond any cell's
     // distance (e at most two bricks here; larger triangles are always considered): the
     // exact FP64 path's near-ties and its band pass need them, the mixed path two
     const float lim = (U + 2.f * q.rb) * (1.f + 4e-5f) + 2.f * tol;
+    // ... and, around the centroid of the triangle that gave the bound (a point of the
+    // surface), the box test with the same margins: a brick's sphere gives away 2 r_B in
+    // every direction, most of the list of a brick far from the surface
+    const bool boxed = ut != INT_MAX;
+    BoxTest box;
+    if (boxed) {
+        const float4 ti = tinfo[ut];
+        const float h = static_cast<float>(s.g.h);
+        box = box_test(ti.x - q.cx, ti.y - q.cy, ti.z - q.cz, 0.5f * (q.x1 - q.x0 - 1) * h,
+                       0.5f * (q.y1 - q.y0 - 1) * h, 0.5f * (q.z1 - q.z0 - 1) * h, q.rb,
+                       fmaf(4e-5f, U + 2.f * q.rb, 4.f * tol), tol);
+    }
     const int64_t out = FILL ? cand_off[gb] : 0;
     const unsigned below = (1u << lane) - 1u;
     float bemax = 0.f;
@@ -520,6 +553,7 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
                         float dx2 = ti[j].x - q.cx, dy2 = ti[j].y - q.cy, dz2 = ti[j].z - q.cz;
                         float d = sqrtf(dx2 * dx2 + dy2 * dy2 + dz2 * dz2) * (1.f - 4.f * kU32);
                         take = d - ti[j].w <= lim;  // |v - c_t| - e_t >= d - r_B - e_t
+                        if (boxed) take = take && box_ball(box, dx2, dy2, dz2, ti[j].w, tol);
                         et = ti[j].w;
                     }
                     f(take, t[j], et);
@@ -1109,7 +1143,7 @@ int brick_walk_warps(int64_t nbricks, int walk_warps) {
 void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
                        const int64_t* bin_off, const int* bin_list, const int* large_list,
-                       float* bound, int* cand_cnt, const int64_t* cand_off, int* cand,
+                       float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
                        float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st) {
     if (nbricks == 0) return;
     const int W = brick_walk_warps(nbricks, walk_warps);
@@ -1119,7 +1153,7 @@ void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks
         constexpr int WW = decltype(w_tag)::value;
         k_brick_walk<F, WW><<<grid, kWalkThreads, 0, st>>>(segs, nseg, nbricks, soup, tinfo, tlo, thi,
                                                            bin_off, bin_list, large_list, bound,
-                                                           cand_cnt, cand_off, cand, brick_emax, stats);
+                                                           bound_tri, cand_cnt, cand_off, cand, brick_emax, stats);
     };
     using T = std::true_type;
     using Fa = std::false_type;
