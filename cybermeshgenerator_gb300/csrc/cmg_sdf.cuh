@@ -25,6 +25,69 @@ __device__ __forceinline__ double d2r(const d3& p, double qx, double qy, double 
     return dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
 }
 
+// Whether a double is <= 0 or >= 0 by its bits: the FP64 pipe's comparisons cost as much as
+// its additions. Not for NaN.
+__device__ __forceinline__ bool le0(double v) { return __double_as_longlong(v) <= 0; }
+__device__ __forceinline__ bool ge0(double v) {
+    const long long b = __double_as_longlong(v);
+    return b >= 0 || b == LLONG_MIN;
+}
+
+// The same values and regions as ericson() below in one path for a warp whose lanes lie in
+// different regions: all six dot products, the region by the reference's tests in their
+// order, then one division and one closest point with the region's operands selected (a
+// term that a region does not have is skipped, not added as zero times something).
+// ericson()'s seven exits, taken one after the other by a mixed warp, cost about twice the
+// FP64 instructions, and this part issues one FP64 warp instruction per 16 cycles and SM.
+__device__ __forceinline__ double ericson_sel(const d3& p, const d3& a, const d3& b, const d3& c,
+                                              int* region) {
+    const double abx = dsub(b.x, a.x), aby = dsub(b.y, a.y), abz = dsub(b.z, a.z);
+    const double acx = dsub(c.x, a.x), acy = dsub(c.y, a.y), acz = dsub(c.z, a.z);
+    const double apx = dsub(p.x, a.x), apy = dsub(p.y, a.y), apz = dsub(p.z, a.z);
+    const double d1 = dot3r(abx, aby, abz, apx, apy, apz), d2 = dot3r(acx, acy, acz, apx, apy, apz);
+    const double bpx = dsub(p.x, b.x), bpy = dsub(p.y, b.y), bpz = dsub(p.z, b.z);
+    const double d3v = dot3r(abx, aby, abz, bpx, bpy, bpz), d4 = dot3r(acx, acy, acz, bpx, bpy, bpz);
+    const double cpx = dsub(p.x, c.x), cpy = dsub(p.y, c.y), cpz = dsub(p.z, c.z);
+    const double d5 = dot3r(abx, aby, abz, cpx, cpy, cpz), d6 = dot3r(acx, acy, acz, cpx, cpy, cpz);
+    const double vc = dsub(dmul(d1, d4), dmul(d3v, d2));
+    const double vb = dsub(dmul(d5, d2), dmul(d1, d6));
+    const double va = dsub(dmul(d3v, d6), dmul(d5, d4));
+    const double d43 = dsub(d4, d3v), d56 = dsub(d5, d6);  // their signs compare the two
+    int g = 6;
+    if (le0(va) && ge0(d43) && ge0(d56)) g = 5;
+    if (le0(vb) && ge0(d2) && le0(d6)) g = 4;
+    if (ge0(d6) && le0(d56)) g = 3;
+    if (le0(vc) && ge0(d1) && le0(d3v)) g = 2;
+    if (ge0(d3v) && le0(d43)) g = 1;
+    if (le0(d1) && le0(d2)) g = 0;
+    *region = g;
+    // the nearest vertex's offset, or the region's first vertex
+    double qx = g == 1 || g == 5 ? b.x : (g == 3 ? c.x : a.x);
+    double qy = g == 1 || g == 5 ? b.y : (g == 3 ? c.y : a.y);
+    double qz = g == 1 || g == 5 ? b.z : (g == 3 ? c.z : a.z);
+    if (g == 2 || g >= 4) {
+        // v = d1 / (d1 - d3), w = d2 / (d2 - d6), w = d43 / (d43 + d56), 1 / (va + vb + vc)
+        const double num = g == 2 ? d1 : (g == 4 ? d2 : (g == 5 ? d43 : 1.0));
+        const double x = g == 2 ? d1 : (g == 4 ? d2 : (g == 5 ? d43 : dadd(va, vb)));
+        const double y = g == 2 ? -d3v : (g == 4 ? -d6 : (g == 5 ? d56 : vc));
+        const double f = ddiv(num, dadd(x, y));
+        const double s = g == 6 ? dmul(vb, f) : f;
+        const double ux = g == 4 ? acx : (g == 5 ? dsub(c.x, b.x) : abx);
+        const double uy = g == 4 ? acy : (g == 5 ? dsub(c.y, b.y) : aby);
+        const double uz = g == 4 ? acz : (g == 5 ? dsub(c.z, b.z) : abz);
+        qx = dadd(qx, dmul(s, ux));
+        qy = dadd(qy, dmul(s, uy));
+        qz = dadd(qz, dmul(s, uz));
+        if (g == 6) {
+            const double w = dmul(vc, f);
+            qx = dadd(qx, dmul(acx, w));
+            qy = dadd(qy, dmul(acy, w));
+            qz = dadd(qz, dmul(acz, w));
+        }
+    }
+    return d2r(p, qx, qy, qz);
+}
+
 static __device__ __noinline__ double ericson(const d3& p, const d3& a, const d3& b, const d3& c,
                                               int* region) {
     double abx = dsub(b.x, a.x), aby = dsub(b.y, a.y), abz = dsub(b.z, a.z);
@@ -98,6 +161,7 @@ struct alignas(16) TriRec {
     float pad_[3];
 };
 static_assert(sizeof(TriRec) == 96, "record layout");
+constexpr float kRecNormalErr = 2.4e-7f;  // TriRec::nerr of every record
 constexpr int kRecVec = static_cast<int>(sizeof(TriRec) / 16);  // float4 words per record
 
 __device__ __forceinline__ void load_rec(const TriRec* __restrict__ recs, int t, TriRec& r) {

@@ -252,6 +252,7 @@ struct Batch::Impl {
     uint32_t* work = nullptr;
     void* sort_tmp = nullptr;
     int* cand = nullptr;
+    float4* cand_c = nullptr;  // (sdf_near.cu) the candidates' centroids and radii
     int grid_exact = 0;
     int grid_eval = 0;
     cudaGraph_t graph = nullptr;
@@ -406,7 +407,10 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     // persistent evaluation grid: resident CTAs per SM for the chosen kernel
     if (opts_.grab <= 0) opts_.grab = 1;
     if (opts_.stage < 0) opts_.stage = 0;
-    if (brick == 16) impl_->grid_eval = sdf ? sdf_sub_grid(sub_precision(opts_), opts_.stage != 0, opts_.ctas) : sms;
+    if (brick == 16) {
+        const int prec = sub_precision(opts_);
+        impl_->grid_eval = !sdf ? sms : (prec == kPrecFP64 ? sdf_sub_grid(opts_.ctas) : sdf_near_grid(prec));
+    }
     else impl_->grid_eval = (brick == 4 ? 8 : 3) * sms;
     if (sdf) {  // made here: a graph capture must not create them
         CMG_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
@@ -567,7 +571,7 @@ void Batch::run_impl(bool sizing) {
         launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.bin_list, dsegs_, nseg,
                         I.large_cnt + nseg, I.large_list, ss);
         launch_brick_walk(false, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
-                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, nullptr, nullptr, nullptr,
+                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, nullptr, nullptr, nullptr, nullptr,
                           stats_, opts_.walk_warps, ss);
         exclusive_scan(I.cand_cnt, I.cand_off, nbrick_, tmp, ss);
     };
@@ -576,9 +580,11 @@ void Batch::run_impl(bool sizing) {
         CMG_CUDA(cudaMemcpyAsync(&C, I.cand_off + nbrick_, sizeof(int64_t), cudaMemcpyDeviceToHost, ss));
         CMG_CUDA(cudaStreamSynchronize(ss));
         Arena& Cn = I.cands;
+        const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
         auto planc = [&]() {
             Cn.reset();
             I.cand = carve<int>(Cn, C);
+            I.cand_c = near_list ? carve<float4>(Cn, C) : nullptr;
         };
         Cn.clear_need();
         planc();
@@ -591,7 +597,7 @@ void Batch::run_impl(bool sizing) {
     auto prep_tail = [&]() {
         launch_brick_walk(true, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
                           I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, I.cand_off, I.cand,
-                          I.brick_emax, stats_, opts_.walk_warps, ss);
+                          I.cand_c, I.brick_emax, stats_, opts_.walk_warps, ss);
         if (opts_.brick == 16) launch_sub_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);
         else launch_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);
         radix_sort_pairs(I.work_keys, I.work, nwork_, 32, I.sort_tmp, ss);
@@ -616,11 +622,15 @@ void Batch::run_impl(bool sizing) {
     CMG_CUDA(cudaStreamWaitEvent(st, join_, 0));
     side_open_ = false;
     if (timed) CMG_CUDA(cudaEventRecord(ev_[2], st));
-    if (opts_.brick == 16)
-        launch_sdf_sub(sub_precision(opts_), opts_.stage != 0, opts_.grab, opts_.probe, opts_.ctas, dsegs_,
-                       nseg, I.work, nwork_, queue_, I.soup, I.tinfo,
-                       I.tinfo_lo, I.trec, I.tnorm, I.cand_off, I.cand, I.brick_emax, opts_.band, occ,
-                       sdf32_, sdf64_, near_tri_, near_reg_, err_, stats_, I.grid_eval, st);
+    if (opts_.brick == 16 && sub_precision(opts_) == kPrecFP64)
+        launch_sdf_sub(opts_.grab, opts_.ctas, dsegs_, nseg, I.work, nwork_, queue_, I.soup, I.tinfo,
+                       I.tinfo_lo, I.trec, I.tnorm, I.cand_off, I.cand, occ, sdf32_, sdf64_,
+                       near_tri_, near_reg_, stats_, I.grid_eval, st);
+    else if (opts_.brick == 16)
+        launch_sdf_near(sub_precision(opts_), opts_.grab, opts_.probe, dsegs_, nseg,
+                        I.work, nwork_, queue_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.cand_off,
+                        I.cand, I.cand_c, opts_.band, occ, sdf32_, sdf64_, near_tri_, near_reg_, err_, stats_,
+                        I.grid_eval, st);
     else
         launch_sdf_eval(opts_.precision, opts_.brick, dsegs_, nseg, I.work, nbrick_, queue_,
                         I.soup, I.tinfo, I.cand_off, I.cand, I.brick_emax, opts_.band, occ,
@@ -678,8 +688,9 @@ RunInfo Batch::info() {
     r.brick = opts_.brick;
     r.grab = opts_.brick == 16 ? opts_.grab : 0;
     r.walk_warps = brick_walk_warps(nbrick_, opts_.walk_warps);
-    r.probe = sub_precision(opts_) != kPrecFP64 ? (opts_.probe > 0 ? opts_.probe : 1024) : 0;
-    r.ctas = opts_.brick == 16 ? sdf_sub_minb(opts_.ctas) : 0;
+    const bool plain = sub_precision(opts_) == kPrecFP64;
+    r.probe = plain || opts_.brick != 16 ? 0 : std::max(opts_.probe, 0);
+    r.ctas = opts_.brick != 16 ? 0 : (plain ? sdf_sub_minb(opts_.ctas) : impl_->grid_eval / device_sms());
     r.cells = nvox_;
     r.pairs = pairs_cap_;
     r.candidates = cand_cap_;
@@ -717,9 +728,7 @@ void Batch::download(std::vector<HostResult>& out, RunInfo* info) {
 //      taken 1 or 2 per grab, or 8^3 bricks with one evaluation CTA each;
 //   2. warps per brick of the candidate walk: 1, 2, 4 (the heaviest bricks' walks set
 //      the SDF preparation time when the bricks are few);
-//   3. mixed precision, 16^3 bricks: the probe head, 256 / 512 / 1024 / 2048 entries (a
-//      longer head gives a tighter bound and shorter filtered lists for more loads);
-//   4. 16^3 bricks: evaluation CTAs per SM, 12 (80 registers) or 16 (64 registers).
+//   3. plain FP64, 16^3 bricks: evaluation CTAs per SM, 12 (80 registers) or 16 (64).
 // Each step keeps the fastest value and moves on; the result is cached per process by
 // workload shape.
 namespace {
@@ -801,15 +810,7 @@ void autotune(const std::vector<HostMesh>& meshes, VoxOpts& opts, cudaStream_t s
         t.walk_warps = w;
         try_set(t);
     }
-    if (cur.brick == 16) {
-        if (sub_precision(opts) != kPrecFP64) {  // the FP32 pass's probe head
-            const Tuned step2 = cur;
-            for (int pr : {256, 512, 2048}) {
-                Tuned t = step2;
-                t.probe = pr;
-                try_set(t);
-            }
-        }
+    if (cur.brick == 16 && sub_precision(opts) == kPrecFP64) {
         Tuned t = cur;
         t.ctas = 16;
         try_set(t);

@@ -39,12 +39,11 @@ struct VoxOpts {
     bool want_err = false;         // mixed: stated per-cell FP32 error bound
     bool autotune = false;
     int grab = 0;                  // sub-bricks per queue grab (1, 2, 4, 8); 0 = default
-    int stage = -1;                // mixed: stage candidate records in shared memory
-                                   // (1) or read them from L1/L2 (0); -1 = default
+    int stage = -1;                // no effect (records are always staged)
     int walk_warps = 0;            // warps per brick in the candidate walk (1, 2, 4); 0 =
                                    // by the brick count
-    int probe = 0;                 // mixed: brick-list head the probe scans; 0 = default
-    int ctas = 0;                  // evaluation CTAs per SM (12 or 16); 0 = default (12)
+    int probe = 0;                 // FP32 pass: brick-list head the probe scans; 0 = all of it
+    int ctas = 0;                  // plain FP64: evaluation CTAs per SM (12 or 16); 0 = default (12)
 };
 
 struct HostMesh {
@@ -139,7 +138,7 @@ struct RunInfo {
     int brick = 0;
     int grab = 0;
     int walk_warps = 0;  // warps per brick of the candidate walk
-    int probe = 0;       // probe head (mixed)
+    int probe = 0;       // probe head (FP32 pass; 0: the whole list)
     int ctas = 0;        // evaluation CTAs per SM
     int64_t cells = 0;
     int64_t pairs = 0;       // (triangle, column) bucket entries
@@ -242,7 +241,7 @@ private:
     void sized_run();
 };
 
-// Sets opts.brick, grab, walk_warps, probe and ctas for a workload by timing the
+// Sets opts.brick, grab, walk_warps and ctas for a workload by timing the
 // candidates on the device (see engine.cu); the choice is cached per process by
 // workload shape (precision, log2 of triangle and cell counts, number of meshes,
 // whether FP64 distances are kept).

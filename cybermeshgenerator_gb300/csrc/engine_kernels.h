@@ -44,11 +44,12 @@ void launch_bin_fill(int64_t ntris, const int64_t* tbin, const int64_t* bin_off,
                      cudaStream_t st);
 void launch_seg_finish(MeshSeg* segs, int nseg, const int64_t* large_off, const unsigned* emax_bits,
                        cudaStream_t st);
+// cand_c (null: not wanted): per candidate, its centroid from the brick's centre and radius.
 void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
                        const int64_t* bin_off, const int* bin_list, const int* large_list,
                        float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
-                       float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st);
+                       float4* cand_c, float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st);
 // Warps per brick the walk uses: walk_warps when it is 1, 2 or 4, else by the brick
 // count (4 while 4-warp bricks fit about twice in the GPU, 2 up to twice that, then 1).
 int brick_walk_warps(int64_t nbricks, int walk_warps);
@@ -65,20 +66,31 @@ void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, co
                      double* sdf64, int* near_tri, uint8_t* near_reg, float* errbound, Stats* stats,
                      int grid, cudaStream_t st);
 
-// sdf_sub.cu: evaluation by 4^3 sub-bricks of 16^3 candidate bricks.
+// sdf_sub.cu: the work order of the 4^3 sub-bricks of 16^3 candidate bricks; plain FP64.
 void launch_sub_work_keys(const int* cand_cnt, int64_t nbricks, uint32_t* keys, uint32_t* vals,
                           cudaStream_t st);
-// ctas: resident CTAs per SM of the evaluation kernel (16, or 12 for any other value);
-// probe: brick-list head scanned by the mixed probe (<= 0: the default).
+// ctas: resident CTAs per SM of the evaluation kernel (16, or 12 for any other value).
 int sdf_sub_minb(int ctas);
-int sdf_sub_grid(int precision, bool stage, int ctas);
-void launch_sdf_sub(int precision, bool stage, int grab, int probe, int ctas, const MeshSeg* segs,
-                    int nseg, const uint32_t* work, int64_t nwork, unsigned long long* queue,
-                    const double* soup, const float4* tinfo, const float4* tinfo_lo, const void* trec,
-                    const float4* tnorm, const int64_t* cand_off, const int* cand, const float* brick_emax,
-                    float band_cells, const uint8_t* occ, float* sdf32, double* sdf64,
-                    int* near_tri, uint8_t* near_reg, float* errbound, Stats* stats, int grid,
-                    cudaStream_t st);
+int sdf_sub_grid(int ctas);
+// Plain FP64.
+void launch_sdf_sub(int grab, int ctas, const MeshSeg* segs, int nseg, const uint32_t* work,
+                    int64_t nwork, unsigned long long* queue, const double* soup,
+                    const float4* tinfo, const float4* tinfo_lo, const void* trec,
+                    const float4* tnorm, const int64_t* cand_off, const int* cand,
+                    const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
+                    uint8_t* near_reg, Stats* stats, int grid, cudaStream_t st);
+
+// sdf_near.cu: mixed precision and exact FP64 through the FP32 pass, a warp per
+// sub-brick. probe: head of the brick list scanned for the seed (<= 0: all of it). cand_c:
+// the candidates' centroids and radii (launch_brick_walk).
+int sdf_near_grid(int precision);
+void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, int nseg,
+                     const uint32_t* work, int64_t nwork, unsigned long long* queue,
+                     const double* soup, const float4* tinfo, const float4* tinfo_lo,
+                     const void* trec, const int64_t* cand_off, const int* cand, const float4* cand_c,
+                     float band_cells,
+                     const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
+                     uint8_t* near_reg, float* errbound, Stats* stats, int grid, cudaStream_t st);
 
 // adjoint.cu: dL/d(points) of the signed distance from the nearest-feature
 // checkpoint, per-cell terms in FP64 (kPrecFP64) or FP32 on triangle-recentred

@@ -33,6 +33,7 @@
 #include "cmg_device.cuh"
 #include "cmg_sdf.cuh"
 #include "cmg_seg.cuh"
+#include "cmg_sub.cuh"
 #include "cmg_types.h"
 #include "cmg_util.h"
 #include "engine_kernels.h"
@@ -147,7 +148,7 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
         }
         // the triangle lies in the frame's plane (to FP64 rounding), every triangle has
         // one, and its FP32 normal is within the rounding of a unit vector (sqrt(3) u)
-        r.nerr = 2.4e-7f;
+        r.nerr = kRecNormalErr;
         r.bx = static_cast<float>(bx);
         r.cx = static_cast<float>(ccx);
         r.cy = static_cast<float>(ccy);
@@ -248,9 +249,9 @@ __device__ __forceinline__ BrickGeo brick_geo(const MeshSeg& s, int64_t lb) {
     q.y0 = q.by * B; q.y1 = min(q.y0 + B, s.g.ny);
     q.z0 = (q.bz + s.bzo) * B; q.z1 = min(q.z0 + B, s.g.nz);  // bz counts from the slab's bricks
     const float h = static_cast<float>(s.g.h);
-    q.cx = 0.5f * (q.x0 + q.x1) * h;
-    q.cy = 0.5f * (q.y0 + q.y1) * h;
-    q.cz = 0.5f * (q.z0 + q.z1) * h;
+    q.cx = span_centre(q.x0, q.x1, h);
+    q.cy = span_centre(q.y0, q.y1, h);
+    q.cz = span_centre(q.z0, q.z1, h);
     double hx = 0.5 * (q.x1 - q.x0 - 1) * s.g.h, hy = 0.5 * (q.y1 - q.y0 - 1) * s.g.h,
            hz = 0.5 * (q.z1 - q.z0 - 1) * s.g.h;
     q.rb = __double2float_ru(sqrt(hx * hx + hy * hy + hz * hz) * (1.0 + 1e-9));
@@ -398,7 +399,7 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
              const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
              const int* __restrict__ large_list, float* __restrict__ bound,
              int* __restrict__ bound_tri, int* __restrict__ cand_cnt, const int64_t* __restrict__ cand_off,
-             int* __restrict__ cand, float* __restrict__ brick_emax,
+             int* __restrict__ cand, float4* __restrict__ cand_c, float* __restrict__ brick_emax,
              Stats* __restrict__ st) {
     constexpr int kWarps = kWalkThreads / 32;
     __shared__ float s_f[kWarps];
@@ -417,7 +418,7 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
     const MeshSeg& s = segs[si];
     const BrickGeo q = brick_geo(s, gb - s.brick_begin);
     const float bw = static_cast<float>(s.brick * s.g.h);
-    const float tol = 8.f * kU32 * s.scale + 1e-30f;
+    const float tol = list_tol(s.scale);
     const float emax = s.emax;
     const int rmax = max(s.bnx, max(s.bny, s.bnz));
     // reductions over the brick's warps (each of its threads calls them, at points
@@ -531,6 +532,13 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
     const int64_t out = FILL ? cand_off[gb] : 0;
     const unsigned below = (1u << lane) - 1u;
     float bemax = 0.f;
+    // a list entry: the triangle and, for the warp-per-sub-brick evaluation, its centroid
+    // from the brick's centre and its radius, so that the scans read them in order (each
+    // brick's list is scanned twice by its 64 sub-bricks)
+    auto put = [&](int64_t at, int t, const float4& ti) {
+        cand[at] = t;
+        if (cand_c) cand_c[at] = make_float4(ti.x - q.cx, ti.y - q.cy, ti.z - q.cz, ti.w);
+    };
     // walks this warp's groups of shell r; f(take, t, e_t) per entry, in walk order,
     // called by the whole warp
     auto walk = [&](int r, int n, int g0, int g1, bool& inside, auto&& f) {
@@ -548,15 +556,13 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
 #pragma unroll
                 for (int j = 0; j < kWalkRounds; ++j) {
                     bool take = false;
-                    float et = 0.f;
                     if (t[j] >= 0) {
                         float dx2 = ti[j].x - q.cx, dy2 = ti[j].y - q.cy, dz2 = ti[j].z - q.cz;
                         float d = sqrtf(dx2 * dx2 + dy2 * dy2 + dz2 * dz2) * (1.f - 4.f * kU32);
                         take = d - ti[j].w <= lim;  // |v - c_t| - e_t >= d - r_B - e_t
                         if (boxed) take = take && box_ball(box, dx2, dy2, dz2, ti[j].w, tol);
-                        et = ti[j].w;
                     }
-                    f(take, t[j], et);
+                    f(take, t[j], ti[j]);
                 }
             });
         }
@@ -568,17 +574,17 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
             const int64_t e = e0 + lane;
             bool take = false;
             int t = 0;
-            float et = 0.f;
+            float4 ti = make_float4(0.f, 0.f, 0.f, 0.f);
             if (e < s.large_end) {
                 t = large_list[e];
                 float4 lo = tlo[t], hi = thi[t];
                 float d = aabb_dist(q.cx, q.cy, q.cz, lo, hi);
                 take = d <= lim;  // d(v,t) >= d - r_B must reach U + r_B
-                et = tinfo[t].w;
+                ti = tinfo[t];
             }
             const unsigned m = __ballot_sync(0xffffffffu, take);
-            if (FILL && take) cand[out + c + __popc(m & below)] = t;
-            if (take) bemax = fmaxf(bemax, et);
+            if (FILL && take) put(out + c + __popc(m & below), t, ti);
+            if (take) bemax = fmaxf(bemax, ti.w);
             c += __popc(m);
         }
         if (lane == 0) s_c[first] = c;
@@ -596,18 +602,18 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
         int c = 0;
         if (FILL && W == 1) {
             // one warp per brick: written in the one walk, at a running offset
-            walk(r, n, g0, g1, any_inside, [&](bool take, int t, float et) {
+            walk(r, n, g0, g1, any_inside, [&](bool take, int t, const float4& ti) {
                 const unsigned m = __ballot_sync(0xffffffffu, take);
                 if (take) {
-                    cand[out + base + c + __popc(m & below)] = t;
-                    bemax = fmaxf(bemax, et);
+                    put(out + base + c + __popc(m & below), t, ti);
+                    bemax = fmaxf(bemax, ti.w);
                 }
                 c += __popc(m);
             });
             base += c;
         } else {
             walk(r, n, g0, g1, any_inside,
-                 [&](bool take, int, float) { c += __popc(__ballot_sync(0xffffffffu, take)); });
+                 [&](bool take, int, const float4&) { c += __popc(__ballot_sync(0xffffffffu, take)); });
         }
         if (FILL && W > 1) {
             // several warps: prefix sums of this shell's counts, then the writing walk
@@ -623,11 +629,11 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
             brick_sync();
             int k = 0;
             bool again = false;
-            walk(r, n, g0, g1, again, [&](bool take, int t, float et) {
+            walk(r, n, g0, g1, again, [&](bool take, int t, const float4& ti) {
                 const unsigned m = __ballot_sync(0xffffffffu, take);
                 if (take) {
-                    cand[out + off + k + __popc(m & below)] = t;
-                    bemax = fmaxf(bemax, et);
+                    put(out + off + k + __popc(m & below), t, ti);
+                    bemax = fmaxf(bemax, ti.w);
                 }
                 k += __popc(m);
             });
@@ -1144,7 +1150,7 @@ void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks
                        const float4* tinfo, const float4* tlo, const float4* thi,
                        const int64_t* bin_off, const int* bin_list, const int* large_list,
                        float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
-                       float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st) {
+                       float4* cand_c, float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st) {
     if (nbricks == 0) return;
     const int W = brick_walk_warps(nbricks, walk_warps);
     const unsigned grid = static_cast<unsigned>((nbricks * W + 3) / 4);
@@ -1153,7 +1159,8 @@ void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks
         constexpr int WW = decltype(w_tag)::value;
         k_brick_walk<F, WW><<<grid, kWalkThreads, 0, st>>>(segs, nseg, nbricks, soup, tinfo, tlo, thi,
                                                            bin_off, bin_list, large_list, bound,
-                                                           bound_tri, cand_cnt, cand_off, cand, brick_emax, stats);
+                                                           bound_tri, cand_cnt, cand_off, cand, cand_c, brick_emax,
+                                                           stats);
     };
     using T = std::true_type;
     using Fa = std::false_type;

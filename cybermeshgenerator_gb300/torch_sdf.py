@@ -45,8 +45,8 @@ class SDFPlan:
     cubic cell edge and ``(nx, ny, nz)``. ``precision`` is ``PREC_FP64`` (plain,
     bit-identical to the reference's distances) or ``PREC_MIXED``. ``autotune`` times
     the pipeline's tunables on this mesh and grid at creation (brick edge, queue grab,
-    walk warps, probe head, evaluation CTAs per SM) and keeps the fastest; ``tuning``
-    (keys of ``make_opts``) sets them instead."""
+    walk warps) and keeps the fastest; ``tuning`` (keys of ``make_opts``) sets them
+    instead."""
 
     def __init__(self, vertices, faces, grid, precision: int = PREC_FP64,
                  predicates: int = PRED_COMPAT, band: float = 1.0, brick: int = 0,

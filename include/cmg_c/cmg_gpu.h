@@ -54,16 +54,17 @@ typedef struct cmg_voxel_opts {
     int brick;           /* SDF candidate brick edge: 0 = default (16, evaluated by 4^3
                             sub-bricks), 8 or 4 (one evaluation CTA per brick) */
     int autotune;        /* nonzero (with brick 0): time the brick edges, queue grab sizes,
-                            walk warps, probe heads and evaluation CTAs per SM on this
+                            walk warps and (plain FP64) evaluation CTAs per SM on this
                             input and keep the fastest */
     int grab;            /* sub-bricks taken per work-queue grab: 0 = default, 1, 2, 4, 8 */
-    int stage;           /* mixed: 1 stage candidate records in shared memory, 0 read them
-                            through L1/L2, -1 = default */
+    int stage;           /* no effect: candidate records are always staged in shared memory
+                            (kept for callers that set it) */
     int walk_warps;      /* warps per brick of the candidate walk: 1, 2 or 4; 0 = by the
                             brick count */
-    int probe;           /* mixed: brick-list head the probe scans (entries); 0 = 1024 */
-    int ctas;            /* evaluation CTAs per SM the registers are budgeted for: 16, or
-                            0 / 12 = 12 */
+    int probe;           /* entries of the brick list the probe of the FP32 pass scans; 0 =
+                            the whole list */
+    int ctas;            /* plain FP64: evaluation CTAs per SM the registers are budgeted for,
+                            16, or 0 / 12 = 12 */
     int z_begin, z_end;  /* cell layers [z_begin, z_end) of the grid to evaluate (a z-slab,
                             e.g. one rank's share); z_end 0 = through the last layer. The
                             slab's cells equal the whole grid's bit for bit (same centres,
@@ -88,7 +89,7 @@ typedef struct cmg_voxel_stats {
     int grab;                  /* sub-bricks per work-queue grab used (16^3 bricks) */
     double max_error_bound;    /* mixed: largest stated per-cell bound (0 for FP64) */
     int walk_warps;            /* warps per brick of the candidate walk used */
-    int probe;                 /* probe head used (mixed; 0 for FP64) */
+    int probe;                 /* probe head asked for (0: the whole list) */
     int ctas;                  /* evaluation CTAs per SM used (16^3 bricks) */
 } cmg_voxel_stats;
 
