@@ -245,6 +245,163 @@ __device__ __forceinline__ bool insphere_int_exact64(const d3& a, const d3& b, c
     return insphere_int(a, b, c, d, e, sign);
 }
 
+// ---- wide integers
+// N 64-bit limbs, little-endian, two's complement.
+template <int N>
+struct Big {
+    unsigned long long w[N];
+};
+template <int N>
+__device__ __forceinline__ bool negative(const Big<N>& a) {
+    return static_cast<long long>(a.w[N - 1]) < 0;
+}
+template <int N>
+__device__ __forceinline__ Big<N> negate_if(const Big<N>& a, bool neg) {
+    const unsigned long long m = neg ? ~0ull : 0ull;
+    Big<N> r;
+    unsigned long long carry = neg ? 1ull : 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r.w[i] = (a.w[i] ^ m) + carry;
+        carry = carry && r.w[i] == 0ull ? 1ull : 0ull;
+    }
+    return r;
+}
+// a + b, or a - b (NEG).
+template <bool NEG, int N>
+__device__ __forceinline__ Big<N> add(const Big<N>& a, const Big<N>& b) {
+    Big<N> r;
+    unsigned long long carry = NEG ? 1ull : 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const unsigned long long y = NEG ? ~b.w[i] : b.w[i];
+        const unsigned long long x = a.w[i] + y, z = x + carry;
+        carry = (x < y ? 1ull : 0ull) | (z < x ? 1ull : 0ull);
+        r.w[i] = z;
+    }
+    return r;
+}
+// The product, exactly, in N + M limbs.
+template <int N, int M>
+__device__ __forceinline__ Big<N + M> mul(const Big<N>& a, const Big<M>& b) {
+    const bool na = negative(a), nb = negative(b);
+    const Big<N> x = negate_if(a, na);
+    const Big<M> y = negate_if(b, nb);
+    Big<N + M> r;
+#pragma unroll
+    for (int i = 0; i < N + M; ++i) r.w[i] = 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        unsigned long long carry = 0ull;
+#pragma unroll
+        for (int j = 0; j < M; ++j) {
+            const unsigned __int128 t =
+                static_cast<unsigned __int128>(x.w[i]) * y.w[j] + r.w[i + j] + carry;
+            r.w[i + j] = static_cast<unsigned long long>(t);
+            carry = static_cast<unsigned long long>(t >> 64);
+        }
+        r.w[i + M] = carry;
+    }
+    return negate_if(r, na != nb);
+}
+template <int N>
+__device__ __forceinline__ int sign_of(const Big<N>& a) {
+    unsigned long long any = 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) any |= a.w[i];
+    return negative(a) ? -1 : (any != 0ull ? 1 : 0);
+}
+
+// The n coordinates of a query as integers of at most 100 bits in a common power-of-two
+// scale 2^L, exactly; false when they span more, or lie where the expansions below could
+// underflow or overflow too (L < lmin_ok, or a coordinate of 2^emax_ok or more). A query
+// within a few ulps of an integer tie spans some 70 bits.
+__device__ __forceinline__ bool scale_to_wide(const double* v, int n, int lmin_ok, int emax_ok,
+                                              __int128* out) {
+    int lmin = 0x7fffffff, emax = -0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+        const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v[i]));
+        if ((b << 1) == 0ull) continue;  // +-0
+        const int ef = static_cast<int>((b >> 52) & 0x7ffull);
+        if (ef == 0 || ef == 0x7ff) return false;  // subnormal, infinite or NaN
+        const unsigned long long m = (b & 0xfffffffffffffull) | (1ull << 52);
+        lmin = min(lmin, ef - 1075 + (__ffsll(static_cast<long long>(m)) - 1));
+        emax = max(emax, ef - 1023);
+    }
+    if (lmin == 0x7fffffff) lmin = emax = 0;  // all zero
+    if (emax - lmin + 1 > 100 || lmin < lmin_ok || emax >= emax_ok) return false;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+        const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v[i]));
+        out[i] = 0;
+        if ((b << 1) == 0ull) continue;
+        const unsigned long long m = (b & 0xfffffffffffffull) | (1ull << 52);
+        const int tz = __ffsll(static_cast<long long>(m)) - 1;
+        const int lb = static_cast<int>((b >> 52) & 0x7ffull) - 1075 + tz;
+        const __int128 x = static_cast<__int128>(m >> tz) << (lb - lmin);
+        out[i] = (b >> 63) ? -x : x;
+    }
+    return true;
+}
+__device__ __forceinline__ Big<2> wide_diff(__int128 a, __int128 b) {
+    const __int128 d = a - b;
+    return {{static_cast<unsigned long long>(d), static_cast<unsigned long long>(d >> 64)}};
+}
+// ux vy - vx uy
+__device__ __forceinline__ Big<4> wide_minor(const Big<2>& ux, const Big<2>& uy, const Big<2>& vx,
+                                             const Big<2>& vy) {
+    return add<true>(mul(ux, vy), mul(vx, uy));
+}
+
+// Exact signs in wide integers, on the integer pipe (expansion arithmetic for the same
+// queries runs on FP64, which issues one warp instruction per 16 cycles and SM, out of local
+// memory: 106k near-tie insphere queries took 3.7 ms that way, 70k orient3d 0.37 ms).
+// orient3d: differences < 2^101, minors < 2^203, the determinant < 2^306 (6 limbs).
+static __device__ __noinline__ bool orient3d_wide(const d3& a, const d3& b, const d3& c, const d3& d,
+                                                  int* sign) {
+    const double v[12] = {a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z, d.x, d.y, d.z};
+    __int128 X[12];
+    if (!scale_to_wide(v, 12, -320, 300, X)) return false;
+    const Big<2> adx = wide_diff(X[0], X[9]), ady = wide_diff(X[1], X[10]), adz = wide_diff(X[2], X[11]);
+    const Big<2> bdx = wide_diff(X[3], X[9]), bdy = wide_diff(X[4], X[10]), bdz = wide_diff(X[5], X[11]);
+    const Big<2> cdx = wide_diff(X[6], X[9]), cdy = wide_diff(X[7], X[10]), cdz = wide_diff(X[8], X[11]);
+    Big<6> det = mul(adz, wide_minor(bdx, bdy, cdx, cdy));
+    det = add<false>(det, mul(bdz, wide_minor(cdx, cdy, adx, ady)));
+    det = add<false>(det, mul(cdz, wide_minor(adx, ady, bdx, bdy)));
+    *sign = sign_of(det);
+    return true;
+}
+
+// insphere (the lifted 4x4 form, e as origin): differences < 2^101, minors < 2^203, 3x3
+// minors < 2^306, lifts < 2^204, the determinant < 2^512 (10 limbs).
+static __device__ __noinline__ bool insphere_wide(const d3& a, const d3& b, const d3& c, const d3& d,
+                                                  const d3& e, int* sign) {
+    const double v[15] = {a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z,
+                          d.x, d.y, d.z, e.x, e.y, e.z};
+    __int128 X[15];
+    if (!scale_to_wide(v, 15, -190, 180, X)) return false;
+    Big<2> p[4][3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[i][k] = wide_diff(X[3 * i + k], X[12 + k]);
+    // minors of rows (i, j): ab, bc, cd, da, ac, bd
+    auto minor = [&](int i, int j) { return wide_minor(p[i][0], p[i][1], p[j][0], p[j][1]); };
+    auto lift = [&](int i) {
+        return add<false>(add<false>(mul(p[i][0], p[i][0]), mul(p[i][1], p[i][1])), mul(p[i][2], p[i][2]));
+    };
+    const Big<4> ab = minor(0, 1), bc = minor(1, 2), cd = minor(2, 3), da = minor(3, 0), ac = minor(0, 2),
+                 bd = minor(1, 3);
+    // det = dl abc - cl dab + bl cda - al bcd
+    Big<10> det = mul(lift(3), add<false>(add<true>(mul(p[0][2], bc), mul(p[1][2], ac)), mul(p[2][2], ab)));
+    det = add<true>(det, mul(lift(2), add<false>(add<false>(mul(p[3][2], ab), mul(p[0][2], bd)), mul(p[1][2], da))));
+    det = add<false>(det, mul(lift(1), add<false>(add<false>(mul(p[2][2], da), mul(p[3][2], ac)), mul(p[0][2], cd))));
+    det = add<true>(det, mul(lift(0), add<false>(add<true>(mul(p[1][2], cd), mul(p[2][2], bd)), mul(p[3][2], bc))));
+    *sign = sign_of(det);
+    return true;
+}
+
 // h = e + f: merge by magnitude, then a Two-Sum sweep, zero-eliminated.
 // h holds elen + flen doubles and may not alias e or f.
 static __device__ __noinline__ int sum(int elen, const double* e, int flen, const double* f,
@@ -364,7 +521,7 @@ static __device__ __noinline__ int orient3d_homogeneous(const d3& a, const d3& b
 static __device__ __noinline__ int orient3d_sign(const d3& a, const d3& b, const d3& c, const d3& d) {
     {
         int sg;
-        if (orient3d_int(a, b, c, d, &sg)) return sg;
+        if (orient3d_int(a, b, c, d, &sg) || orient3d_wide(a, b, c, d, &sg)) return sg;
         double det;
         if (orient3d_certified(a, b, c, d, &det)) return det > 0.0 ? 1 : (det < 0.0 ? -1 : 0);
     }
@@ -425,8 +582,6 @@ constexpr int kInsphereCap = 256;
 static __device__ __noinline__ int insphere_sign(const d3& a, const d3& b, const d3& c, const d3& d,
                                           const d3& e, int* overflow) {
     {
-        int sg;
-        if (insphere_int(a, b, c, d, e, &sg)) return sg;
         double det;
         if (insphere_certified(a, b, c, d, e, &det)) return det > 0.0 ? 1 : (det < 0.0 ? -1 : 0);
     }

@@ -16,11 +16,10 @@
 //                 operation, plus the FP64 filter bound of the reference: a sign it
 //                 certifies is the exact sign and also the sign of the FP64 rounded
 //                 determinant, so it serves both modes;
-//   k_pred_fp64   the reference's rounded determinant (and, in EXACT mode, its
-//                 permanent bound); when that does not decide, an evaluation with
-//                 exactness tracking (cmg_exact.cuh): if no operation rounded, its
-//                 value is the exact determinant;
-//   k_pred_exact  expansion arithmetic (cmg_exact.cuh).
+//   k_pred_fp64   integer coordinates (after a common power-of-two scaling): the exact
+//                 determinant on the integer pipe; else the reference's rounded
+//                 determinant (and, in EXACT mode, its permanent bound);
+//   k_pred_exact  wide integers, else expansion arithmetic (cmg_exact.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -498,7 +497,13 @@ __device__ __forceinline__ void seg_prefix(const Seg& L, unsigned long long* pre
 }
 
 // The FP64 pass over the segmented list of the FP32 pass (list position k counts
-// through the segments in order); writes the list's length to *n32.
+// through the segments in order); writes the list's length to *n32. Integer coordinates
+// first, on the integer pipe: in EXACT mode their sign decides; in COMPAT mode too when
+// the FP64 evaluation is provably exact there (it then equals the exact determinant). The
+// queries that need the FP64 determinant wait in shared memory and are evaluated 256 at a
+// time, so that the FP64 pipe (one warp instruction per 16 cycles and SM) works on full
+// warps: where half the list is integer ties, every warp had run it half empty.
+constexpr int kWaiting = 2 * kThreads;
 template <int NPT, int MODE>
 __global__ void __launch_bounds__(kThreads) k_pred_fp64(Soa s, Seg L,
                                                         unsigned long long* __restrict__ n32,
@@ -507,15 +512,31 @@ __global__ void __launch_bounds__(kThreads) k_pred_fp64(Soa s, Seg L,
                                                         unsigned long long* __restrict__ count,
                                                         unsigned long long* __restrict__ ncert) {
     __shared__ unsigned long long s_pre[kMaxSeg + 1];
+    __shared__ int64_t s_at[kWaiting];  // query index << 2 | 1 + exact sign (3: not known)
+    __shared__ int64_t s_slot[kWaiting];  // its compact coordinates, or -1
+    __shared__ int s_n;
     seg_prefix(L, s_pre);
     const int64_t n = static_cast<int64_t>(s_pre[L.nseg]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n32 = static_cast<unsigned long long>(n);
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const int64_t n_round = (n + 31) & ~int64_t(31);
-    for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n_round;
-         k += stride) {
-        bool undecided = false, certified = false;
-        int64_t i = 0;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        s_n = 0;
+        if (blockIdx.x == 0) *n32 = static_cast<unsigned long long>(n);
+    }
+    __syncthreads();
+    auto load = [&](int64_t i, int64_t slot, double* v) {
+        if (slot >= 0) {
+#pragma unroll
+            for (int c = 0; c < 3 * NPT; ++c) v[c] = L.cc[c][slot];
+        } else {
+            load_query<NPT>(s, i, v);
+        }
+    };
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
+    for (int64_t k0 = static_cast<int64_t>(blockIdx.x) * kThreads; k0 < n || s_n > 0; k0 += stride) {
+        const int64_t k = k0 + threadIdx.x;
+        bool waits = false, certified = false;
+        int64_t i = 0, slot = -1;
+        int known = 3;
         if (k < n) {
             // the segment holding position k: the last with pre[b] <= k
             int lo = 0, hi = L.nseg - 1;
@@ -526,74 +547,80 @@ __global__ void __launch_bounds__(kThreads) k_pred_fp64(Soa s, Seg L,
             }
             const int64_t j = k - static_cast<int64_t>(s_pre[lo]);
             i = L.list[static_cast<int64_t>(lo) * L.segcap + j];
+            if (j < L.ccap) slot = static_cast<int64_t>(lo) * L.ccap + j;
             double v[3 * NPT];
-            if (j < L.ccap) {
-#pragma unroll
-                for (int c = 0; c < 3 * NPT; ++c) v[c] = L.cc[c][static_cast<int64_t>(lo) * L.ccap + j];
-            } else {
-                load_query<NPT>(s, i, v);
-            }
+            load(i, slot, v);
             const d3 a{v[0], v[1], v[2]}, b{v[3], v[4], v[5]}, c{v[6], v[7], v[8]}, d{v[9], v[10], v[11]};
-            // integer coordinates first (integer pipe): in EXACT mode their sign decides;
-            // in COMPAT mode too when the FP64 evaluation is provably exact there (it then
-            // equals the exact determinant), which spares the narrow FP64 pipe
+            const d3 e{NPT == 5 ? v[12] : 0.0, NPT == 5 ? v[13] : 0.0, NPT == 5 ? v[14] : 0.0};
             int isg = 0;
-            bool ic = false;
-            {
-                const d3 e5{NPT == 5 ? v[12] : 0.0, NPT == 5 ? v[13] : 0.0, NPT == 5 ? v[14] : 0.0};
-                bool fexact = false;
-                ic = NPT == 4 ? exact::orient3d_int_exact64(a, b, c, d, &isg, &fexact)
-                              : exact::insphere_int_exact64(a, b, c, d, e5, &isg, &fexact);
-                if (ic && (MODE == kPredExact || fexact)) {
-                    out[i] = static_cast<int8_t>(isg);
-                    certified = true;
-                }
+            bool fexact = false;
+            const bool ic = NPT == 4 ? exact::orient3d_int_exact64(a, b, c, d, &isg, &fexact)
+                                     : exact::insphere_int_exact64(a, b, c, d, e, &isg, &fexact);
+            if (ic && (MODE == kPredExact || fexact)) {
+                out[i] = static_cast<int8_t>(isg);
+                certified = true;
+            } else {
+                waits = true;
+                if (ic) known = 1 + isg;
             }
-            double perm = 0.0, det = 0.0;
-            if (certified) {
-            } else if (NPT == 4) {
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, waits);
+        int base = 0;
+        if (lane == 0 && m) base = atomicAdd(&s_n, __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (waits) {
+            const int at = base + __popc(m & ((1u << lane) - 1u));
+            s_at[at] = i << 2 | known;
+            s_slot[at] = slot;
+        }
+        __syncthreads();
+        // the last 256 waiting; all of them once the list has ended
+        const int have = s_n;
+        const bool last = k0 + stride >= n;
+        const int take = have >= kThreads ? kThreads : (last ? have : 0);
+        __syncthreads();
+        if (threadIdx.x == 0) s_n = have - take;
+        bool undecided = false;
+        if (static_cast<int>(threadIdx.x) < take) {
+            const int at = have - take + threadIdx.x;
+            i = s_at[at] >> 2;
+            known = static_cast<int>(s_at[at] & 3);
+            double v[3 * NPT];
+            load(i, s_slot[at], v);
+            const d3 a{v[0], v[1], v[2]}, b{v[3], v[4], v[5]}, c{v[6], v[7], v[8]}, d{v[9], v[10], v[11]};
+            double perm = 0.0, det;
+            if (NPT == 4) {
                 det = o3d_fast(a, b, c, d, MODE == kPredExact ? &perm : nullptr);
                 perm *= kO3dErrA;
             } else {
-                const d3 e{v[12], v[13], v[14]};
-                det = isp_fast(a, b, c, d, e, MODE == kPredExact ? &perm : nullptr);
+                det = isp_fast(a, b, c, d, {v[12], v[13], v[14]}, MODE == kPredExact ? &perm : nullptr);
                 perm *= kIspErrA;
             }
-            bool decided = certified || (MODE == kPredCompat ? det != 0.0 : (det > perm || -det > perm));
-            if (certified) {
-            } else if (decided) {
+            if (MODE == kPredCompat ? det != 0.0 : (det > perm || -det > perm)) {
                 out[i] = static_cast<int8_t>(sgn(det));
+            } else if (known != 3) {
+                // the exact determinant from the integer pipe
+                out[i] = static_cast<int8_t>(known - 1);
+                certified = true;
             } else {
-                // integer coordinates after a common power-of-two scaling gave the
-                // exact determinant on the integer pipe above; else an FP64 evaluation
-                // in which no operation rounded is the exact determinant
-                const d3 e{NPT == 5 ? v[12] : 0.0, NPT == 5 ? v[13] : 0.0, NPT == 5 ? v[14] : 0.0};
-                if (ic) {
-                    out[i] = static_cast<int8_t>(isg);
-                    decided = certified = true;
-                } else {
-                    double ex;
-                    const bool cert = NPT == 4 ? exact::orient3d_certified(a, b, c, d, &ex)
-                                               : exact::insphere_certified(a, b, c, d, e, &ex);
-                    if (cert) {
-                        out[i] = static_cast<int8_t>(sgn(ex));
-                        decided = certified = true;
-                    }
-                }
+                undecided = true;
             }
-            undecided = !decided;
         }
         const unsigned cm = __ballot_sync(0xffffffffu, certified);
-        if (cm && (threadIdx.x & 31) == 0) atomicAdd(ncert, static_cast<unsigned long long>(__popc(cm)));
+        if (cm && lane == 0) atomicAdd(ncert, static_cast<unsigned long long>(__popc(cm)));
         push(undecided, i, list, count);
+        __syncthreads();
     }
 }
 
+// The queries left: wide integers (near-ties span some 70 bits), then an FP64 evaluation in
+// which no operation rounded, then expansions (counted).
 template <int NPT>
-__global__ void __launch_bounds__(128) k_pred_exact(Soa s, const int64_t* __restrict__ in,
-                                                    const unsigned long long* __restrict__ nin,
-                                                    int8_t* __restrict__ out,
-                                                    unsigned long long* __restrict__ overflow) {
+__global__ void __launch_bounds__(64) k_pred_exact(Soa s, const int64_t* __restrict__ in,
+                                                   const unsigned long long* __restrict__ nin,
+                                                   int8_t* __restrict__ out,
+                                                   unsigned long long* __restrict__ overflow,
+                                                   unsigned long long* __restrict__ nexp) {
     const int64_t n = static_cast<int64_t>(*nin);
     for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
          k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -603,11 +630,18 @@ __global__ void __launch_bounds__(128) k_pred_exact(Soa s, const int64_t* __rest
         const d3 a{v[0], v[1], v[2]}, b{v[3], v[4], v[5]}, c{v[6], v[7], v[8]}, d{v[9], v[10], v[11]};
         int sg;
         if (NPT == 4) {
-            sg = exact::orient3d_sign(a, b, c, d);
+            if (!exact::orient3d_wide(a, b, c, d, &sg)) {
+                sg = exact::orient3d_sign(a, b, c, d);
+                atomicAdd(nexp, 1ull);
+            }
         } else {
-            int of = 0;
-            sg = exact::insphere_sign(a, b, c, d, {v[12], v[13], v[14]}, &of);
-            if (of) atomicAdd(overflow, 1ull);
+            const d3 e{v[12], v[13], v[14]};
+            if (!exact::insphere_wide(a, b, c, d, e, &sg)) {
+                int of = 0;
+                sg = exact::insphere_sign(a, b, c, d, e, &of);
+                if (of) atomicAdd(overflow, 1ull);
+                atomicAdd(nexp, 1ull);
+            }
         }
         out[i] = static_cast<int8_t>(sg);
     }
@@ -657,6 +691,7 @@ struct Counters {
     unsigned long long n64;  // left by the FP64 pass
     unsigned long long overflow;
     unsigned long long certified;  // decided in the FP64 pass by an exact evaluation
+    unsigned long long expanded;   // needed more than wide integers in the exact pass
     unsigned long long fault;      // a TMA wait of the FP32 pass ran out
     unsigned long long drain_fault;  // ... and so did the drain of the copies in flight
     unsigned long long seg[kMaxSeg];  // entries per segment of the FP32 pass's list
@@ -705,8 +740,8 @@ static void pred_stream_finish(int npt, const Soa& s, int mode, int8_t* d_out, S
         k_pred_fp64<5, kPredCompat><<<2 * sms, kThreads, 0, st>>>(s, L, &c->n32, d_out, list_b, &c->n64,
                                                                       &c->certified);
     CMG_LAUNCH();
-    if (npt == 4) k_pred_exact<4><<<2 * sms, 128, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow);
-    else k_pred_exact<5><<<2 * sms, 128, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow);
+    if (npt == 4) k_pred_exact<4><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded);
+    else k_pred_exact<5><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded);
     CMG_LAUNCH();
 }
 
@@ -914,6 +949,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
                 hc.n32 += hcs[c].n32;
                 hc.n64 += hcs[c].n64;
                 hc.certified += hcs[c].certified;
+                hc.expanded += hcs[c].expanded;
                 hc.overflow |= hcs[c].overflow;
                 float ms = 0.f;
                 CMG_CUDA(cudaEventElapsedTime(&ms, w.chunk_ev[2 * c], w.chunk_ev[2 * c + 1]));
@@ -992,6 +1028,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
                 hc.n32 += hcs[c].n32;
                 hc.n64 += hcs[c].n64;
                 hc.certified += hcs[c].certified;
+                hc.expanded += hcs[c].expanded;
                 hc.overflow |= hcs[c].overflow;
                 float ms = 0.f;
                 CMG_CUDA(cudaEventElapsedTime(&ms, w.chunk_ev[2 * c], w.chunk_ev[2 * c + 1]));
@@ -1003,7 +1040,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
             stats->queries = n;
             stats->fp64_queries = static_cast<int64_t>(hc.n32);
             stats->exact_queries = static_cast<int64_t>(hc.n64 + hc.certified);
-            stats->expansion_queries = static_cast<int64_t>(hc.n64);
+            stats->expansion_queries = static_cast<int64_t>(hc.expanded);
             stats->tma_reruns = reruns;
         }
         if (hc.overflow) {
