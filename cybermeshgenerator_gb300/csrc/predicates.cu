@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -297,12 +298,18 @@ __global__ void k_put_bytes(const int8_t* __restrict__ src, int8_t* __restrict__
 // reruns the pass with the per-thread loads. When the drain's own bounded waits run out
 // as well, the CTA sets `drain_fault` too: copies may still have been writing its
 // shared memory, and the host reports an error instead of rerunning.
-template <int NPT>
+// Columns that start 8 bytes off a 16-byte boundary (SKEW: the bulk copies move whole
+// 16-byte words; every second column of a matrix with an odd row length) are copied from the
+// boundary below, one word more per tile, and read one value later: the words at both
+// ends hold a value of the column, so they lie in its allocation. (2,000,003 queries a
+// kind from such rows, FP32 passes: 66 + 95 us by per-thread loads, 38 + 54 us by these:
+// 5.1 + 4.5 TB/s.)
+template <int NPT, bool SKEW>
 struct Tma {
     static constexpr int kCols = 3 * NPT;
     static constexpr int kStages = NPT == 4 ? 4 : 3;
-    static constexpr unsigned kStageBytes = kCols * kTile * 8u;
-    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kStageBytes;
+    static constexpr int kPitch = kTile + (SKEW ? 2 : 0);  // values per column and stage
+    static constexpr size_t kSmem = static_cast<size_t>(kStages) * kCols * kPitch * 8u;
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -361,16 +368,21 @@ constexpr int kTmaThreads = kThreads + 32;
 // fail_at >= 0 (tests): consumer warp 0 of CTA 0 takes its wait for tile fail_at as
 // having run out, which drives the abort, the drain and the host's rerun without a
 // wait that really runs out.
-template <int NPT>
+template <int NPT, bool SKEW>
 __global__ void __launch_bounds__(kTmaThreads) k_pred_fp32_tma(Soa s, int64_t ntiles,
                                                                int8_t* __restrict__ out, Seg L,
                                                                unsigned long long* __restrict__ fault,
                                                                unsigned long long* __restrict__ drain_fault,
                                                                int64_t fail_at) {
-    using T = Tma<NPT>;
-    constexpr int C = T::kCols, S = T::kStages;
+    using T = Tma<NPT, SKEW>;
+    constexpr int C = T::kCols, S = T::kStages, W = T::kPitch;
     extern __shared__ __align__(128) unsigned char smem[];
-    double* buf = reinterpret_cast<double*>(smem);  // [S][C][kTile]
+    double* buf = reinterpret_cast<double*>(smem);  // [S][C][W]
+    unsigned skew = 0;  // bit c: column c starts 8 bytes off
+    if (SKEW) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) skew |= static_cast<unsigned>((reinterpret_cast<uintptr_t>(s.c[c]) >> 3) & 1u) << c;
+    }
     __shared__ __align__(8) unsigned long long full[S], empty[S];
     __shared__ unsigned long long s_cnt;  // entries of this CTA's segment so far
     __shared__ long long s_last[S];       // the last tile issued into each stage (-1: none)
@@ -403,11 +415,13 @@ __global__ void __launch_bounds__(kTmaThreads) k_pred_fp32_tma(Soa s, int64_t nt
                 // the copy into the stage follows the consumers' generic reads of it
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 const int64_t tile = b + k * gridDim.x;
-                mbar_expect_tx(&full[st], T::kStageBytes);
+                mbar_expect_tx(&full[st], C * kTile * 8u + (SKEW ? __popc(skew) * 16u : 0u));
 #pragma unroll
-                for (int c = 0; c < C; ++c)
-                    bulk_copy(buf + (static_cast<size_t>(st) * C + c) * kTile, s.c[c] + tile * kTile,
-                              kTile * 8u, &full[st]);
+                for (int c = 0; c < C; ++c) {
+                    const unsigned off = SKEW ? (skew >> c) & 1u : 0u;
+                    bulk_copy(buf + (static_cast<size_t>(st) * C + c) * W, s.c[c] + tile * kTile - off,
+                              kTile * 8u + off * 16u, &full[st]);
+                }
                 s_last[st] = k;
             }
         }
@@ -423,12 +437,13 @@ __global__ void __launch_bounds__(kTmaThreads) k_pred_fp32_tma(Soa s, int64_t nt
                 break;
             }
             const int64_t i = (b + k * gridDim.x) * kTile + tid;
-            const double* sb = buf + static_cast<size_t>(st) * C * kTile;
+            const double* sb = buf + static_cast<size_t>(st) * C * W + tid;
+            auto at = [&](int c) { return c * W + (SKEW ? (skew >> c) & 1u : 0u); };
             int sg;
             {
                 double v[C];
 #pragma unroll
-                for (int c = 0; c < C; ++c) v[c] = sb[c * kTile + tid];
+                for (int c = 0; c < C; ++c) v[c] = sb[at(c)];
                 sg = NPT == 4 ? o3d_fp32(v) : isp_fp32(v);
                 out[i] = static_cast<int8_t>(sg);
             }
@@ -441,7 +456,7 @@ __global__ void __launch_bounds__(kTmaThreads) k_pred_fp32_tma(Soa s, int64_t nt
                 if (pos < L.ccap) {
                     const volatile double* vb = sb;
 #pragma unroll
-                    for (int c = 0; c < C; ++c) L.cc[c][cbase + pos] = vb[c * kTile + tid];
+                    for (int c = 0; c < C; ++c) L.cc[c][cbase + pos] = vb[at(c)];
                 }
             }
             // this warp is done with the stage
@@ -510,7 +525,10 @@ __global__ void __launch_bounds__(kThreads) k_pred_fp64(Soa s, Seg L,
                                                         int8_t* __restrict__ out,
                                                         int64_t* __restrict__ list,
                                                         unsigned long long* __restrict__ count,
-                                                        unsigned long long* __restrict__ ncert) {
+                                                        unsigned long long* __restrict__ ncert,
+                                                        const unsigned long long* __restrict__ halt) {
+    // copies of the FP32 pass that could not be drained may still be landing in shared memory
+    if (*halt) return;
     __shared__ unsigned long long s_pre[kMaxSeg + 1];
     __shared__ int64_t s_at[kWaiting];  // query index << 2 | 1 + exact sign (3: not known)
     __shared__ int64_t s_slot[kWaiting];  // its compact coordinates, or -1
@@ -620,7 +638,9 @@ __global__ void __launch_bounds__(64) k_pred_exact(Soa s, const int64_t* __restr
                                                    const unsigned long long* __restrict__ nin,
                                                    int8_t* __restrict__ out,
                                                    unsigned long long* __restrict__ overflow,
-                                                   unsigned long long* __restrict__ nexp) {
+                                                   unsigned long long* __restrict__ nexp,
+                                                   const unsigned long long* __restrict__ halt) {
+    if (*halt) return;
     const int64_t n = static_cast<int64_t>(*nin);
     for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
          k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -729,19 +749,21 @@ static void pred_stream_finish(int npt, const Soa& s, int mode, int8_t* d_out, S
     L.cnt = c->seg;
     if (npt == 4 && mode == kPredExact)
         k_pred_fp64<4, kPredExact><<<2 * sms, kThreads, 0, st>>>(s, L, &c->n32, d_out, list_b, &c->n64,
-                                                                      &c->certified);
+                                                                      &c->certified, &c->drain_fault);
     else if (npt == 4)
         k_pred_fp64<4, kPredCompat><<<2 * sms, kThreads, 0, st>>>(s, L, &c->n32, d_out, list_b, &c->n64,
-                                                                      &c->certified);
+                                                                      &c->certified, &c->drain_fault);
     else if (mode == kPredExact)
         k_pred_fp64<5, kPredExact><<<2 * sms, kThreads, 0, st>>>(s, L, &c->n32, d_out, list_b, &c->n64,
-                                                                      &c->certified);
+                                                                      &c->certified, &c->drain_fault);
     else
         k_pred_fp64<5, kPredCompat><<<2 * sms, kThreads, 0, st>>>(s, L, &c->n32, d_out, list_b, &c->n64,
-                                                                      &c->certified);
+                                                                      &c->certified, &c->drain_fault);
     CMG_LAUNCH();
-    if (npt == 4) k_pred_exact<4><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded);
-    else k_pred_exact<5><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded);
+    if (npt == 4) k_pred_exact<4><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded,
+                                                          &c->drain_fault);
+    else k_pred_exact<5><<<8 * sms, 64, 0, st>>>(s, list_b, &c->n64, d_out, &c->overflow, &c->expanded,
+                                                          &c->drain_fault);
     CMG_LAUNCH();
 }
 
@@ -753,62 +775,67 @@ static void pred_fp32_loads(int npt, const Soa& s, int64_t t0, int64_t t1, int64
     CMG_LAUNCH();
 }
 
-// Runs the three passes on device-resident SoA coordinates, the FP32 pass's list in
-// the segments of L (shaped for at least n queries). Returns the number of times the
-// FP32 pass was rerun with per-thread loads after a TMA wait ran out (0 or 1); throws
-// when copies may have outlived their CTA.
-int pred_stream_device(int npt, const double* const* coords, int64_t n, int mode, int8_t* d_out,
-                        Seg L, int64_t* list_b, void* counters, cudaStream_t st, int sms,
-                        cudaEvent_t* fp32_events) {
+template <int NPT, bool SKEW>
+static void pred_fp32_tma(const Soa& s, int64_t ntiles, int8_t* d_out, const Seg& L, Counters* c,
+                          int64_t fail_at, cudaStream_t st) {
+    constexpr size_t bytes = Tma<NPT, SKEW>::kSmem;
+    CMG_CUDA(cudaFuncSetAttribute(k_pred_fp32_tma<NPT, SKEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(bytes)));
+    k_pred_fp32_tma<NPT, SKEW><<<L.nseg, kTmaThreads, bytes, st>>>(s, ntiles, d_out, L, &c->fault,
+                                                                   &c->drain_fault, fail_at);
+    CMG_LAUNCH();
+}
+
+// Enqueues the three passes on device-resident SoA coordinates, the FP32 pass's list in
+// the segments of L (shaped for at least n queries). `loads`: the FP32 pass with per-thread
+// loads throughout (the rerun after a wait of the TMA-staged one ran out).
+static void pred_stream_enqueue(int npt, const double* const* coords, int64_t n, int mode, int8_t* d_out,
+                                Seg L, int64_t* list_b, Counters* c, cudaStream_t st, int sms,
+                                cudaEvent_t* fp32_events, bool loads) {
     Soa s{};
     for (int k = 0; k < 3 * npt; ++k) s.c[k] = coords[k];
-    Counters* c = static_cast<Counters*>(counters);
     L.cnt = c->seg;
     const int64_t T = (n + kTile - 1) / kTile;
     if ((T + L.nseg - 1) / L.nseg > L.segcap / kTile)
         throw std::logic_error("predicate stream: list segments too small for the stream");
     CMG_CUDA(cudaMemsetAsync(c, 0, sizeof(Counters), st));
-    // the TMA pass takes the whole tiles when every column starts on a 16-byte boundary
-    // (the bulk copies' rule); the rest, and unaligned columns, take the per-thread loads
-    bool aligned = true;
-    for (int k = 0; k < 3 * npt; ++k) aligned = aligned && (reinterpret_cast<uintptr_t>(coords[k]) % 16 == 0);
-    const int64_t ntiles = aligned ? n / kTile : 0;
+    // the TMA pass takes the whole tiles; the rest takes the per-thread loads
+    bool aligned = true, skew = false;
+    for (int k = 0; k < 3 * npt; ++k) {
+        aligned = aligned && reinterpret_cast<uintptr_t>(coords[k]) % 8 == 0;
+        skew = skew || reinterpret_cast<uintptr_t>(coords[k]) % 16 != 0;
+    }
+    const int64_t ntiles = aligned && !loads ? n / kTile : 0;
     if (fp32_events) CMG_CUDA(cudaEventRecord(fp32_events[0], st));
     if (ntiles > 0) {
         const int64_t fail_at = g_fail_wait_at.exchange(-1);
-        if (npt == 4) {
-            CMG_CUDA(cudaFuncSetAttribute(k_pred_fp32_tma<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(Tma<4>::kSmem)));
-            k_pred_fp32_tma<4><<<L.nseg, kTmaThreads, Tma<4>::kSmem, st>>>(s, ntiles, d_out, L, &c->fault,
-                                                                           &c->drain_fault, fail_at);
-        } else {
-            CMG_CUDA(cudaFuncSetAttribute(k_pred_fp32_tma<5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(Tma<5>::kSmem)));
-            k_pred_fp32_tma<5><<<L.nseg, kTmaThreads, Tma<5>::kSmem, st>>>(s, ntiles, d_out, L, &c->fault,
-                                                                           &c->drain_fault, fail_at);
-        }
-        CMG_LAUNCH();
+        if (npt == 4 && skew) pred_fp32_tma<4, true>(s, ntiles, d_out, L, c, fail_at, st);
+        else if (npt == 4) pred_fp32_tma<4, false>(s, ntiles, d_out, L, c, fail_at, st);
+        else if (skew) pred_fp32_tma<5, true>(s, ntiles, d_out, L, c, fail_at, st);
+        else pred_fp32_tma<5, false>(s, ntiles, d_out, L, c, fail_at, st);
     }
     if (ntiles < T) pred_fp32_loads(npt, s, ntiles, T, n, d_out, L, st);
     if (fp32_events) CMG_CUDA(cudaEventRecord(fp32_events[1], st));
-    int reruns = 0;
-    if (ntiles > 0) {
-        // a TMA wait that ran out (it never should) reruns the pass with per-thread loads,
-        // unless the copies in flight could not be drained either
-        unsigned long long fault[2] = {0, 0};
-        CMG_CUDA(cudaMemcpyAsync(fault, &c->fault, sizeof(fault), cudaMemcpyDeviceToHost, st));
+    pred_stream_finish(npt, s, mode, d_out, L, list_b, c, st, sms);
+}
+
+// Runs the three passes and reads the counts back into *h (all but the segments'),
+// synchronising once: the later passes are enqueued before it is known whether a TMA wait
+// of the FP32 pass ran out (it never should; they then work on a part of the list). If one
+// did, the passes run again with per-thread loads, unless the copies in flight could not
+// be drained either (an error). Returns the number of reruns (0 or 1).
+static int pred_stream_device(int npt, const double* const* coords, int64_t n, int mode, int8_t* d_out,
+                              Seg L, int64_t* list_b, Counters* c, Counters* h, cudaStream_t st, int sms,
+                              cudaEvent_t* fp32_events) {
+    for (int run = 0;; ++run) {
+        pred_stream_enqueue(npt, coords, n, mode, d_out, L, list_b, c, st, sms, fp32_events, run > 0);
+        CMG_CUDA(cudaMemcpyAsync(h, c, offsetof(Counters, seg), cudaMemcpyDeviceToHost, st));
         CMG_CUDA(cudaStreamSynchronize(st));
-        if (fault[1])
+        if (h->drain_fault)
             throw std::runtime_error(
                 "predicate stream: a bulk copy of the FP32 pass did not complete within its wait");
-        if (fault[0]) {
-            CMG_CUDA(cudaMemsetAsync(c, 0, sizeof(Counters), st));
-            pred_fp32_loads(npt, s, 0, T, n, d_out, L, st);
-            reruns = 1;
-        }
+        if (!h->fault) return run;
     }
-    pred_stream_finish(npt, s, mode, d_out, L, list_b, c, st, sms);
-    return reruns;
 }
 
 }  // namespace cmg::gpu
@@ -861,7 +888,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const int sms = device_sms();
         const bool host = where == CMG_MEM_HOST;
-        auto plan = [&](Arena& a, Seg* la, int64_t** lb, void** cnt) {
+        auto plan = [&](Arena& a, Seg* la, int64_t** lb, Counters** cnt) {
             a.reset();
             *la = take_seg(a, n, 3 * npt, sms, 2);
             *lb = a.take<int64_t>(n);
@@ -875,7 +902,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
         if (!host) {
             Seg la;
             int64_t* lb;
-            void* cnt;
+            Counters* cnt;
             w.arena.clear_need();
             plan(w.arena, &la, &lb, &cnt);
             if (w.arena.overflowed()) {
@@ -883,9 +910,7 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
                 plan(w.arena, &la, &lb, &cnt);
             }
             reruns += pred_stream_device(npt, coords, n, mode == CMG_PRED_EXACT ? kPredExact : kPredCompat,
-                                         reinterpret_cast<int8_t*>(out), la, lb, cnt, st, sms, w.ev);
-            CMG_CUDA(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
-            CMG_CUDA(cudaStreamSynchronize(st));
+                                         reinterpret_cast<int8_t*>(out), la, lb, cnt, &hc, st, sms, w.ev);
             if (stats) CMG_CUDA(cudaEventElapsedTime(&stats->fp32_pass_ms, w.ev[0], w.ev[1]));
         } else if (use_pull(w)) {
             // Host arrays read by the device through the host's page tables (the GPU
@@ -1015,21 +1040,20 @@ cmg_status run_stream(int npt, const double* const* coords, int64_t n, int mode,
                 if (c + 1 < nch) upload(c + 1);
                 const double* dc[15];
                 for (int k = 0; k < ncol; ++k) dc[k] = col[b][k];
+                Counters h{};
                 reruns += pred_stream_device(npt, dc, m, mode == CMG_PRED_EXACT ? kPredExact : kPredCompat,
-                                   sg[b], la, lb, cnt + c, st, sms, &w.chunk_ev[2 * c]);
+                                             sg[b], la, lb, cnt + c, &h, st, sms, &w.chunk_ev[2 * c]);
+                hc.n32 += h.n32;
+                hc.n64 += h.n64;
+                hc.certified += h.certified;
+                hc.expanded += h.expanded;
+                hc.overflow |= h.overflow;
                 CMG_CUDA(cudaMemcpyAsync(out + i0, sg[b], m, cudaMemcpyDeviceToHost, st));
                 CMG_CUDA(cudaEventRecord(w.done[b], st));
             }
-            std::vector<Counters> hcs(static_cast<size_t>(nch));
-            CMG_CUDA(cudaMemcpyAsync(hcs.data(), cnt, sizeof(Counters) * nch, cudaMemcpyDeviceToHost, st));
             CMG_CUDA(cudaStreamSynchronize(st));
             float total = 0.f;
             for (int64_t c = 0; c < nch; ++c) {
-                hc.n32 += hcs[c].n32;
-                hc.n64 += hcs[c].n64;
-                hc.certified += hcs[c].certified;
-                hc.expanded += hcs[c].expanded;
-                hc.overflow |= hcs[c].overflow;
                 float ms = 0.f;
                 CMG_CUDA(cudaEventElapsedTime(&ms, w.chunk_ev[2 * c], w.chunk_ev[2 * c + 1]));
                 total += ms;
@@ -1089,7 +1113,7 @@ cmg_status cmg_orient3d_signs(const double* xyz, int npts, const int* tets, int 
         const int64_t N = n;
         const int sms = device_sms();
         auto plan = [&](Arena& a, double** dx, int** dt, double** soa, int8_t** d8, int** dsg,
-                        Seg* la, int64_t** lb, void** cnt) {
+                        Seg* la, int64_t** lb, Counters** cnt) {
             a.reset();
             *dx = a.take<double>(3 * static_cast<size_t>(npts));
             *dt = a.take<int>(4 * N);
@@ -1105,7 +1129,7 @@ cmg_status cmg_orient3d_signs(const double* xyz, int npts, const int* tets, int 
         int8_t* d8;
         Seg la;
         int64_t* lb;
-        void* cnt;
+        Counters* cnt;
         w.arena.clear_need();
         plan(w.arena, &dx, &dt, &soa, &d8, &dsg, &la, &lb, &cnt);
         if (w.arena.overflowed()) {
@@ -1118,7 +1142,8 @@ cmg_status cmg_orient3d_signs(const double* xyz, int npts, const int* tets, int 
         CMG_LAUNCH();
         const double* cols[12];
         for (int k = 0; k < 12; ++k) cols[k] = soa + k * N;
-        pred_stream_device(4, cols, N, kPredCompat, d8, la, lb, cnt, st, sms, nullptr);
+        Counters h{};
+        pred_stream_device(4, cols, N, kPredCompat, d8, la, lb, cnt, &h, st, sms, nullptr);
         k_widen<<<static_cast<unsigned>((N + 255) / 256), 256, 0, st>>>(d8, N, dsg);
         CMG_LAUNCH();
         CMG_CUDA(cudaMemcpyAsync(out_sign, dsg, sizeof(int) * N, cudaMemcpyDeviceToHost, st));

@@ -36,3 +36,23 @@ def test_spans_match_oracle(cm, orc, kind, scale_exp):
         assert np.array_equal(got, orc.stream(kind, S, om))
         # some spans are beyond the wide integers, most are not
         assert st["expansion_queries"] < 0.4 * S.shape[1]
+
+
+@pytest.mark.parametrize("kind", ["orient3d", "insphere"])
+@pytest.mark.parametrize("n,first", [(255, 1), (257, 1), (1023, 0), (1025, 3), (70_001, 1)])
+def test_columns_off_a_16_byte_boundary(cm, orc, kind, n, first):
+    """Device columns whose starts are 0 or 8 bytes off a 16-byte boundary (rows of odd length
+    in one matrix, from an odd or even first value): the bulk copies read the words around
+    them and the signs equal the oracle's."""
+    import torch
+    import oracle as O
+    from cybermeshgenerator_gb300 import workloads as W
+    S = W.predicate_stream(n, kind, degenerate=0.1, near=0.1, seed=n)
+    d = torch.full((S.shape[0] * n + 8,), float("nan"), dtype=torch.float64, device="cuda")
+    d[first:first + S.size] = torch.from_numpy(S.ravel())
+    out = torch.zeros(n, dtype=torch.int8, device="cuda")
+    fn = cm.orient3d_stream if kind == "orient3d" else cm.insphere_stream
+    _, st = fn(([d.data_ptr() + 8 * (first + k * n) for k in range(S.shape[0])], n, out.data_ptr()),
+               cm.PRED_COMPAT, torch.cuda.current_stream().cuda_stream)
+    assert np.array_equal(out.cpu().numpy(), orc.stream(kind, S, O.COMPAT))
+    assert st["tma_reruns"] == 0
