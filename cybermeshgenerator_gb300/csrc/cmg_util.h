@@ -48,6 +48,11 @@ void exclusive_scan(const int* in, int64_t* out, int64_t n, int64_t* tmp, cudaSt
 void exclusive_scan(const int64_t* in, int64_t* out, int64_t n, int64_t* tmp, cudaStream_t st);
 size_t scan_tmp_elems(int64_t n);
 
+// order: 0 .. n-1 by descending count, to within an eighth (a work order). keys: n entries
+// of scratch; tmp: radix_sort_tmp_bytes(n).
+void order_descending(const int* count, int64_t n, uint32_t* order, uint32_t* keys, void* tmp,
+                      cudaStream_t st);
+
 // Stable LSD radix sort of (key, value) pairs on the low key_bits bits, in place.
 size_t radix_sort_tmp_bytes(int64_t n);
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, void* tmp,

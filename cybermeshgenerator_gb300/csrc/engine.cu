@@ -240,7 +240,7 @@ struct Batch::Impl {
     int64_t* bin_off = nullptr;
     int* bin_list = nullptr;
     int* large_cnt = nullptr;
-    int64_t* large_off = nullptr;
+    char* zero_end = nullptr;  // end of the counters that start at zero (from the stats)
     int* large_list = nullptr;
     unsigned* emax_bits = nullptr;
     float* bound = nullptr;
@@ -321,13 +321,20 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         pts_ = carve<double>(A, 3 * npts_);
         tris_ = carve<int>(A, 3 * ntris_);
         dsegs_ = carve<MeshSeg>(A, nseg);
+        // counters that start at zero, next to each other (one memset per run)
         stats_ = carve<Stats>(A, 1);
         queue_ = carve<unsigned long long>(A, 1);
+        impl_->colcnt = carve<int>(A, ncol_);
+        if (sdf) {
+            impl_->bincnt = carve<int>(A, nbrick_);
+            impl_->large_cnt = carve<int>(A, 2 * nseg);
+            impl_->emax_bits = carve<unsigned>(A, 3 * nseg);  // emax, scale, emax_all
+        }
+        impl_->zero_end = carve<char>(A, 1);
         impl_->soup = carve<double>(A, kSoupStride * ntris_);
         impl_->xybox = carve<int4>(A, ntris_);
         impl_->pairs_n = carve<int64_t>(A, ntris_ + 1);
         impl_->pair_off = carve<int64_t>(A, ntris_ + 1);
-        impl_->colcnt = carve<int>(A, ncol_);
         impl_->col_off = carve<int64_t>(A, ncol_ + 1);
         impl_->flagged = carve<int64_t>(A, ncol_);
         int64_t smax = std::max(std::max(ntris_, ncol_), std::max(nbrick_, int64_t(nseg)));
@@ -342,21 +349,17 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
             impl_->tlo = carve<float4>(A, ntris_);
             impl_->thi = carve<float4>(A, ntris_);
             impl_->tbin = carve<int64_t>(A, ntris_);
-            impl_->bincnt = carve<int>(A, nbrick_);
             impl_->bin_off = carve<int64_t>(A, nbrick_ + 1);
             impl_->bin_list = carve<int>(A, ntris_);
-            impl_->large_cnt = carve<int>(A, 2 * nseg);
-            impl_->large_off = carve<int64_t>(A, nseg + 1);
             impl_->large_list = carve<int>(A, ntris_);
-            impl_->emax_bits = carve<unsigned>(A, 3 * nseg);  // emax, scale, emax_all
             impl_->bound = carve<float>(A, nbrick_);
             impl_->bound_tri = carve<int>(A, nbrick_);
             impl_->cand_cnt = carve<int>(A, nbrick_);
             impl_->cand_off = carve<int64_t>(A, nbrick_ + 1);
             impl_->brick_emax = carve<float>(A, nbrick_);
-            impl_->work_keys = carve<uint32_t>(A, nwork_);
-            impl_->work = carve<uint32_t>(A, nwork_);
-            impl_->sort_tmp = carve<char>(A, radix_sort_tmp_bytes(nwork_));
+            impl_->work_keys = carve<uint32_t>(A, nbrick_);
+            impl_->work = carve<uint32_t>(A, nbrick_);
+            impl_->sort_tmp = carve<char>(A, radix_sort_tmp_bytes(nbrick_));
         }
         if (commit) return;
     };
@@ -502,7 +505,7 @@ void Batch::run_impl(bool sizing) {
     }
     if (timed) CMG_CUDA(cudaEventRecord(ev_[0], st));
 
-    CMG_CUDA(cudaMemsetAsync(stats_, 0, sizeof(Stats), st));
+    CMG_CUDA(cudaMemsetAsync(stats_, 0, static_cast<size_t>(I.zero_end - reinterpret_cast<char*>(stats_)), st));
     launch_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.soup, I.xybox, I.pairs_n, st);
 
     // Ray-parity occupancy: (triangle, column) pairs, filter, exact pass. The pair count
@@ -530,11 +533,9 @@ void Batch::run_impl(bool sizing) {
     };
     auto occ_tail = [&](cudaStream_t s) {
         const int pair_grid = 4 * device_sms();
-        CMG_CUDA(cudaMemsetAsync(I.colcnt, 0, sizeof(int) * std::max<int64_t>(ncol_, 1), s));
         launch_col_pairs(false, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, nullptr, nullptr,
                          pair_grid, s);
         exclusive_scan(I.colcnt, I.col_off, ncol_, I.scan_tmp, s);
-        CMG_CUDA(cudaMemsetAsync(I.colcnt, 0, sizeof(int) * std::max<int64_t>(ncol_, 1), s));
         launch_col_pairs(true, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, I.col_off,
                          I.col_list, pair_grid, s);
         launch_occ_filter(opts_.predicates, dsegs_, nseg, nrow_, I.soup, I.col_off, I.col_list, occ,
@@ -558,16 +559,10 @@ void Batch::run_impl(bool sizing) {
     int64_t* tmp = I.scan_tmp_side;
     auto prep_head = [&]() {
         if (timed) CMG_CUDA(cudaEventRecord(ev_[4], ss));
-        CMG_CUDA(cudaMemsetAsync(I.bincnt, 0, sizeof(int) * nbrick_, ss));
-        CMG_CUDA(cudaMemsetAsync(I.large_cnt, 0, sizeof(int) * 2 * nseg, ss));
-        CMG_CUDA(cudaMemsetAsync(I.emax_bits, 0, sizeof(unsigned) * 3 * nseg, ss));
         launch_sdf_tri_prep(dsegs_, nseg, ntris_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.tnorm, I.tlo,
                             I.thi, I.tbin, I.bincnt, I.large_cnt, I.emax_bits, ss);
         exclusive_scan(I.bincnt, I.bin_off, nbrick_, tmp, ss);
-        exclusive_scan(I.large_cnt, I.large_off, nseg, tmp, ss);
-        launch_seg_finish(dsegs_, nseg, I.large_off, I.emax_bits, ss);
-        CMG_CUDA(cudaMemsetAsync(I.bincnt, 0, sizeof(int) * nbrick_, ss));
-        CMG_CUDA(cudaMemsetAsync(I.large_cnt + nseg, 0, sizeof(int) * nseg, ss));
+        launch_seg_finish(dsegs_, nseg, I.large_cnt, I.emax_bits, ss);
         launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.bin_list, dsegs_, nseg,
                         I.large_cnt + nseg, I.large_list, ss);
         launch_brick_walk(false, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
@@ -598,10 +593,7 @@ void Batch::run_impl(bool sizing) {
         launch_brick_walk(true, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
                           I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, I.cand_off, I.cand,
                           I.cand_c, I.brick_emax, stats_, opts_.walk_warps, ss);
-        if (opts_.brick == 16) launch_sub_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);
-        else launch_work_keys(I.cand_cnt, nbrick_, I.work_keys, I.work, ss);
-        radix_sort_pairs(I.work_keys, I.work, nwork_, 32, I.sort_tmp, ss);
-        CMG_CUDA(cudaMemsetAsync(queue_, 0, sizeof(unsigned long long), ss));
+        order_descending(I.cand_cnt, nbrick_, I.work, I.work_keys, I.sort_tmp, ss);
         if (timed) CMG_CUDA(cudaEventRecord(ev_[5], ss));
     };
 

@@ -42,7 +42,7 @@ void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const dou
 void launch_bin_fill(int64_t ntris, const int64_t* tbin, const int64_t* bin_off, int* bincur,
                      int* bin_list, const MeshSeg* segs, int nseg, int* large_cur, int* large_list,
                      cudaStream_t st);
-void launch_seg_finish(MeshSeg* segs, int nseg, const int64_t* large_off, const unsigned* emax_bits,
+void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsigned* emax_bits,
                        cudaStream_t st);
 // cand_c (null: not wanted): per candidate, its centroid from the brick's centre and radius.
 void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
@@ -57,8 +57,6 @@ void launch_count_K(int brick, const MeshSeg* segs, int nseg, int64_t nbricks, c
                     const int64_t* cand_off, const int* cand, const double* sdf64,
                     const float* sdf32, float band_cells, unsigned long long* out,
                     cudaStream_t st);
-void launch_work_keys(const int* cand_cnt, int64_t n, uint32_t* keys, uint32_t* vals,
-                      cudaStream_t st);
 void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, const uint32_t* work,
                      int64_t nwork, unsigned long long* queue, const double* soup,
                      const float4* tinfo, const int64_t* cand_off, const int* cand,
@@ -66,9 +64,8 @@ void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, co
                      double* sdf64, int* near_tri, uint8_t* near_reg, float* errbound, Stats* stats,
                      int grid, cudaStream_t st);
 
-// sdf_sub.cu: the work order of the 4^3 sub-bricks of 16^3 candidate bricks; plain FP64.
-void launch_sub_work_keys(const int* cand_cnt, int64_t nbricks, uint32_t* keys, uint32_t* vals,
-                          cudaStream_t st);
+// sdf_sub.cu: evaluation by 4^3 sub-bricks of 16^3 candidate bricks. work: the bricks in
+// work order; nwork = 64 sub-bricks each.
 // ctas: resident CTAs per SM of the evaluation kernel (16, or 12 for any other value).
 int sdf_sub_minb(int ctas);
 int sdf_sub_grid(int ctas);

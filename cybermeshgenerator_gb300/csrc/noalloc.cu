@@ -196,7 +196,6 @@ extern "C" cmg_status cmg_gpu_occupancy_static(const double* d_points, int64_t n
         CMG_CUDA(cudaMemsetAsync(colcnt, 0, sizeof(int) * ncol, st));
         launch_col_pairs(false, segs, 1, T, xybox, pair_off, colcnt, nullptr, nullptr, grid, st);
         exclusive_scan(colcnt, col_off, ncol, scan_tmp, st);
-        CMG_CUDA(cudaMemsetAsync(colcnt, 0, sizeof(int) * ncol, st));
         launch_col_pairs(true, segs, 1, T, xybox, pair_off, colcnt, col_off, col_list, grid, st);
         launch_occ_filter(predicates, segs, 1, nrows, soup, col_off, col_list, d_occupancy, flagged,
                           stats, st);

@@ -144,7 +144,8 @@ __global__ void k_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64_t n
     pairs[t] = static_cast<int64_t>(i1 - i0 + 1) * (j1 - j0 + 1);
 }
 
-// FILL=false: count bucket sizes; FILL=true: write bucket entries.
+// FILL=false: count bucket sizes into the zeroed colcnt; FILL=true: write bucket entries,
+// taking the counts down to zero again.
 template <bool FILL>
 __global__ void k_col_pairs(const MeshSeg* __restrict__ segs, int nseg, int64_t ntris,
                             const int4* __restrict__ xybox, const int64_t* __restrict__ pair_off,
@@ -162,8 +163,8 @@ __global__ void k_col_pairs(const MeshSeg* __restrict__ segs, int nseg, int64_t 
         int i = bx.x + static_cast<int>(local % w);
         int j = bx.z + static_cast<int>(local / w);
         int64_t col = s.col_begin + static_cast<int64_t>(j) * s.g.nx + i;
-        int slot = atomicAdd(&colcnt[col], 1);
-        if (FILL) col_list[col_off[col] + slot] = static_cast<int>(t);
+        if (FILL) col_list[col_off[col] + atomicSub(&colcnt[col], 1) - 1] = static_cast<int>(t);
+        else atomicAdd(&colcnt[col], 1);
     }
 }
 

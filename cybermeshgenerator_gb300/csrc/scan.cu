@@ -73,11 +73,22 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int64_t* __restrict_
     if (threadIdx.x == 0) sums[m] = carry;
 }
 
-template <typename T>
+// The scan of a tile. SCANNED: sums holds the tile sums' exclusive prefix; else the sums
+// themselves, and each block adds up those before its own.
+template <typename T, bool SCANNED>
 __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const T* __restrict__ in, int64_t n,
                                                             const int64_t* __restrict__ sums,
                                                             int64_t* __restrict__ out) {
     __shared__ int64_t sh[kScanThreads / 32];
+    int64_t before = 0, own = 0;
+    if (SCANNED) {
+        before = sums[blockIdx.x];
+    } else {
+        int64_t s = 0;
+        for (int64_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) s += sums[b];
+        block_exclusive<int64_t>(s, sh, &before);
+        own = sums[blockIdx.x];
+    }
     int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
     int64_t v[kScanItems];
     int64_t s = 0;
@@ -86,14 +97,46 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const T* __restrict_
         v[i] = base + i < n ? static_cast<int64_t>(in[base + i]) : 0;
         s += v[i];
     }
-    int64_t before = block_exclusive<T>(s, sh, nullptr) + sums[blockIdx.x];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = SCANNED ? sums[gridDim.x] : before + own;
+    before += block_exclusive<T>(s, sh, nullptr);
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
         if (base + i < n) out[base + i] = before;
         before += v[i];
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = sums[gridDim.x];
 }
+
+// A whole scan in one block, tile by tile.
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(const T* __restrict__ in, int64_t n,
+                                                           int64_t* __restrict__ out) {
+    __shared__ int64_t sh[kScanThreads / 32];
+    int64_t carry = 0;
+    for (int64_t tile = 0; tile < n; tile += kScanTile) {
+        const int64_t base = tile + threadIdx.x * kScanItems;
+        int64_t v[kScanItems];
+        int64_t s = 0;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = base + i < n ? static_cast<int64_t>(in[base + i]) : 0;
+            s += v[i];
+        }
+        int64_t total;
+        int64_t before = carry + block_exclusive<T>(s, sh, &total);
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            if (base + i < n) out[base + i] = before;
+            before += v[i];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
+// Launches set the time of a short scan (about 2 us each beside a small call's 0.35 ms): up
+// to 4 tiles one block does it all (1 launch), up to 4096 every block adds up the tile
+// sums before its own (2), beyond one block scans the sums (3).
+constexpr int64_t kOneBlockTiles = 4, kAddedTiles = 4096;
 
 template <typename T>
 void exclusive_scan_impl(const T* in, int64_t* out, int64_t n, int64_t* tmp, cudaStream_t st) {
@@ -102,11 +145,64 @@ void exclusive_scan_impl(const T* in, int64_t* out, int64_t n, int64_t* tmp, cud
         cudaMemsetAsync(out, 0, sizeof(int64_t), st);
         return;
     }
-    k_tile_sums<T><<<static_cast<unsigned>(tiles), kScanThreads, 0, st>>>(in, n, tmp);
-    k_scan_sums<<<1, kScanThreads, 0, st>>>(tmp, tiles);
-    k_tile_scan<T><<<static_cast<unsigned>(tiles), kScanThreads, 0, st>>>(in, n, tmp, out);
-    note_launch(2);
+    const unsigned grid = static_cast<unsigned>(tiles);
+    if (tiles <= kOneBlockTiles) {
+        k_scan_one<T><<<1, kScanThreads, 0, st>>>(in, n, out);
+    } else {
+        k_tile_sums<T><<<grid, kScanThreads, 0, st>>>(in, n, tmp);
+        note_launch();
+        if (tiles <= kAddedTiles) {
+            k_tile_scan<T, false><<<grid, kScanThreads, 0, st>>>(in, n, tmp, out);
+        } else {
+            k_scan_sums<<<1, kScanThreads, 0, st>>>(tmp, tiles);
+            note_launch();
+            k_tile_scan<T, true><<<grid, kScanThreads, 0, st>>>(in, n, tmp, out);
+        }
+    }
     CMG_LAUNCH();
+}
+
+// Numbers 0 .. n-1 by descending count, to within an eighth (the count's exponent and top
+// three bits): the 256 keys of a counting sort.
+__device__ __forceinline__ unsigned order_key(int count) {
+    return 255u - min(255u, (__float_as_uint(static_cast<float>(count) + 1.f) >> 20) - 1016u);
+}
+constexpr int kOrderThreads = 1024;
+constexpr int64_t kOrderOne = 32768;
+__global__ void __launch_bounds__(kOrderThreads) k_order_one(const int* __restrict__ count, int n,
+                                                             uint32_t* __restrict__ order) {
+    __shared__ int start[256];
+    __shared__ int warp_sum[8];
+    const int tid = threadIdx.x;
+    if (tid < 256) start[tid] = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += kOrderThreads) atomicAdd(&start[order_key(count[i])], 1);
+    __syncthreads();
+    int v = 0, x = 0;
+    if (tid < 256) {
+        x = v = start[tid];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((tid & 31) >= o) x += y;
+        }
+        if ((tid & 31) == 31) warp_sum[tid >> 5] = x;
+    }
+    __syncthreads();
+    if (tid < 256) {
+        for (int w = 0; w < (tid >> 5); ++w) x += warp_sum[w];
+        start[tid] = x - v;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kOrderThreads)
+        order[atomicAdd(&start[order_key(count[i])], 1)] = static_cast<uint32_t>(i);
+}
+__global__ void k_order_keys(const int* __restrict__ count, int64_t n, uint32_t* __restrict__ keys,
+                             uint32_t* __restrict__ order) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    keys[i] = order_key(count[i]);
+    order[i] = static_cast<uint32_t>(i);
 }
 
 // ------------------------------------------------------------------ radix sort
@@ -183,6 +279,19 @@ void exclusive_scan(const int64_t* in, int64_t* out, int64_t n, int64_t* tmp, cu
     exclusive_scan_impl<int64_t>(in, out, n, tmp, st);
 }
 size_t scan_tmp_elems(int64_t n) { return static_cast<size_t>((n + kScanTile - 1) / kScanTile + 2); }
+
+void order_descending(const int* count, int64_t n, uint32_t* order, uint32_t* keys, void* tmp,
+                      cudaStream_t st) {
+    if (n <= 0) return;
+    if (n <= kOrderOne) {
+        k_order_one<<<1, kOrderThreads, 0, st>>>(count, static_cast<int>(n), order);
+        CMG_LAUNCH();
+        return;
+    }
+    k_order_keys<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(count, n, keys, order);
+    CMG_LAUNCH();
+    radix_sort_pairs(keys, order, n, 8, tmp, st);
+}
 
 size_t radix_sort_tmp_bytes(int64_t n) {
     int64_t ntiles = (n + kSortTile - 1) / kSortTile;

@@ -205,7 +205,7 @@ __global__ void k_bin_fill(int64_t ntris, const int64_t* __restrict__ tbin,
     if (t >= ntris) return;
     int64_t b = tbin[t];
     if (b >= 0) {
-        int slot = atomicAdd(&bincur[b], 1);
+        int slot = atomicSub(&bincur[b], 1) - 1;  // the counts, taken down to zero
         bin_list[bin_off[b] + slot] = static_cast<int>(t);
     } else {
         const int si = find_seg<&MeshSeg::tri_begin>(segs, nseg, t);
@@ -214,21 +214,45 @@ __global__ void k_bin_fill(int64_t ntris, const int64_t* __restrict__ tbin,
     }
 }
 
-// Writes each mesh's always-considered range, emax and coordinate scale (the
+// Scans the meshes' always-considered counts (one block) and writes each mesh's range, emax and coordinate scale (the
 // larger of max |v - K| over its points and the grid extent, with 1e-4 slack)
 // into its segment.
-__global__ void k_seg_finish(MeshSeg* segs, int nseg, const int64_t* __restrict__ large_off,
-                             const unsigned* __restrict__ emax_bits) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nseg) return;
-    segs[i].large_begin = large_off[i];
-    segs[i].large_end = large_off[i + 1];
-    segs[i].emax = __uint_as_float(emax_bits[i]);
-    segs[i].emax_all = __uint_as_float(emax_bits[2 * nseg + i]);
-    const GridDesc& g = segs[i].g;
-    const double ext = g.h * static_cast<double>(max(g.nx, max(g.ny, g.nz)));
-    const double sc = fmax(static_cast<double>(__uint_as_float(emax_bits[nseg + i])), ext);
-    segs[i].scale = __double2float_ru(sc * 1.0001);
+constexpr int kSegThreads = 128;
+__global__ void __launch_bounds__(kSegThreads) k_seg_finish(MeshSeg* segs, int nseg, const int* __restrict__ large_cnt,
+                                                            const unsigned* __restrict__ emax_bits) {
+    __shared__ int64_t s_w[kSegThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for (int i0 = 0; i0 < nseg; i0 += kSegThreads) {
+        const int i = i0 + threadIdx.x;
+        const int64_t n = i < nseg ? large_cnt[i] : 0;
+        int64_t end = n;  // inclusive prefix
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += y;
+        }
+        if (lane == 31) s_w[warp] = end;
+        __syncthreads();
+        int64_t total = 0;
+#pragma unroll
+        for (int w = 0; w < kSegThreads / 32; ++w) {
+            if (w < warp) end += s_w[w];
+            total += s_w[w];
+        }
+        __syncthreads();
+        end += carry;
+        carry += total;
+        if (i >= nseg) continue;
+        segs[i].large_begin = end - n;
+        segs[i].large_end = end;
+        segs[i].emax = __uint_as_float(emax_bits[i]);
+        segs[i].emax_all = __uint_as_float(emax_bits[2 * nseg + i]);
+        const GridDesc& g = segs[i].g;
+        const double ext = g.h * static_cast<double>(max(g.nx, max(g.ny, g.nz)));
+        const double sc = fmax(static_cast<double>(__uint_as_float(emax_bits[nseg + i])), ext);
+        segs[i].scale = __double2float_ru(sc * 1.0001);
+    }
 }
 
 // ------------------------------------------------------------------ brick geometry
@@ -1098,16 +1122,6 @@ k_count_K(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
     }
 }
 
-// LPT order of the bricks: key = ~count so an ascending sort puts the most
-// expensive bricks first.
-__global__ void k_work_keys(const int* __restrict__ cand_cnt, int64_t n, uint32_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals) {
-    int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    keys[b] = ~static_cast<uint32_t>(cand_cnt[b]);
-    vals[b] = static_cast<uint32_t>(b);
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
@@ -1132,9 +1146,9 @@ void launch_bin_fill(int64_t ntris, const int64_t* tbin, const int64_t* bin_off,
     CMG_LAUNCH();
 }
 
-void launch_seg_finish(MeshSeg* segs, int nseg, const int64_t* large_off, const unsigned* emax_bits,
+void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsigned* emax_bits,
                        cudaStream_t st) {
-    k_seg_finish<<<(nseg + 127) / 128, 128, 0, st>>>(segs, nseg, large_off, emax_bits);
+    k_seg_finish<<<1, kSegThreads, 0, st>>>(segs, nseg, large_cnt, emax_bits);
     CMG_LAUNCH();
 }
 
@@ -1193,13 +1207,6 @@ void launch_count_K(int brick, const MeshSeg* segs, int nseg, int64_t nbricks, c
     else
         k_count_K<8, 128><<<static_cast<unsigned>(nbricks), 128, 0, st>>>(
             segs, nseg, nbricks, tinfo, cand_off, cand, sdf64, sdf32, band_cells, out);
-    CMG_LAUNCH();
-}
-
-void launch_work_keys(const int* cand_cnt, int64_t n, uint32_t* keys, uint32_t* vals,
-                      cudaStream_t st) {
-    if (n == 0) return;
-    k_work_keys<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(cand_cnt, n, keys, vals);
     CMG_LAUNCH();
 }
 

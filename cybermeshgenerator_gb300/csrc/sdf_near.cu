@@ -209,14 +209,14 @@ struct Shared {
 };
 
 // One sub-brick: by this warp alone, or (COOP) by the CTA's warps together, each over its
-// part of the list.
+// part of the list. item: sub-brick of the queue.
 template <int PREC, bool COOP>
-__device__ __forceinline__ void sub_brick(const Args& g, const uint32_t w, WarpMem& M, Shared& S,
+__device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, WarpMem& M, Shared& S,
                                           const WarpMem* all) {
     constexpr bool EXACT = PREC == kPrecExact;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
-    const int64_t gb = static_cast<int64_t>(w >> 6);
+    const int64_t gb = g.work[item >> 6];  // the bricks in order, 64 sub-bricks each
     const MeshSeg& s = g.segs[find_seg<&MeshSeg::brick_begin>(g.segs, g.nseg, gb)];
     float px, py;
     Cell A, B;
@@ -224,7 +224,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const uint32_t w, WarpM
     //      per warp instruction), the others get it by shuffles
     float hx, hy, hz;
     {
-        const SubGeo q = sub_geo(s, gb - s.brick_begin, static_cast<int>(w & 63u));
+        const SubGeo q = sub_geo(s, gb - s.brick_begin, static_cast<int>(item & 63));
         if (q.empty) return;
         const double h = s.g.h;
         const int a = lane < 12 ? lane >> 2 : min(lane - 12, 2), i = lane & 3;
@@ -568,8 +568,8 @@ __device__ __forceinline__ void sub_brick(const Args& g, const uint32_t w, WarpM
 // longest lists a loose bound, 7.1 ms before they were shared).
 // The queue's first sub-bricks, those whose lists are long beside a warp's share of all the
 // work, are shared by a CTA's warps, each taking a quarter of the list (the minima over the
-// parts are the minimum over the list); the lists only get shorter, so the first light one
-// ends the sharing. With few sub-bricks in all, every one is shared. (128^3 grid around 65k
+// parts are the minimum over the list); the lists get shorter (to within an eighth), so the
+// first light one ends the sharing. With few sub-bricks in all, every one is shared. (128^3 grid around 65k
 // triangles: 3.1 -> 1.4 ms, the warp with the longest list had ended last; 63^3 around 1280
 // triangles, all shared: 0.28 -> 0.19 ms.)
 template <int PREC>
@@ -593,13 +593,13 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
         __syncthreads();
         item = static_cast<int64_t>(S.grab) * g.grab_n;
         if (item >= g.nwork) break;
-        const int64_t b = g.work[item] >> 6;
+        const int64_t b = g.work[item >> 6];
         if (static_cast<float>(g.cand_off[b + 1] - g.cand_off[b]) < heavy) {
             own = wid == 0;
             break;
         }
         for (int k = 0; k < g.grab_n && item + k < g.nwork; ++k)
-            sub_brick<PREC, true>(g, g.work[item + k], M, S, all);
+            sub_brick<PREC, true>(g, item + k, M, S, all);
     }
     for (;;) {
         if (!own) {
@@ -610,7 +610,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
         own = false;
         if (item >= g.nwork) break;
         for (int k = 0; k < g.grab_n && item + k < g.nwork; ++k)
-            sub_brick<PREC, false>(g, g.work[item + k], M, S, all);
+            sub_brick<PREC, false>(g, item + k, M, S, all);
     }
     if (lane == 0) {
         // a triangle evaluated for a sub-brick counts its 64 cells

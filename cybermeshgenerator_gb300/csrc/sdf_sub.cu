@@ -71,9 +71,8 @@ k_sdf_sub(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict
       for (int gi = 0; gi < grab_n; ++gi) {
         const int64_t item = grab * grab_n + gi;
         if (item >= nwork) break;
-        const uint32_t w = work[item];
-        const int64_t gb = static_cast<int64_t>(w >> 6);
-        const int sub = static_cast<int>(w & 63u);
+        const int64_t gb = work[item >> 6];  // the bricks in order, 64 sub-bricks each
+        const int sub = static_cast<int>(item & 63);
         const MeshSeg& s = segs[find_seg<&MeshSeg::brick_begin>(segs, nseg, gb)];
         const GridDesc g = s.g;
         const SubGeo q = sub_geo(s, gb - s.brick_begin, sub);
@@ -260,25 +259,7 @@ k_sdf_sub(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict
     }
 }
 
-// Work ids of the sub-bricks (brick * 64 + sub) in LPT order: key = ~brick count.
-__global__ void k_sub_work_keys(const int* __restrict__ cand_cnt, int64_t nbricks,
-                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (w >= nbricks * 64) return;
-    keys[w] = ~static_cast<uint32_t>(cand_cnt[w >> 6]);
-    vals[w] = static_cast<uint32_t>(w);
-}
-
 }  // namespace
-
-void launch_sub_work_keys(const int* cand_cnt, int64_t nbricks, uint32_t* keys, uint32_t* vals,
-                          cudaStream_t st) {
-    if (nbricks == 0) return;
-    const int64_t n = nbricks * 64;
-    k_sub_work_keys<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(cand_cnt, nbricks, keys,
-                                                                           vals);
-    CMG_LAUNCH();
-}
 
 // Resident CTAs per SM targeted by the evaluation kernel: 16 when asked for, else 12.
 int sdf_sub_minb(int ctas) { return ctas == 16 ? 16 : 12; }
