@@ -38,6 +38,8 @@ struct MeshSeg {
     int bnx, bny, bnz;              // bricks per axis (along z: those overlapping the slab)
     int bzo;                        // brick layer of the mesh's first brick (the slab's)
     int brick;                      // brick edge in cells
+    int walk_warps;                 // warps per brick of the candidate walk
+    int64_t walk_begin;             // the walk's CTAs
     int64_t large_begin, large_end; // always-considered triangles (global list)
     float emax;                     // max centroid-to-vertex distance of binned triangles
     float emax_all;                 // the same over all the mesh's triangles

@@ -243,10 +243,11 @@ struct Batch::Impl {
     char* zero_end = nullptr;  // end of the counters that start at zero (from the stats)
     int* large_list = nullptr;
     unsigned* emax_bits = nullptr;
-    float* bound = nullptr;
-    int* bound_tri = nullptr;  // the triangle that gave the bound
+    float4* bin_info = nullptr;
+    float4* bin_ball = nullptr;
+    float* bin_reach = nullptr;
     int* cand_cnt = nullptr;
-    int64_t* cand_off = nullptr;
+    int64_t* cand_rng = nullptr;
     float* brick_emax = nullptr;
     uint32_t* work_keys = nullptr;
     uint32_t* work = nullptr;
@@ -313,6 +314,12 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     if (nwork_ >= (int64_t(1) << 32)) throw std::invalid_argument("voxelize: grid too large");
     const int nseg = static_cast<int>(segs_.size());
     const bool sdf = opts_.want_sdf32 || opts_.want_sdf64 || opts_.want_near;
+    for (MeshSeg& s : segs_) {
+        const int64_t n = static_cast<int64_t>(s.bnx) * s.bny * s.bnz;
+        s.walk_warps = brick_walk_warps(nbrick_, n, s.tri_end - s.tri_begin, opts_.walk_warps);
+        s.walk_begin = nwalk_;
+        nwalk_ += brick_walk_ctas(n, s.walk_warps);
+    }
 
     // ---- fixed workspace
     Arena& A = impl_->fixed;
@@ -352,10 +359,11 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
             impl_->bin_off = carve<int64_t>(A, nbrick_ + 1);
             impl_->bin_list = carve<int>(A, ntris_);
             impl_->large_list = carve<int>(A, ntris_);
-            impl_->bound = carve<float>(A, nbrick_);
-            impl_->bound_tri = carve<int>(A, nbrick_);
+            impl_->bin_info = carve<float4>(A, ntris_);
+            impl_->bin_ball = carve<float4>(A, nbrick_);
+            impl_->bin_reach = carve<float>(A, nbrick_);
             impl_->cand_cnt = carve<int>(A, nbrick_);
-            impl_->cand_off = carve<int64_t>(A, nbrick_ + 1);
+            impl_->cand_rng = carve<int64_t>(A, 2 * nbrick_);
             impl_->brick_emax = carve<float>(A, nbrick_);
             impl_->work_keys = carve<uint32_t>(A, nbrick_);
             impl_->work = carve<uint32_t>(A, nbrick_);
@@ -456,9 +464,10 @@ void Batch::update_points_device(const double* d_pts) {
 // drops the captured graph when a grown arena moved the buffers it refers to.
 void Batch::sized_run() {
     const size_t pc = impl_->pairs.capacity(), cc = impl_->cands.capacity();
+    const int64_t cap = cand_cap_;
     run_impl(true);
     resize_ = false;
-    if ((impl_->pairs.capacity() != pc || impl_->cands.capacity() != cc) && graph_) {
+    if ((impl_->pairs.capacity() != pc || impl_->cands.capacity() != cc || cand_cap_ != cap) && graph_) {
         CMG_CUDA(cudaStreamSynchronize(stream_));
         CMG_CUDA(cudaGraphExecDestroy(graph_));
         graph_ = nullptr;
@@ -563,36 +572,45 @@ void Batch::run_impl(bool sizing) {
                             I.thi, I.tbin, I.bincnt, I.large_cnt, I.emax_bits, ss);
         exclusive_scan(I.bincnt, I.bin_off, nbrick_, tmp, ss);
         launch_seg_finish(dsegs_, nseg, I.large_cnt, I.emax_bits, ss);
-        launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.bin_list, dsegs_, nseg,
-                        I.large_cnt + nseg, I.large_list, ss);
-        launch_brick_walk(false, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
-                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, nullptr, nullptr, nullptr, nullptr,
-                          stats_, opts_.walk_warps, ss);
-        exclusive_scan(I.cand_cnt, I.cand_off, nbrick_, tmp, ss);
+        launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.tinfo, I.bin_list, I.bin_info, nbrick_,
+                        I.bin_ball, I.bin_reach, dsegs_, nseg, I.large_cnt + nseg, I.large_list, ss);
     };
+    auto walk = [&]() {
+        launch_brick_walk(dsegs_, nseg, nwalk_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off, I.bin_list,
+                          I.bin_info, I.bin_ball, I.bin_reach, I.large_list, I.cand_cnt, I.cand_rng, I.cand,
+                          I.cand_c, cand_cap_, I.brick_emax, stats_, ss);
+    };
+    const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
+    auto plan_cands = [&](size_t n) {
+        I.cands.reset();
+        I.cand = carve<int>(I.cands, n);
+        I.cand_c = near_list ? carve<float4>(I.cands, n) : nullptr;
+        cand_cap_ = static_cast<int64_t>(n);
+    };
+    // the first sizing run walks into whatever the arena holds (a pooled one is seldom empty)
+    if (sizing && cand_cap_ < 0) {
+        const size_t each = near_list ? 20 : 4, have = I.cands.capacity();
+        plan_cands(have > 4096 ? (have - 1024) / each : 0);
+    }
+    // reads the walk's total back; lists that did not fit are sized (with an eighth to
+    // spare, for points that move) and walked again
     auto prep_size = [&]() {
-        int64_t C = 0;
-        CMG_CUDA(cudaMemcpyAsync(&C, I.cand_off + nbrick_, sizeof(int64_t), cudaMemcpyDeviceToHost, ss));
+        unsigned long long C = 0;
+        CMG_CUDA(cudaMemcpyAsync(&C, &stats_->candidates, sizeof(C), cudaMemcpyDeviceToHost, ss));
         CMG_CUDA(cudaStreamSynchronize(ss));
-        Arena& Cn = I.cands;
-        const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
-        auto planc = [&]() {
-            Cn.reset();
-            I.cand = carve<int>(Cn, C);
-            I.cand_c = near_list ? carve<float4>(Cn, C) : nullptr;
-        };
-        Cn.clear_need();
-        planc();
-        if (Cn.overflowed()) {
-            Cn.reserve(Cn.need());
-            planc();
+        if (static_cast<int64_t>(C) <= cand_cap_) return;
+        const size_t n = static_cast<size_t>(C + C / 8);
+        I.cands.clear_need();
+        plan_cands(n);
+        if (I.cands.overflowed()) {
+            cand_cap_ = 0;  // a failed allocation leaves no list
+            I.cands.reserve(I.cands.need());
+            plan_cands(n);
         }
-        cand_cap_ = C;
+        CMG_CUDA(cudaMemsetAsync(&stats_->candidates, 0, sizeof(C), ss));
+        walk();
     };
     auto prep_tail = [&]() {
-        launch_brick_walk(true, dsegs_, nseg, nbrick_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off,
-                          I.bin_list, I.large_list, I.bound, I.bound_tri, I.cand_cnt, I.cand_off, I.cand,
-                          I.cand_c, I.brick_emax, stats_, opts_.walk_warps, ss);
         order_descending(I.cand_cnt, nbrick_, I.work, I.work_keys, I.sort_tmp, ss);
         if (timed) CMG_CUDA(cudaEventRecord(ev_[5], ss));
     };
@@ -603,6 +621,7 @@ void Batch::run_impl(bool sizing) {
     CMG_CUDA(cudaStreamWaitEvent(ss, fork_, 0));
     side_open_ = true;
     prep_head();
+    walk();
     occ_head(st);
     if (!sizing) prep_tail();
     occ_tail(st);
@@ -616,16 +635,16 @@ void Batch::run_impl(bool sizing) {
     if (timed) CMG_CUDA(cudaEventRecord(ev_[2], st));
     if (opts_.brick == 16 && sub_precision(opts_) == kPrecFP64)
         launch_sdf_sub(opts_.grab, opts_.ctas, dsegs_, nseg, I.work, nwork_, queue_, I.soup, I.tinfo,
-                       I.tinfo_lo, I.trec, I.tnorm, I.cand_off, I.cand, occ, sdf32_, sdf64_,
+                       I.tinfo_lo, I.trec, I.tnorm, I.cand_rng, I.cand, occ, sdf32_, sdf64_,
                        near_tri_, near_reg_, stats_, I.grid_eval, st);
     else if (opts_.brick == 16)
         launch_sdf_near(sub_precision(opts_), opts_.grab, opts_.probe, dsegs_, nseg,
-                        I.work, nwork_, queue_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.cand_off,
+                        I.work, nwork_, queue_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.cand_rng,
                         I.cand, I.cand_c, opts_.band, occ, sdf32_, sdf64_, near_tri_, near_reg_, err_, stats_,
                         I.grid_eval, st);
     else
         launch_sdf_eval(opts_.precision, opts_.brick, dsegs_, nseg, I.work, nbrick_, queue_,
-                        I.soup, I.tinfo, I.cand_off, I.cand, I.brick_emax, opts_.band, occ,
+                        I.soup, I.tinfo, I.cand_rng, I.cand, I.brick_emax, opts_.band, occ,
                         sdf32_, sdf64_, near_tri_, near_reg_, err_, stats_, I.grid_eval, st);
     if (timed) CMG_CUDA(cudaEventRecord(ev_[3], st));
 }
@@ -651,7 +670,7 @@ WorkModel Batch::work_model() {
     unsigned long long* d = nullptr;
     CMG_CUDA(device_alloc(&d, 3 * sizeof(unsigned long long)));
     CMG_CUDA(cudaMemsetAsync(d, 0, 3 * sizeof(unsigned long long), stream_));
-    launch_count_K(opts_.brick, dsegs_, static_cast<int>(segs_.size()), nbrick_, I.tinfo, I.cand_off,
+    launch_count_K(opts_.brick, dsegs_, static_cast<int>(segs_.size()), nbrick_, I.tinfo, I.cand_rng,
                    I.cand, sdf64_, sdf32_, opts_.band, d, stream_);
     unsigned long long h[3];
     CMG_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, stream_));
@@ -679,13 +698,13 @@ RunInfo Batch::info() {
     CMG_CUDA(cudaStreamSynchronize(stream_));
     r.brick = opts_.brick;
     r.grab = opts_.brick == 16 ? opts_.grab : 0;
-    r.walk_warps = brick_walk_warps(nbrick_, opts_.walk_warps);
+    r.walk_warps = segs_[0].walk_warps;
     const bool plain = sub_precision(opts_) == kPrecFP64;
     r.probe = plain || opts_.brick != 16 ? 0 : std::max(opts_.probe, 0);
     r.ctas = opts_.brick != 16 ? 0 : (plain ? sdf_sub_minb(opts_.ctas) : impl_->grid_eval / device_sms());
     r.cells = nvox_;
     r.pairs = pairs_cap_;
-    r.candidates = cand_cap_;
+    r.candidates = static_cast<int64_t>(r.stats.candidates);
     return r;
 }
 

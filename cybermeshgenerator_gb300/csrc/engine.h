@@ -137,7 +137,7 @@ struct RunInfo {
     Stats stats{};
     int brick = 0;
     int grab = 0;
-    int walk_warps = 0;  // warps per brick of the candidate walk
+    int walk_warps = 0;  // warps per brick of the candidate walk (the first mesh's)
     int probe = 0;       // probe head (FP32 pass; 0: the whole list)
     int ctas = 0;        // evaluation CTAs per SM
     int64_t cells = 0;
@@ -210,7 +210,7 @@ private:
     VoxOpts opts_;
     cudaStream_t stream_;
     std::vector<MeshSeg> segs_;
-    int64_t npts_ = 0, ntris_ = 0, ncol_ = 0, nrow_ = 0, nvox_ = 0, nbrick_ = 0, nwork_ = 0;
+    int64_t npts_ = 0, ntris_ = 0, ncol_ = 0, nrow_ = 0, nvox_ = 0, nbrick_ = 0, nwork_ = 0, nwalk_ = 0;
     int64_t pairs_cap_ = -1, cand_cap_ = -1;
     bool resize_ = false;  // points moved since the workspace was sized
     double* pts_ = nullptr;

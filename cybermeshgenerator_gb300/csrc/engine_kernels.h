@@ -39,27 +39,35 @@ void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const dou
                          float4* thi,
                          int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits,
                          cudaStream_t st);
+// The bins' triangles (bin_list) with their centroids and radii in that order (bin_info),
+// and per bin a ball around them (bin_ball, bin_reach).
 void launch_bin_fill(int64_t ntris, const int64_t* tbin, const int64_t* bin_off, int* bincur,
-                     int* bin_list, const MeshSeg* segs, int nseg, int* large_cur, int* large_list,
-                     cudaStream_t st);
+                     const float4* tinfo, int* bin_list, float4* bin_info, int64_t nbins,
+                     float4* bin_ball, float* bin_reach, const MeshSeg* segs, int nseg, int* large_cur,
+                     int* large_list, cudaStream_t st);
 void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsigned* emax_bits,
                        cudaStream_t st);
+// Candidate lists: per brick its count, and its range [cand_rng[2 b], cand_rng[2 b + 1]) in
+// cand (cap entries), in no particular order; stats->candidates (zero before) gets the
+// total. A total above cap leaves lists out: the caller sizes cand and walks again.
 // cand_c (null: not wanted): per candidate, its centroid from the brick's centre and radius.
-void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
+void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
-                       const int64_t* bin_off, const int* bin_list, const int* large_list,
-                       float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
-                       float4* cand_c, float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st);
-// Warps per brick the walk uses: walk_warps when it is 1, 2 or 4, else by the brick
-// count (4 while 4-warp bricks fit about twice in the GPU, 2 up to twice that, then 1).
-int brick_walk_warps(int64_t nbricks, int walk_warps);
+                       const int64_t* bin_off, const int* bin_list, const float4* bin_info,
+                       const float4* bin_ball, const float* bin_reach, const int* large_list,
+                       int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
+                       float* brick_emax, Stats* stats, cudaStream_t st);
+// Warps per brick the walk uses for a mesh of a batch of nbricks in all (walk_warps when it
+// is 1, 2 or 4, else by the counts), and its CTAs for that.
+int brick_walk_warps(int64_t nbricks, int64_t mesh_bricks, int64_t mesh_tris, int walk_warps);
+int64_t brick_walk_ctas(int64_t mesh_bricks, int warps);
 void launch_count_K(int brick, const MeshSeg* segs, int nseg, int64_t nbricks, const float4* tinfo,
-                    const int64_t* cand_off, const int* cand, const double* sdf64,
+                    const int64_t* cand_rng, const int* cand, const double* sdf64,
                     const float* sdf32, float band_cells, unsigned long long* out,
                     cudaStream_t st);
 void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, const uint32_t* work,
                      int64_t nwork, unsigned long long* queue, const double* soup,
-                     const float4* tinfo, const int64_t* cand_off, const int* cand,
+                     const float4* tinfo, const int64_t* cand_rng, const int* cand,
                      const float* brick_emax, float band_cells, const uint8_t* occ, float* sdf32,
                      double* sdf64, int* near_tri, uint8_t* near_reg, float* errbound, Stats* stats,
                      int grid, cudaStream_t st);
@@ -73,7 +81,7 @@ int sdf_sub_grid(int ctas);
 void launch_sdf_sub(int grab, int ctas, const MeshSeg* segs, int nseg, const uint32_t* work,
                     int64_t nwork, unsigned long long* queue, const double* soup,
                     const float4* tinfo, const float4* tinfo_lo, const void* trec,
-                    const float4* tnorm, const int64_t* cand_off, const int* cand,
+                    const float4* tnorm, const int64_t* cand_rng, const int* cand,
                     const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
                     uint8_t* near_reg, Stats* stats, int grid, cudaStream_t st);
 
@@ -84,7 +92,7 @@ int sdf_near_grid(int precision);
 void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, int nseg,
                      const uint32_t* work, int64_t nwork, unsigned long long* queue,
                      const double* soup, const float4* tinfo, const float4* tinfo_lo,
-                     const void* trec, const int64_t* cand_off, const int* cand, const float4* cand_c,
+                     const void* trec, const int64_t* cand_rng, const int* cand, const float4* cand_c,
                      float band_cells,
                      const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
                      uint8_t* near_reg, float* errbound, Stats* stats, int grid, cudaStream_t st);

@@ -28,7 +28,6 @@
 
 #include <cfloat>
 #include <climits>
-#include <type_traits>
 
 #include "cmg_device.cuh"
 #include "cmg_sdf.cuh"
@@ -197,20 +196,63 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
     atomicAdd(&bincnt[bin], 1);
 }
 
+// Bin -> triangle CSR. bin_info: the triangles' tinfo in the list's order, so that the walks
+// read the bins' entries in order and the ids only of those they take.
 __global__ void k_bin_fill(int64_t ntris, const int64_t* __restrict__ tbin,
                            const int64_t* __restrict__ bin_off, int* __restrict__ bincur,
-                           int* __restrict__ bin_list, const MeshSeg* __restrict__ segs, int nseg,
+                           const float4* __restrict__ tinfo, int* __restrict__ bin_list,
+                           float4* __restrict__ bin_info, const MeshSeg* __restrict__ segs, int nseg,
                            int* __restrict__ large_cur, int* __restrict__ large_list) {
     int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= ntris) return;
     int64_t b = tbin[t];
     if (b >= 0) {
-        int slot = atomicSub(&bincur[b], 1) - 1;  // the counts, taken down to zero
-        bin_list[bin_off[b] + slot] = static_cast<int>(t);
+        const int64_t at = bin_off[b] + atomicSub(&bincur[b], 1) - 1;  // the counts, taken down to zero
+        bin_list[at] = static_cast<int>(t);
+        bin_info[at] = tinfo[t];
     } else {
         const int si = find_seg<&MeshSeg::tri_begin>(segs, nseg, t);
         int slot = atomicAdd(&large_cur[si], 1);
         large_list[segs[si].large_begin + slot] = static_cast<int>(t);
+    }
+}
+
+// Per bin, a ball around its triangles: the middle of its centroids' box, the largest
+// distance of a centroid from it (w; -1: an empty bin) and of a triangle (bin_reach), so
+// that the walks skip whole bins. One warp per bin.
+__global__ void k_bin_balls(int64_t nbins, const int64_t* __restrict__ bin_off,
+                            const float4* __restrict__ bin_info, const MeshSeg* __restrict__ segs,
+                            int nseg, float4* __restrict__ bin_ball, float* __restrict__ bin_reach) {
+    const int64_t b = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (b >= nbins) return;
+    const int64_t e0 = bin_off[b], e1 = bin_off[b + 1];
+    if (e0 == e1) {
+        if (lane == 0) bin_ball[b] = make_float4(0.f, 0.f, 0.f, -1.f);
+        return;
+    }
+    float lx = FLT_MAX, ly = FLT_MAX, lz = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX, hz = -FLT_MAX;
+    for (int64_t e = e0 + lane; e < e1; e += 32) {
+        const float4 t = bin_info[e];
+        lx = fminf(lx, t.x); ly = fminf(ly, t.y); lz = fminf(lz, t.z);
+        hx = fmaxf(hx, t.x); hy = fmaxf(hy, t.y); hz = fmaxf(hz, t.z);
+    }
+    const float cx = 0.5f * (warp_min(lx) - warp_min(-hx)), cy = 0.5f * (warp_min(ly) - warp_min(-hy)),
+                cz = 0.5f * (warp_min(lz) - warp_min(-hz));
+    float rc = 0.f, rt = 0.f;
+    for (int64_t e = e0 + lane; e < e1; e += 32) {
+        const float4 t = bin_info[e];
+        const float dx = t.x - cx, dy = t.y - cy, dz = t.z - cz;
+        const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+        rc = fmaxf(rc, d);
+        rt = fmaxf(rt, d + t.w);
+    }
+    rc = -warp_min(-rc);
+    rt = -warp_min(-rt);
+    if (lane == 0) {
+        const float tol = list_tol(segs[find_seg<&MeshSeg::brick_begin>(segs, nseg, b)].scale);
+        bin_ball[b] = make_float4(cx, cy, cz, rc * (1.f + 8.f * kU32) + tol);
+        bin_reach[b] = rt * (1.f + 8.f * kU32) + tol;
     }
 }
 
@@ -312,20 +354,14 @@ __device__ __forceinline__ void shell_offset(int r, int q, int& dx, int& dy, int
 
 __device__ __forceinline__ int shell_count(int r) { return r == 0 ? 1 : 24 * r * r + 2; }
 
-// Bin k of the Chebyshev shell r around the brick (if in the grid): its entry
-// range [b0, b1) in the bin CSR; `inside` is set when the bin lies in the grid.
-__device__ __forceinline__ void shell_bin(const MeshSeg& s, const BrickGeo& q,
-                                          const int64_t* __restrict__ bin_off, int r, int k, int n,
-                                          bool& inside, int64_t& b0, int64_t& b1) {
-    if (k >= n) return;
+// Bin k of the Chebyshev shell r around the brick, or -1 (not in the grid).
+__device__ __forceinline__ int64_t shell_bin(const MeshSeg& s, const BrickGeo& q, int r, int k, int n) {
+    if (k >= n) return -1;
     int dx, dy, dz;
     shell_offset(r, k, dx, dy, dz);
     const int x = q.bx + dx, y = q.by + dy, z = q.bz + dz;
-    if (x < 0 || y < 0 || z < 0 || x >= s.bnx || y >= s.bny || z >= s.bnz) return;
-    inside = true;
-    const int64_t bin = s.brick_begin + (static_cast<int64_t>(z) * s.bny + y) * s.bnx + x;
-    b0 = bin_off[bin];
-    b1 = bin_off[bin + 1];
+    if (x < 0 || y < 0 || z < 0 || x >= s.bnx || y >= s.bny || z >= s.bnz) return -1;
+    return s.brick_begin + (static_cast<int64_t>(z) * s.bny + y) * s.bnx + x;
 }
 
 // Upper bound on the distance from point c (corner-relative) to a large triangle:
@@ -403,71 +439,85 @@ __device__ __forceinline__ void for_group_entries(int64_t b0, int64_t b1, int la
     }
 }
 
-// W warps per brick, 4 / W bricks per CTA of 128 threads. With few bricks the walks of
-// the bricks deep inside a closed surface set the kernel's time (tens of thousands of
-// candidates each: every triangle within U + 2 r_B), and W = 4 splits them; with
-// many bricks the GPU is full anyway and W = 1 walks each with one warp. Each
-// shell's 32-bin groups are split into contiguous ranges, one per warp, range w
-// before range w + 1, so the walk order is that of a single walker; the bound U, the
-// stopping rules and the counts are reduced over the brick's warps after each shell
-// (a named barrier per brick). FILL=false: computes U (stored) and the candidate
-// count. FILL=true: per shell each warp counts its candidates, the brick's warps take
-// prefix sums, and each writes its own at its offset, in walk order.
-constexpr int kWalkThreads = 128;
+// Candidate lists, one kernel: per brick
+//   1. an upper bound U on the distance from its centre to the surface, from the nearest
+//      binned centroid (a point of the surface) and the large triangles' edges;
+//   2. the count of the triangles that can be nearest to some cell of the brick: every
+//      triangle whose lower bound |c - c_t| - e_t - r_B can be <= U + r_B, cut by the box test
+//      around that centroid (a brick's sphere gives away 2 r_B in every direction, most of the
+//      list of a brick far from the surface);
+//   3. space for them (an atomic on the total; the lists' order in memory means nothing) and
+//      the entries, if they fit.
+// Bins are taken in Chebyshev shells around the brick; a bin's ball (k_bin_balls) is tested
+// before its entries, which lie in order (bin_info). W warps per brick (8 / W bricks per
+// CTA), by the mesh (MeshSeg::walk_warps): the walks of the bricks deep inside a closed
+// surface, and of bricks with thousands of triangles each, set the kernel's time when the
+// rest of the GPU has run dry. Each shell's 32-bin groups are split into contiguous ranges,
+// one per warp, and each warp writes its own entries after those of the warps before it;
+// the bound is reduced over the brick's warps after each shell (a named barrier per brick).
+// (231x247x256 surface, 65k triangles, W = 4: 0.57 + 0.87 ms for a counting and a writing
+// kernel that gathered every entry of every shell's bins -> 0.56 ms.)
+constexpr int kWalkThreads = 256;
 
-template <bool FILL, int W>
-__global__ void __launch_bounds__(kWalkThreads)
-k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
+__global__ void __launch_bounds__(kWalkThreads, 3)
+k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
              const double* __restrict__ soup, const float4* __restrict__ tinfo,
              const float4* __restrict__ tlo, const float4* __restrict__ thi,
              const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
-             const int* __restrict__ large_list, float* __restrict__ bound,
-             int* __restrict__ bound_tri, int* __restrict__ cand_cnt, const int64_t* __restrict__ cand_off,
-             int* __restrict__ cand, float4* __restrict__ cand_c, float* __restrict__ brick_emax,
+             const float4* __restrict__ bin_info, const float4* __restrict__ bin_ball,
+             const float* __restrict__ bin_reach, const int* __restrict__ large_list,
+             int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
+             float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
              Stats* __restrict__ st) {
     constexpr int kWarps = kWalkThreads / 32;
-    __shared__ float s_f[kWarps];
-    __shared__ int s_i[kWarps];
+    __shared__ float4 s_q[kWarps];
     __shared__ int s_c[kWarps];
+    __shared__ long long s_off[kWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const MeshSeg& s = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
+    const int W = s.walk_warps;
     const int slot = wid / W, sub = wid % W;  // brick within the CTA, warp within the brick
     const int first = slot * W;               // the brick's first warp
-    const int64_t gb = static_cast<int64_t>(blockIdx.x) * (kWarps / W) + slot;
-    if (gb >= nbricks) return;  // uniform over the brick's warps
+    const int64_t lb = (blockIdx.x - s.walk_begin) * (kWarps / W) + slot;
+    if (lb >= static_cast<int64_t>(s.bnx) * s.bny * s.bnz) return;  // uniform over the brick's warps
+    const int64_t gb = s.brick_begin + lb;
     auto brick_sync = [&]() {
         if (W == 1) __syncwarp();
         else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(32 * W) : "memory");
     };
-    const int si = find_seg<&MeshSeg::brick_begin>(segs, nseg, gb);
-    const MeshSeg& s = segs[si];
-    const BrickGeo q = brick_geo(s, gb - s.brick_begin);
+    const BrickGeo q = brick_geo(s, lb);
     const float bw = static_cast<float>(s.brick * s.g.h);
     const float tol = list_tol(s.scale);
     const float emax = s.emax;
-    const int rmax = max(s.bnx, max(s.bny, s.bnz));
-    // reductions over the brick's warps (each of its threads calls them, at points
-    // uniform over the brick)
-    auto brick_min = [&](float v) {
-        v = warp_min(v);
-        if (W == 1) return v;
-        if (lane == 0) s_f[wid] = v;
+    // the last shell with a bin in the grid
+    const int rmax = max(max(max(q.bx, s.bnx - 1 - q.bx), max(q.by, s.bny - 1 - q.by)), max(q.bz, s.bnz - 1 - q.bz));
+    // the nearest centroid of the brick's warps (called by each of its threads, at points
+    // uniform over the brick): p its offset and squared distance, id its triangle. Ties go to
+    // the lowest triangle, so that the lists do not depend on the bins' order.
+    auto brick_nearest = [&](float4& p, int& id) {
+        const unsigned m = __reduce_min_sync(0xffffffffu, __float_as_uint(p.w));
+        const int best = __reduce_min_sync(0xffffffffu, __float_as_uint(p.w) == m ? id : INT_MAX);
+        const int src = __ffs(__ballot_sync(0xffffffffu, __float_as_uint(p.w) == m && id == best)) - 1;
+        p.x = __shfl_sync(0xffffffffu, p.x, src);
+        p.y = __shfl_sync(0xffffffffu, p.y, src);
+        p.z = __shfl_sync(0xffffffffu, p.z, src);
+        p.w = __uint_as_float(m);
+        id = best;
+        if (W == 1) return;
+        if (lane == 0) {
+            s_q[wid] = p;
+            s_c[wid] = id;
+        }
         brick_sync();
-        float m = s_f[first];
-#pragma unroll
-        for (int w = 1; w < W; ++w) m = fminf(m, s_f[first + w]);
+        for (int w = 0; w < W; ++w) {
+            const float4 o = s_q[first + w];
+            const int oid = s_c[first + w];
+            if (o.w < p.w || (o.w == p.w && oid < id)) {
+                p = o;
+                id = oid;
+            }
+        }
         brick_sync();
-        return m;
-    };
-    auto brick_any = [&](bool v) {
-        const bool wv = __any_sync(0xffffffffu, v);
-        if (W == 1) return wv;
-        if (lane == 0) s_i[wid] = wv ? 1 : 0;
-        brick_sync();
-        int a = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) a |= s_i[first + w];
-        brick_sync();
-        return a != 0;
     };
     // this warp's contiguous range [g0, g1) of the 32-bin groups of a shell of n bins
     auto range = [&](int n, int& g0, int& g1) {
@@ -475,125 +525,109 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
         g0 = static_cast<int>(static_cast<int64_t>(ng) * sub / W);
         g1 = static_cast<int>(static_cast<int64_t>(ng) * (sub + 1) / W);
     };
-    float U;
-    int ut = INT_MAX;  // the binned triangle whose sphere gives the smallest bound
-    if (!FILL) {
-        // ---- upper bound on the distance from the brick centre to the surface
-        U = FLT_MAX;
-        float ub = FLT_MAX;
-        for (int64_t e = s.large_begin + 32 * sub + lane; e < s.large_end; e += 32 * W)
-            U = fminf(U, large_upper(soup, large_list[e], s.g.corner, q.cx, q.cy, q.cz, tol));
-        for (int r = 0; r <= rmax; ++r) {
-            U = brick_min(U);
-            if (r > 0 && (r - 1) * bw > U) break;  // farther bins cannot lower U
-            const int n = shell_count(r);
-            int g0, g1;
-            range(n, g0, g1);
-            bool inside = false;
-            for (int g = g0; g < g1; ++g) {
-                int64_t b0 = 0, b1 = 0;
-                shell_bin(s, q, bin_off, r, 32 * g + lane, n, inside, b0, b1);
-                for_group_entries(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
-                    int t[kWalkRounds];
-#pragma unroll
-                    for (int j = 0; j < kWalkRounds; ++j) t[j] = ok[j] ? bin_list[e[j]] : -1;
-#pragma unroll
-                    for (int j = 0; j < kWalkRounds; ++j) {
-                        if (t[j] < 0) continue;
-                        float4 ti = tinfo[t[j]];
-                        float dx2 = ti.x - q.cx, dy2 = ti.y - q.cy, dz2 = ti.z - q.cz;
-                        float d = sqrtf(dx2 * dx2 + dy2 * dy2 + dz2 * dz2) * (1.f + 4.f * kU32);
-                        const float v = d + ti.w + tol;
-                        U = fminf(U, v);
-                        if (v < ub) { ub = v; ut = t[j]; }
-                    }
-                });
-            }
-            if (r > 0 && !brick_any(inside)) {
-                U = brick_min(U);
-                break;
-            }
-        }
-        U = brick_min(U);
-        {
-            // the lowest index among the triangles at the smallest bound (exact in FP32)
-            const float m = brick_min(ub);
-            const int cand_t = ub == m ? ut : INT_MAX;
-            ut = __reduce_min_sync(0xffffffffu, cand_t);
-            if (W > 1) {
-                if (lane == 0) s_i[wid] = ut;
-                brick_sync();
-#pragma unroll
-                for (int w = 0; w < W; ++w) ut = min(ut, s_i[first + w]);
-                brick_sync();
-            }
-        }
-        if (sub == 0 && lane == 0) {
-            bound[gb] = U;
-            bound_tri[gb] = ut;
-        }
-    } else {
-        U = bound[gb];
-        ut = bound_tri[gb];
+    // ---- 1. the bound. UL: from the large triangles; U: that or the nearest centroid's
+    float UL = FLT_MAX;
+    for (int64_t e = s.large_begin + 32 * sub + lane; e < s.large_end; e += 32 * W)
+        UL = fminf(UL, large_upper(soup, large_list[e], s.g.corner, q.cx, q.cy, q.cz, tol));
+    {
+        float4 p = make_float4(0.f, 0.f, 0.f, UL);
+        int none = INT_MAX;
+        brick_nearest(p, none);
+        UL = p.w;
     }
-    // ---- candidates: lower bound <= U + 2 r_B (+ margins). The relative margin (4e-5,
-    // about 670 u) covers four stated FP32 errors 48u (d + 2e + 2r) beyond any cell's
-    // distance (e at most two bricks here; larger triangles are always considered): the
-    // exact FP64 path's near-ties and its band pass need them, the mixed path two
-    const float lim = (U + 2.f * q.rb) * (1.f + 4e-5f) + 2.f * tol;
-    // ... and, around the centroid of the triangle that gave the bound (a point of the
-    // surface), the box test with the same margins: a brick's sphere gives away 2 r_B in
-    // every direction, most of the list of a brick far from the surface
-    const bool boxed = ut != INT_MAX;
-    BoxTest box;
-    if (boxed) {
-        const float4 ti = tinfo[ut];
-        const float h = static_cast<float>(s.g.h);
-        box = box_test(ti.x - q.cx, ti.y - q.cy, ti.z - q.cz, 0.5f * (q.x1 - q.x0 - 1) * h,
-                       0.5f * (q.y1 - q.y0 - 1) * h, 0.5f * (q.z1 - q.z0 - 1) * h, q.rb,
-                       fmaf(4e-5f, U + 2.f * q.rb, 4.f * tol), tol);
-    }
-    const int64_t out = FILL ? cand_off[gb] : 0;
-    const unsigned below = (1u << lane) - 1u;
-    float bemax = 0.f;
-    // a list entry: the triangle and, for the warp-per-sub-brick evaluation, its centroid
-    // from the brick's centre and its radius, so that the scans read them in order (each
-    // brick's list is scanned twice by its 64 sub-bricks)
-    auto put = [&](int64_t at, int t, const float4& ti) {
-        cand[at] = t;
-        if (cand_c) cand_c[at] = make_float4(ti.x - q.cx, ti.y - q.cy, ti.z - q.cz, ti.w);
-    };
-    // walks this warp's groups of shell r; f(take, t, e_t) per entry, in walk order,
-    // called by the whole warp
-    auto walk = [&](int r, int n, int g0, int g1, bool& inside, auto&& f) {
+    float4 near = make_float4(0.f, 0.f, 0.f, FLT_MAX);
+    int near_t = INT_MAX;
+    float U = UL;
+    for (int r = 0; r <= rmax; ++r) {
+        if (r > 0 && (r - 1) * bw > U) break;  // farther bins cannot lower U
+        const int n = shell_count(r);
+        int g0, g1;
+        range(n, g0, g1);
         for (int g = g0; g < g1; ++g) {
+            const int64_t bin = shell_bin(s, q, r, 32 * g + lane, n);
             int64_t b0 = 0, b1 = 0;
-            shell_bin(s, q, bin_off, r, 32 * g + lane, n, inside, b0, b1);
+            if (bin >= 0) {
+                const float4 ball = bin_ball[bin];
+                const float dx = ball.x - q.cx, dy = ball.y - q.cy, dz = ball.z - q.cz;
+                // only bins with a centroid that can be nearer than the nearest so far
+                const float reach = fminf(U, sqrt_approx(near.w) * (1.f + 8.f * kU32)) + ball.w + tol;
+                if (ball.w >= 0.f && !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > reach * reach * (1.f + 16.f * kU32))) {
+                    b0 = bin_off[bin];
+                    b1 = bin_off[bin + 1];
+                }
+            }
             for_group_entries(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
-                int t[kWalkRounds];
-#pragma unroll
-                for (int j = 0; j < kWalkRounds; ++j) t[j] = ok[j] ? bin_list[e[j]] : -1;
-                float4 ti[kWalkRounds];
+                float4 t[kWalkRounds];
 #pragma unroll
                 for (int j = 0; j < kWalkRounds; ++j)
-                    if (t[j] >= 0) ti[j] = tinfo[t[j]];
+                    t[j] = ok[j] ? bin_info[e[j]] : make_float4(FLT_MAX, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int j = 0; j < kWalkRounds; ++j) {
-                    bool take = false;
-                    if (t[j] >= 0) {
-                        float dx2 = ti[j].x - q.cx, dy2 = ti[j].y - q.cy, dz2 = ti[j].z - q.cz;
-                        float d = sqrtf(dx2 * dx2 + dy2 * dy2 + dz2 * dz2) * (1.f - 4.f * kU32);
-                        take = d - ti[j].w <= lim;  // |v - c_t| - e_t >= d - r_B - e_t
-                        if (boxed) take = take && box_ball(box, dx2, dy2, dz2, ti[j].w, tol);
+                    const float x = t[j].x - q.cx, y = t[j].y - q.cy, z = t[j].z - q.cz;
+                    const float d2 = fmaf(x, x, fmaf(y, y, z * z));
+                    if (d2 <= near.w && ok[j]) {
+                        const int id = bin_list[e[j]];
+                        if (d2 < near.w || id < near_t) {
+                            near = make_float4(x, y, z, d2);
+                            near_t = id;
+                        }
                     }
-                    f(take, t[j], ti[j]);
                 }
             });
         }
+        brick_nearest(near, near_t);
+        U = fminf(UL, near.w < FLT_MAX ? sqrtf(near.w) * (1.f + 8.f * kU32) + tol : FLT_MAX);
+    }
+    // ---- 2. candidates: lower bound <= U + 2 r_B (+ margins). The relative margin (4e-5,
+    // about 670 u) covers four stated FP32 errors 48u (d + 2e + 2r) beyond any cell's
+    // distance (e at most two bricks here; larger triangles are always considered): the
+    // exact FP64 path's near-ties need them, the mixed path two
+    const float lim = (U + 2.f * q.rb) * (1.f + 4e-5f) + 2.f * tol;
+    const bool boxed = near.w < FLT_MAX;
+    BoxTest box;
+    if (boxed) {
+        const float h = static_cast<float>(s.g.h);
+        box = box_test(near.x, near.y, near.z, 0.5f * (q.x1 - q.x0 - 1) * h, 0.5f * (q.y1 - q.y0 - 1) * h,
+                       0.5f * (q.z1 - q.z0 - 1) * h, q.rb, fmaf(4e-5f, U + 2.f * q.rb, 4.f * tol), tol);
+    }
+    const unsigned below = (1u << lane) - 1u;
+    // whether a ball (a bin's or a triangle's, centre from the brick's centre) can matter
+    auto reaches = [&](float x, float y, float z, float w) {
+        const float d2 = fmaf(x, x, fmaf(y, y, z * z)), l = lim + w;  // |v - c| - w >= d - r_B - w
+        return !(d2 > l * l * (1.f + 16.f * kU32)) && (!boxed || box_ball(box, x, y, z, w, tol));
     };
-    // the always-considered large triangles first, by the brick's first warp
-    if (sub == 0) {
-        int c = 0;
+    // walks this warp's groups of every shell; f(take, entry, info) per entry, in walk order,
+    // called by the whole warp
+    auto walk = [&](auto&& f) {
+        for (int r = 0; r <= rmax; ++r) {
+            if (r > 0 && (r - 1) * bw - emax > lim) break;
+            const int n = shell_count(r);
+            int g0, g1;
+            range(n, g0, g1);
+            for (int g = g0; g < g1; ++g) {
+                const int64_t bin = shell_bin(s, q, r, 32 * g + lane, n);
+                int64_t b0 = 0, b1 = 0;
+                if (bin >= 0) {
+                    const float4 ball = bin_ball[bin];
+                    if (ball.w >= 0.f && reaches(ball.x - q.cx, ball.y - q.cy, ball.z - q.cz, bin_reach[bin])) {
+                        b0 = bin_off[bin];
+                        b1 = bin_off[bin + 1];
+                    }
+                }
+                for_group_entries(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
+                    float4 t[kWalkRounds];
+#pragma unroll
+                    for (int j = 0; j < kWalkRounds; ++j)
+                        t[j] = ok[j] ? bin_info[e[j]] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int j = 0; j < kWalkRounds; ++j)
+                        f(ok[j] && reaches(t[j].x - q.cx, t[j].y - q.cy, t[j].z - q.cz, t[j].w), e[j], t[j]);
+                });
+            }
+        }
+    };
+    // the always-considered large triangles, by the brick's first warp
+    auto walk_large = [&](auto&& f) {
         for (int64_t e0 = s.large_begin; e0 < s.large_end; e0 += 32) {
             const int64_t e = e0 + lane;
             bool take = false;
@@ -601,84 +635,61 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
             float4 ti = make_float4(0.f, 0.f, 0.f, 0.f);
             if (e < s.large_end) {
                 t = large_list[e];
-                float4 lo = tlo[t], hi = thi[t];
-                float d = aabb_dist(q.cx, q.cy, q.cz, lo, hi);
-                take = d <= lim;  // d(v,t) >= d - r_B must reach U + r_B
+                take = aabb_dist(q.cx, q.cy, q.cz, tlo[t], thi[t]) <= lim;  // d(v,t) >= d - r_B must reach U + r_B
                 ti = tinfo[t];
             }
-            const unsigned m = __ballot_sync(0xffffffffu, take);
-            if (FILL && take) put(out + c + __popc(m & below), t, ti);
-            if (take) bemax = fmaxf(bemax, ti.w);
-            c += __popc(m);
+            f(take, t, ti);
         }
-        if (lane == 0) s_c[first] = c;
+    };
+    int mine = 0;
+    auto count = [&](bool take, auto, const float4&) { mine += __popc(__ballot_sync(0xffffffffu, take)); };
+    if (sub == 0) walk_large(count);
+    walk(count);
+    // ---- 3. the list's place, and the entries
+    if (lane == 0) s_c[wid] = mine;
+    brick_sync();
+    int before = 0, total = 0;
+    for (int w = 0; w < W; ++w) {
+        if (w < sub) before += s_c[first + w];
+        total += s_c[first + w];
+    }
+    if (sub == 0 && lane == 0) {
+        const long long at = static_cast<long long>(atomicAdd(&st->candidates, static_cast<unsigned long long>(total)));
+        s_off[first] = at;
+        cand_cnt[gb] = total;
+        const bool fits = at + total <= cap;
+        cand_rng[2 * gb] = fits ? at : 0;
+        cand_rng[2 * gb + 1] = fits ? at + total : 0;
     }
     brick_sync();
-    int64_t base = s_c[first];  // entries before the current shell
-    brick_sync();
-    int mine = 0;           // count pass: this warp's entries over all shells
-    for (int r = 0; r <= rmax; ++r) {
-        if (r > 0 && (r - 1) * bw - emax > lim) break;
-        const int n = shell_count(r);
-        int g0, g1;
-        range(n, g0, g1);
-        bool any_inside = false;
-        int c = 0;
-        if (FILL && W == 1) {
-            // one warp per brick: written in the one walk, at a running offset
-            walk(r, n, g0, g1, any_inside, [&](bool take, int t, const float4& ti) {
-                const unsigned m = __ballot_sync(0xffffffffu, take);
-                if (take) {
-                    put(out + base + c + __popc(m & below), t, ti);
-                    bemax = fmaxf(bemax, ti.w);
-                }
-                c += __popc(m);
-            });
-            base += c;
-        } else {
-            walk(r, n, g0, g1, any_inside,
-                 [&](bool take, int, const float4&) { c += __popc(__ballot_sync(0xffffffffu, take)); });
+    int64_t at = s_off[first];
+    if (at + total > cap) return;  // uniform over the brick: the lists are sized and walked again
+    at += before;
+    float bemax = 0.f;
+    // a list entry: the triangle and, for the warp-per-sub-brick evaluation, its centroid from
+    // the brick's centre and its radius, so that the scans read them in order (each brick's
+    // list is scanned twice by its 64 sub-bricks)
+    auto put = [&](bool take, int t, const float4& ti) {
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (take) {
+            const int64_t k = at + __popc(m & below);
+            cand[k] = t;
+            if (cand_c) cand_c[k] = make_float4(ti.x - q.cx, ti.y - q.cy, ti.z - q.cz, ti.w);
+            bemax = fmaxf(bemax, ti.w);
         }
-        if (FILL && W > 1) {
-            // several warps: prefix sums of this shell's counts, then the writing walk
-            if (lane == 0) s_c[wid] = c;
+        at += __popc(m);
+    };
+    if (sub == 0) walk_large(put);
+    walk([&](bool take, int64_t e, const float4& ti) { put(take, take ? bin_list[e] : 0, ti); });
+    {
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        bemax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bemax)));
+        if (W > 1) {
+            p.w = bemax;
+            if (lane == 0) s_q[wid] = p;
             brick_sync();
-            int64_t off = base;
-            int tot = 0;
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                if (w < sub) off += s_c[first + w];
-                tot += s_c[first + w];
-            }
-            brick_sync();
-            int k = 0;
-            bool again = false;
-            walk(r, n, g0, g1, again, [&](bool take, int t, const float4& ti) {
-                const unsigned m = __ballot_sync(0xffffffffu, take);
-                if (take) {
-                    put(out + off + k + __popc(m & below), t, ti);
-                    bemax = fmaxf(bemax, ti.w);
-                }
-                k += __popc(m);
-            });
-            base += tot;
-        } else if (!FILL) {
-            mine += c;
+            for (int w = 0; w < W; ++w) bemax = fmaxf(bemax, s_q[first + w].w);
         }
-        if (r > 0 && !brick_any(any_inside)) break;
-    }
-    if (!FILL) {
-        if (lane == 0) s_c[wid] = mine;
-        brick_sync();
-        if (sub == 0 && lane == 0) {
-            int64_t total = base;
-#pragma unroll
-            for (int w = 0; w < W; ++w) total += s_c[first + w];
-            cand_cnt[gb] = static_cast<int>(total);
-            atomicAdd(&st->candidates, static_cast<unsigned long long>(total));
-        }
-    } else {
-        bemax = -brick_min(-bemax);
         if (sub == 0 && lane == 0) brick_emax[gb] = bemax;
     }
 }
@@ -704,7 +715,7 @@ template <int B, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 k_sdf_fp64(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict__ work,
            int64_t nwork, unsigned long long* __restrict__ queue, const double* __restrict__ soup,
-           const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_off,
+           const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_rng,
            const int* __restrict__ cand, Out o, Stats* __restrict__ st) {
     using M = CellMap<B, THREADS>;
     constexpr int VPT = M::VPT;
@@ -742,7 +753,7 @@ k_sdf_fp64(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restric
             bt[v] = INT_MAX;
             br[v] = 0;
         }
-        const int64_t c0 = cand_off[gb], c1 = cand_off[gb + 1];
+        const int64_t c0 = cand_rng[2 * gb], c1 = cand_rng[2 * gb + 1];
         for (int64_t base = c0; base < c1; base += kChunk) {
             const int n = static_cast<int>(c1 - base < kChunk ? c1 - base : kChunk);
             __syncthreads();
@@ -900,7 +911,7 @@ template <int B, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 k_sdf_mixed(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict__ work,
             int64_t nwork, unsigned long long* __restrict__ queue, const double* __restrict__ soup,
-            const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_off,
+            const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_rng,
             const int* __restrict__ cand, const float* __restrict__ brick_emax, float band_cells,
             Out o, Stats* __restrict__ st) {
     using M = CellMap<B, THREADS>;
@@ -944,7 +955,7 @@ k_sdf_mixed(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restri
             bt[v] = INT_MAX;
             br[v] = 0;
         }
-        const int64_t c0 = cand_off[gb], c1 = cand_off[gb + 1];
+        const int64_t c0 = cand_rng[2 * gb], c1 = cand_rng[2 * gb + 1];
         for (int64_t base = c0; base < c1; base += kChunk) {
             const int n = static_cast<int>(c1 - base < kChunk ? c1 - base : kChunk);
             __syncthreads();
@@ -1078,7 +1089,7 @@ k_sdf_mixed(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restri
 template <int B, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 k_count_K(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
-          const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_off,
+          const float4* __restrict__ tinfo, const int64_t* __restrict__ cand_rng,
           const int* __restrict__ cand, const double* __restrict__ sdf64,
           const float* __restrict__ sdf32, float band_cells, unsigned long long* __restrict__ out) {
     using M = CellMap<B, THREADS>;
@@ -1100,7 +1111,7 @@ k_count_K(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
         float d = sdf64 ? static_cast<float>(fabs(sdf64[idx])) : fabsf(sdf32[idx]);
         float px = (x + 0.5f) * h, py = (y + 0.5f) * h, pz = (z + 0.5f) * h;
         unsigned kk = 0;
-        for (int64_t e = cand_off[gb]; e < cand_off[gb + 1]; ++e) {
+        for (int64_t e = cand_rng[2 * gb]; e < cand_rng[2 * gb + 1]; ++e) {
             float4 ti = tinfo[cand[e]];
             float dx = px - ti.x, dy = py - ti.y, dz = pz - ti.z;
             kk += sqrtf(dx * dx + dy * dy + dz * dz) - ti.w <= d;
@@ -1138,11 +1149,15 @@ void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const dou
 }
 
 void launch_bin_fill(int64_t ntris, const int64_t* tbin, const int64_t* bin_off, int* bincur,
-                     int* bin_list, const MeshSeg* segs, int nseg, int* large_cur, int* large_list,
-                     cudaStream_t st) {
+                     const float4* tinfo, int* bin_list, float4* bin_info, int64_t nbins,
+                     float4* bin_ball, float* bin_reach, const MeshSeg* segs, int nseg, int* large_cur,
+                     int* large_list, cudaStream_t st) {
     if (ntris == 0) return;
     k_bin_fill<<<static_cast<unsigned>((ntris + 255) / 256), 256, 0, st>>>(
-        ntris, tbin, bin_off, bincur, bin_list, segs, nseg, large_cur, large_list);
+        ntris, tbin, bin_off, bincur, tinfo, bin_list, bin_info, segs, nseg, large_cur, large_list);
+    CMG_LAUNCH();
+    k_bin_balls<<<static_cast<unsigned>((nbins + 3) / 4), 128, 0, st>>>(nbins, bin_off, bin_info, segs, nseg,
+                                                                        bin_ball, bin_reach);
     CMG_LAUNCH();
 }
 
@@ -1152,67 +1167,52 @@ void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsi
     CMG_LAUNCH();
 }
 
-int brick_walk_warps(int64_t nbricks, int walk_warps) {
+int brick_walk_warps(int64_t nbricks, int64_t mesh_bricks, int64_t mesh_tris, int walk_warps) {
     if (walk_warps == 1 || walk_warps == 2 || walk_warps == 4) return walk_warps;
-    // 4 while 4-warp bricks fit about twice in the GPU's warp slots (a few heavy bricks
-    // set the time), 2 up to twice that, then 1
+    // 8 while the bricks are few, or for a mesh whose bricks see hundreds of triangles each;
+    // else 4 while 4-warp bricks fit about twice in the GPU, 2 up to twice that, then 1
     const int64_t sms = device_sms();
+    if (nbricks <= 8 * sms || mesh_tris > 128 * mesh_bricks) return 8;
     return nbricks <= 32 * sms ? 4 : (nbricks <= 64 * sms ? 2 : 1);
 }
+int64_t brick_walk_ctas(int64_t mesh_bricks, int warps) {
+    const int64_t per = kWalkThreads / 32 / warps;
+    return (mesh_bricks + per - 1) / per;
+}
 
-void launch_brick_walk(bool fill, const MeshSeg* segs, int nseg, int64_t nbricks, const double* soup,
+void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
-                       const int64_t* bin_off, const int* bin_list, const int* large_list,
-                       float* bound, int* bound_tri, int* cand_cnt, const int64_t* cand_off, int* cand,
-                       float4* cand_c, float* brick_emax, Stats* stats, int walk_warps, cudaStream_t st) {
-    if (nbricks == 0) return;
-    const int W = brick_walk_warps(nbricks, walk_warps);
-    const unsigned grid = static_cast<unsigned>((nbricks * W + 3) / 4);
-    auto go = [&](auto fill_tag, auto w_tag) {
-        constexpr bool F = decltype(fill_tag)::value;
-        constexpr int WW = decltype(w_tag)::value;
-        k_brick_walk<F, WW><<<grid, kWalkThreads, 0, st>>>(segs, nseg, nbricks, soup, tinfo, tlo, thi,
-                                                           bin_off, bin_list, large_list, bound,
-                                                           bound_tri, cand_cnt, cand_off, cand, cand_c, brick_emax,
-                                                           stats);
-    };
-    using T = std::true_type;
-    using Fa = std::false_type;
-    using W1 = std::integral_constant<int, 1>;
-    using W2 = std::integral_constant<int, 2>;
-    using W4 = std::integral_constant<int, 4>;
-    if (fill) {
-        if (W == 4) go(T{}, W4{});
-        else if (W == 2) go(T{}, W2{});
-        else go(T{}, W1{});
-    } else {
-        if (W == 4) go(Fa{}, W4{});
-        else if (W == 2) go(Fa{}, W2{});
-        else go(Fa{}, W1{});
-    }
+                       const int64_t* bin_off, const int* bin_list, const float4* bin_info,
+                       const float4* bin_ball, const float* bin_reach, const int* large_list,
+                       int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
+                       float* brick_emax, Stats* stats, cudaStream_t st) {
+    if (ctas == 0) return;
+    k_brick_walk<<<static_cast<unsigned>(ctas), kWalkThreads, 0, st>>>(
+        segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list,
+        cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, stats);
     CMG_LAUNCH();
 }
 
 void launch_count_K(int brick, const MeshSeg* segs, int nseg, int64_t nbricks, const float4* tinfo,
-                    const int64_t* cand_off, const int* cand, const double* sdf64,
+                    const int64_t* cand_rng, const int* cand, const double* sdf64,
                     const float* sdf32, float band_cells, unsigned long long* out,
                     cudaStream_t st) {
     if (nbricks == 0) return;
     if (brick == 4)
         k_count_K<4, 64><<<static_cast<unsigned>(nbricks), 64, 0, st>>>(
-            segs, nseg, nbricks, tinfo, cand_off, cand, sdf64, sdf32, band_cells, out);
+            segs, nseg, nbricks, tinfo, cand_rng, cand, sdf64, sdf32, band_cells, out);
     else if (brick == 16)
         k_count_K<16, 256><<<static_cast<unsigned>(nbricks), 256, 0, st>>>(
-            segs, nseg, nbricks, tinfo, cand_off, cand, sdf64, sdf32, band_cells, out);
+            segs, nseg, nbricks, tinfo, cand_rng, cand, sdf64, sdf32, band_cells, out);
     else
         k_count_K<8, 128><<<static_cast<unsigned>(nbricks), 128, 0, st>>>(
-            segs, nseg, nbricks, tinfo, cand_off, cand, sdf64, sdf32, band_cells, out);
+            segs, nseg, nbricks, tinfo, cand_rng, cand, sdf64, sdf32, band_cells, out);
     CMG_LAUNCH();
 }
 
 void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, const uint32_t* work,
                      int64_t nwork, unsigned long long* queue, const double* soup,
-                     const float4* tinfo, const int64_t* cand_off, const int* cand,
+                     const float4* tinfo, const int64_t* cand_rng, const int* cand,
                      const float* brick_emax, float band_cells, const uint8_t* occ, float* sdf32,
                      double* sdf64, int* near_tri, uint8_t* near_reg, float* errbound, Stats* stats,
                      int grid, cudaStream_t st) {
@@ -1221,18 +1221,18 @@ void launch_sdf_eval(int precision, int brick, const MeshSeg* segs, int nseg, co
     if (precision == kPrecMixed) {
         if (brick == 4)
             k_sdf_mixed<4, 64><<<grid, 64, 0, st>>>(segs, nseg, work, nwork, queue, soup, tinfo,
-                                                    cand_off, cand, brick_emax, band_cells, o, stats);
+                                                    cand_rng, cand, brick_emax, band_cells, o, stats);
         else
             k_sdf_mixed<8, 128><<<grid, 128, 0, st>>>(segs, nseg, work, nwork, queue, soup, tinfo,
-                                                      cand_off, cand, brick_emax, band_cells, o,
+                                                      cand_rng, cand, brick_emax, band_cells, o,
                                                       stats);
     } else {
         if (brick == 4)
             k_sdf_fp64<4, 64><<<grid, 64, 0, st>>>(segs, nseg, work, nwork, queue, soup, tinfo,
-                                                   cand_off, cand, o, stats);
+                                                   cand_rng, cand, o, stats);
         else
             k_sdf_fp64<8, 128><<<grid, 128, 0, st>>>(segs, nseg, work, nwork, queue, soup, tinfo,
-                                                     cand_off, cand, o, stats);
+                                                     cand_rng, cand, o, stats);
     }
     CMG_LAUNCH();
 }

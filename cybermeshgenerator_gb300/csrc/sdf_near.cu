@@ -194,7 +194,7 @@ struct Args {
     const double* soup;
     const float4 *tinfo, *tinfo_lo;
     const TriRec* trec;
-    const int64_t* cand_off;
+    const int64_t* cand_rng;
     const int* cand;
     const float4* cand_c;
     float band_cells;
@@ -286,8 +286,8 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         }
         __syncwarp();
     }
-    const int64_t c0 = g.cand_off[gb];
-    const int nc = static_cast<int>(g.cand_off[gb + 1] - c0);
+    const int64_t c0 = g.cand_rng[2 * gb];
+    const int nc = static_cast<int>(g.cand_rng[2 * gb + 1] - c0);
     const int* __restrict__ list = g.cand + c0;
     const float4* __restrict__ listc = g.cand_c + c0;
     const int first = COOP ? wid * 32 * kStep : 0, step = COOP ? kWarps * 32 * kStep : 32 * kStep;
@@ -581,7 +581,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     WarpMem& M = all[wid];
     const float items = static_cast<float>(g.nwork);
-    const float share = (static_cast<float>(g.cand_off[g.nwork >> 6]) * 64.f + kItemCost * items) /
+    const float share = (static_cast<float>(st->candidates) * 64.f + kItemCost * items) /
                         static_cast<float>(gridDim.x * kWarps);
     const float heavy = kHeavy * share - kItemCost;
     if (lane == 0) M.evals = M.filtered = M.evals64 = M.bandc = 0;
@@ -594,7 +594,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
         item = static_cast<int64_t>(S.grab) * g.grab_n;
         if (item >= g.nwork) break;
         const int64_t b = g.work[item >> 6];
-        if (static_cast<float>(g.cand_off[b + 1] - g.cand_off[b]) < heavy) {
+        if (static_cast<float>(g.cand_rng[2 * b + 1] - g.cand_rng[2 * b]) < heavy) {
             own = wid == 0;
             break;
         }
@@ -638,7 +638,7 @@ int sdf_near_grid(int precision) {
 void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, int nseg,
                      const uint32_t* work, int64_t nwork, unsigned long long* queue,
                      const double* soup, const float4* tinfo, const float4* tinfo_lo,
-                     const void* trec, const int64_t* cand_off, const int* cand, const float4* cand_c,
+                     const void* trec, const int64_t* cand_rng, const int* cand, const float4* cand_c,
                      float band_cells,
                      const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
                      uint8_t* near_reg, float* errbound, Stats* stats, int grid, cudaStream_t st) {
@@ -647,7 +647,7 @@ void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, in
     const int64_t need = (nwork + kWarps - 1) / kWarps;
     const unsigned blocks = static_cast<unsigned>(need < grid ? need : grid);
     const Args g{segs, nseg, work, nwork, grab, probe > 0 ? probe : INT_MAX, soup, tinfo, tinfo_lo,
-                 static_cast<const TriRec*>(trec), cand_off, cand, cand_c, band_cells,
+                 static_cast<const TriRec*>(trec), cand_rng, cand, cand_c, band_cells,
                  {occ, sdf32, sdf64, near_tri, near_reg, errbound}};
     auto go = [&](auto kernel) {
         kernel<<<blocks, 32 * kWarps, kWarps * sizeof(WarpMem), st>>>(g, queue, stats);

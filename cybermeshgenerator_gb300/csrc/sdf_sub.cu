@@ -48,7 +48,7 @@ k_sdf_sub(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict
           const double* __restrict__ soup,
           const float4* __restrict__ tinfo, const float4* __restrict__ tinfo_lo,
           const TriRec* __restrict__ trec, const float4* __restrict__ tnorm,
-          const int64_t* __restrict__ cand_off,
+          const int64_t* __restrict__ cand_rng,
           const int* __restrict__ cand, Out o, Stats* __restrict__ st) {
     __shared__ float4 s_c[kCap];  // centroid relative to the sub-brick centre, radius
     // unit normal and plane offset n . centroid, and a bound on the error of the plane
@@ -93,7 +93,7 @@ k_sdf_sub(const MeshSeg* __restrict__ segs, int nseg, const uint32_t* __restrict
         const float px = static_cast<float>((x + 0.5) * g.h - ckx);
         const float py = static_cast<float>((y + 0.5) * g.h - cky);
         const float pz = static_cast<float>((z + 0.5) * g.h - ckz);
-        const int64_t c0 = cand_off[gb], c1 = cand_off[gb + 1];
+        const int64_t c0 = cand_rng[2 * gb], c1 = cand_rng[2 * gb + 1];
 
         // ---- 1. probe: upper bound on the distance from the centre to the surface,
         //         and the triangle that gives it (the seed of every cell below)
@@ -275,7 +275,7 @@ int sdf_sub_grid(int ctas) {
 void launch_sdf_sub(int grab, int ctas, const MeshSeg* segs, int nseg, const uint32_t* work,
                     int64_t nwork, unsigned long long* queue, const double* soup,
                     const float4* tinfo, const float4* tinfo_lo, const void* trec,
-                    const float4* tnorm, const int64_t* cand_off, const int* cand,
+                    const float4* tnorm, const int64_t* cand_rng, const int* cand,
                     const uint8_t* occ, float* sdf32, double* sdf64, int* near_tri,
                     uint8_t* near_reg, Stats* stats, int grid, cudaStream_t st) {
     if (nwork == 0) return;
@@ -284,7 +284,7 @@ void launch_sdf_sub(int grab, int ctas, const MeshSeg* segs, int nseg, const uin
     if (grab != 1 && grab != 2 && grab != 4 && grab != 8) grab = 1;
     auto go = [&](auto kernel) {
         kernel<<<grid, kSubThreads, 0, st>>>(segs, nseg, work, nwork, grab, queue, soup, tinfo,
-                                            tinfo_lo, r, tnorm, cand_off, cand, o, stats);
+                                            tinfo_lo, r, tnorm, cand_rng, cand, o, stats);
     };
     sdf_sub_minb(ctas) == 16 ? go(k_sdf_sub<16>) : go(k_sdf_sub<12>);
     CMG_LAUNCH();

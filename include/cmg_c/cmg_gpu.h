@@ -59,8 +59,8 @@ typedef struct cmg_voxel_opts {
     int grab;            /* sub-bricks taken per work-queue grab: 0 = default, 1, 2, 4, 8 */
     int stage;           /* no effect: candidate records are always staged in shared memory
                             (kept for callers that set it) */
-    int walk_warps;      /* warps per brick of the candidate walk: 1, 2 or 4; 0 = by the
-                            brick count */
+    int walk_warps;      /* warps per brick of the candidate walk: 1, 2 or 4; 0 = 1 to 8 by the
+                            brick and triangle counts */
     int probe;           /* entries of the brick list the probe of the FP32 pass scans; 0 =
                             the whole list */
     int ctas;            /* plain FP64: evaluation CTAs per SM the registers are budgeted for,
@@ -88,7 +88,7 @@ typedef struct cmg_voxel_stats {
     int brick;                 /* brick edge used */
     int grab;                  /* sub-bricks per work-queue grab used (16^3 bricks) */
     double max_error_bound;    /* mixed: largest stated per-cell bound (0 for FP64) */
-    int walk_warps;            /* warps per brick of the candidate walk used */
+    int walk_warps;            /* warps per brick of the walk (a batch: the first mesh's) */
     int probe;                 /* probe head asked for (0: the whole list) */
     int ctas;                  /* evaluation CTAs per SM used (16^3 bricks) */
 } cmg_voxel_stats;
