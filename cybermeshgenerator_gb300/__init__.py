@@ -302,19 +302,15 @@ def voxelize(plc: PLC, resolution: int = 64, mode="occupancy", pad: int = 1) -> 
     code, name = _mode(mode)
     out = ctypes.c_void_p()
     err = ctypes.create_string_buffer(256)
-    _check(_clib.cmg_plc_voxelize(plc._handle, int(resolution), code, int(pad), ctypes.byref(out),
-                                 err, 256), err)
-    h = out.value
-    try:
-        dims, origin, spacing = _geometry(h)
-        n = dims[0] * dims[1] * dims[2]
-        if code == 0:
-            flat = np.ctypeslib.as_array(_clib.cmg_voxels_occupancy(h), (n,)).astype(np.uint8)
-        else:
-            flat = np.ctypeslib.as_array(_clib.cmg_voxels_distance(h), (n,)).astype(np.float32)
-        grid = _to_xyz(flat, dims)
-    finally:
-        _clib.cmg_voxels_destroy(h)
+    _check(_clib.cmg_plc_voxelize_xyz(plc._handle, int(resolution), code, int(pad), ctypes.byref(out),
+                                     err, 256), err)
+    # the array views the handle's page-locked block (no host copy: the device wrote it in
+    # this order), which lives as long as the array
+    h, owner = out.value, _Owner(out.value)
+    dims, origin, spacing = _geometry(h)
+    fn, dtype = (_clib.cmg_voxels_occupancy, np.uint8) if code == 0 else (_clib.cmg_voxels_distance, np.float32)
+    ptr = ctypes.cast(fn(h), ctypes.c_void_p).value
+    grid = np.asarray(_View(owner, ptr, dims[0] * dims[1] * dims[2], dtype)).reshape(dims)
     return VoxelGrid(grid=grid, origin=origin, spacing=spacing, mode=name)
 
 

@@ -23,7 +23,7 @@ BUILD = os.path.join(ROOT, "_build")
 LIB = os.path.join(HERE, "libcmg_c.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU_SOURCES = ["scan.cu", "occupancy.cu", "sdf.cu", "sdf_sub.cu", "sdf_near.cu", "engine.cu", "peak.cu", "noalloc.cu", "predicates.cu", "adjoint.cu", "stl.cu", "detect.cu", "simplify.cu", "sizing.cu"]
+CU_SOURCES = ["scan.cu", "occupancy.cu", "sdf.cu", "sdf_sub.cu", "sdf_near.cu", "layout.cu", "engine.cu", "peak.cu", "noalloc.cu", "predicates.cu", "adjoint.cu", "stl.cu", "detect.cu", "simplify.cu", "sizing.cu"]
 # per-file flags: sizing.cu rounds every product and sum separately, as the reference does
 CU_FLAGS = {"sizing.cu": ["-fmad=false"]}
 CXX_SOURCES = ["cmg_c.cpp", "cmg_cpp.cpp"]
@@ -76,7 +76,7 @@ def build(jobs: int | None = None, verbose: bool = False) -> str:
         s, o = os.path.join(CSRC, src), os.path.join(BUILD, src + ".o")
         objs.append(o)
         if _stale(o, [s] + headers):
-            steps.append(["g++", "-O2", CXX_STD.get(src, "-std=c++17"), "-fPIC", "-ffp-contract=off",
+            steps.append(["g++", "-O3", CXX_STD.get(src, "-std=c++17"), "-fPIC", "-ffp-contract=off",
                           "-fvisibility=default", "-I" + inc, "-I" + os.path.join(ROOT, "include"),
                           "-c", s, "-o", o])
     with cf.ThreadPoolExecutor(max_workers=jobs or os.cpu_count() or 4) as ex:

@@ -51,6 +51,7 @@ struct cmg_plc {
     cmg::gpu::HostVec<int> markers;
     std::vector<double> holes;
     std::vector<Region> regions;
+    bool triangles = true;                 // every facet has three corners: fidx is the fan
     cmg::gpu::HostVec<double> pts_cache;
     cmg::gpu::HostVec<int> tri_cache;
 };
@@ -142,19 +143,14 @@ cudaStream_t gpu_stream() {
 // (src/voxelize/voxelize.cpp:29-38).
 cmg::gpu::HostVec<int> fan(const cmg_plc& p) {
     const size_t nf = p.foff.size() - 1;
+    if (p.triangles) return p.fidx;
     size_t total = 0;
-    bool all3 = true;
     for (size_t f = 0; f < nf; ++f) {
         const size_t n = p.foff[f + 1] - p.foff[f];
         total += n >= 3 ? 3 * (n - 2) : 0;
-        all3 = all3 && n == 3;
     }
     cmg::gpu::HostVec<int> t(total);
     if (total == 0) return t;
-    if (all3 && total == p.fidx.size()) {  // every facet a triangle: as stored
-        std::memcpy(t.data(), p.fidx.data(), sizeof(int) * total);
-        return t;
-    }
     size_t o = 0;
     for (size_t f = 0; f < nf; ++f) {
         const int* v = p.fidx.data() + p.foff[f];
@@ -171,13 +167,32 @@ cmg::gpu::HostVec<int> fan(const cmg_plc& p) {
 // make_grid (src/voxelize/voxelize.cpp:52-74), same operations in the same order;
 // pts holds n points of 3 coordinates (n >= 1).
 bool make_grid(const double* pts, size_t n, int resolution, int pad, GridDesc& g) {
-    double lo[3] = {pts[0], pts[1], pts[2]}, hi[3] = {pts[0], pts[1], pts[2]};
-    for (size_t i = 0; i < n; ++i)
-        for (int a = 0; a < 3; ++a) {
-            double v = pts[3 * i + a];
-            if (v < lo[a]) lo[a] = v;
-            if (v > hi[a]) hi[a] = v;
+    // eight points at a time, each coordinate its own minimum and maximum, all starting from the
+    // first point (independent comparisons, which the compiler runs as vectors); the minimum
+    // of those in order is the minimum in order
+    constexpr size_t kB = 24;
+    double pl[kB], ph[kB];
+    for (size_t j = 0; j < kB; ++j) pl[j] = ph[j] = pts[j % 3];
+    size_t i = 0;
+    for (; i + kB <= 3 * n; i += kB)
+        for (size_t j = 0; j < kB; ++j) {
+            const double v = pts[i + j];
+            pl[j] = v < pl[j] ? v : pl[j];
+            ph[j] = v > ph[j] ? v : ph[j];
         }
+    for (size_t j = 0; i < 3 * n; ++i, ++j) {
+        pl[j] = pts[i] < pl[j] ? pts[i] : pl[j];
+        ph[j] = pts[i] > ph[j] ? pts[i] : ph[j];
+    }
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = pl[a];
+        hi[a] = ph[a];
+        for (size_t j = a + 3; j < kB; j += 3) {
+            if (pl[j] < lo[a]) lo[a] = pl[j];
+            if (ph[j] > hi[a]) hi[a] = ph[j];
+        }
+    }
     double ext = 0;
     for (int a = 0; a < 3; ++a) ext = std::max(ext, hi[a] - lo[a]);
     g = GridDesc{};
@@ -206,14 +221,28 @@ void check_mesh(int64_t npts, const int* tris, int64_t ntris) {
     if (npts == 0) throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: PLC has no points"};
     if (ntris == 0)
         throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: PLC has no boundary triangles"};
-    for (int64_t i = 0; i < 3 * ntris; ++i)
-        if (tris[i] < 0 || tris[i] >= npts)
-            throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: facet vertex index out of range"};
+    // the largest index as unsigned (a negative one is larger than any count)
+    constexpr int kB = 32;
+    unsigned top[kB] = {};
+    int64_t i = 0;
+    for (; i + kB <= 3 * ntris; i += kB)
+        for (int j = 0; j < kB; ++j) {
+            const unsigned v = static_cast<unsigned>(tris[i + j]);
+            top[j] = v > top[j] ? v : top[j];
+        }
+    unsigned m = 0;
+    for (; i < 3 * ntris; ++i) m = std::max(m, static_cast<unsigned>(tris[i]));
+    for (unsigned v : top) m = std::max(m, v);
+    if (m > static_cast<unsigned>(INT32_MAX) || static_cast<int64_t>(m) >= npts)
+        throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: facet vertex index out of range"};
 }
 
-cmg::gpu::HostVec<int> checked_triangles(const cmg_plc& p) {
+// The PLC's fan triangles, checked: its own index array when every facet is a triangle
+// (`own` stays empty), else in `own`.
+const cmg::gpu::HostVec<int>& checked_triangles(const cmg_plc& p, cmg::gpu::HostVec<int>& own) {
     if (p.points.empty()) throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: PLC has no points"};
-    cmg::gpu::HostVec<int> t = fan(p);
+    if (!p.triangles) own = fan(p);
+    const cmg::gpu::HostVec<int>& t = p.triangles ? p.fidx : own;
     check_mesh(static_cast<int64_t>(p.points.size() / 3), t.data(), static_cast<int64_t>(t.size() / 3));
     return t;
 }
@@ -302,8 +331,9 @@ bool has_layers(const cmg_voxel_opts& o) { return o.z_begin != 0 || o.z_end != 0
 
 // One voxelization of host arrays: pts (npts points of 3 coordinates), tris (ntris
 // triangles of 3 indices, already fanned and checked).
+// xyz: the arrays with x slowest and z fastest.
 cmg_voxels* voxelize_arrays(const double* pts, int64_t npts, const int* tris, int64_t ntris,
-                            const cmg_voxel_opts& o) {
+                            const cmg_voxel_opts& o, bool xyz = false) {
     GridDesc g{};
     if (o.explicit_grid) {
         for (int a = 0; a < 3; ++a) g.corner[a] = o.corner[a];
@@ -319,6 +349,7 @@ cmg_voxels* voxelize_arrays(const double* pts, int64_t npts, const int* tris, in
     set_layers(o, g);
     const int outputs = effective_outputs(o);
     cmg::gpu::VoxOpts vo = to_vox(o, outputs);
+    vo.xyz = xyz;
     cmg::gpu::HostMesh m;
     m.pts = pts;
     m.npts = npts;
@@ -340,12 +371,13 @@ cmg_voxels* voxelize_arrays(const double* pts, int64_t npts, const int* tris, in
     return v.release();
 }
 
-cmg_voxels* voxelize_one(const cmg_plc& p, const cmg_voxel_opts& o) {
+cmg_voxels* voxelize_one(const cmg_plc& p, const cmg_voxel_opts& o, bool xyz = false) {
     if (!o.explicit_grid && o.resolution < 1)
         throw CoreError{CMG_ERR_INVALID_INPUT, "voxelize: resolution must be >= 1"};
-    cmg::gpu::HostVec<int> tris = checked_triangles(p);
+    cmg::gpu::HostVec<int> own;
+    const cmg::gpu::HostVec<int>& tris = checked_triangles(p, own);
     return voxelize_arrays(p.points.data(), static_cast<int64_t>(p.points.size() / 3), tris.data(),
-                           static_cast<int64_t>(tris.size() / 3), o);
+                           static_cast<int64_t>(tris.size() / 3), o, xyz);
 }
 
 template <typename F>
@@ -431,6 +463,7 @@ cmg_status cmg_plc_add_facet(cmg_plc* plc, const int* idx, size_t count, int mar
     if (!plc || (!idx && count)) return CMG_ERR_INVALID_INPUT;
     if (count < 3) return CMG_ERR_INVALID_INPUT;
     try {
+        plc->triangles = plc->triangles && count == 3;
         plc->fidx.insert(plc->fidx.end(), idx, idx + count);
         plc->foff.push_back(plc->fidx.size());
         plc->markers.push_back(marker);
@@ -499,8 +532,9 @@ void cmg_voxel_opts_init(cmg_voxel_opts* o) {
     o->stage = -1;
 }
 
-cmg_status cmg_plc_voxelize(const cmg_plc* in, int resolution, int mode, int pad,
-                            cmg_voxels** out, char* errbuf, size_t len) {
+namespace {
+cmg_status plc_voxelize(const cmg_plc* in, int resolution, int mode, int pad, bool xyz,
+                        cmg_voxels** out, char* errbuf, size_t len) {
     if (out) *out = nullptr;
     if (!in || !out) return CMG_ERR_INVALID_INPUT;
     if (resolution < 1) {
@@ -512,7 +546,18 @@ cmg_status cmg_plc_voxelize(const cmg_plc* in, int resolution, int mode, int pad
     o.resolution = resolution;
     o.pad = pad;
     o.mode = mode == 1 ? 1 : 0;
-    return guarded(errbuf, len, [&] { *out = voxelize_one(*in, o); });
+    return guarded(errbuf, len, [&] { *out = voxelize_one(*in, o, xyz); });
+}
+}  // namespace
+
+cmg_status cmg_plc_voxelize(const cmg_plc* in, int resolution, int mode, int pad,
+                            cmg_voxels** out, char* errbuf, size_t len) {
+    return plc_voxelize(in, resolution, mode, pad, false, out, errbuf, len);
+}
+
+cmg_status cmg_plc_voxelize_xyz(const cmg_plc* in, int resolution, int mode, int pad,
+                                cmg_voxels** out, char* errbuf, size_t len) {
+    return plc_voxelize(in, resolution, mode, pad, true, out, errbuf, len);
 }
 
 cmg_status cmg_plc_voxelize_ex(const cmg_plc* in, const cmg_voxel_opts* opts, cmg_voxels** out,
@@ -628,7 +673,7 @@ cmg_status cmg_batch_create(const cmg_plc* const* plcs, const int* resolutions, 
         for (int i = 0; i < n; ++i) {
             if (!plcs[i]) throw CoreError{CMG_ERR_INVALID_INPUT, "cmg_batch_create: NULL plc"};
             const cmg_plc& p = *plcs[i];
-            tris[i] = checked_triangles(p);
+            const cmg::gpu::HostVec<int>& t = checked_triangles(p, tris[i]);
             GridDesc g{};
             if (opts->explicit_grid) {
                 for (int a = 0; a < 3; ++a) g.corner[a] = opts->corner[a];
@@ -645,8 +690,8 @@ cmg_status cmg_batch_create(const cmg_plc* const* plcs, const int* resolutions, 
             check_grid_size(g);
             meshes[i].pts = p.points.data();
             meshes[i].npts = static_cast<int64_t>(p.points.size() / 3);
-            meshes[i].tris = tris[i].data();
-            meshes[i].ntris = static_cast<int64_t>(tris[i].size() / 3);
+            meshes[i].tris = t.data();
+            meshes[i].ntris = static_cast<int64_t>(t.size() / 3);
             meshes[i].g = g;
             b->grids.push_back(g);
         }

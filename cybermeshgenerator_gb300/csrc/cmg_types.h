@@ -61,6 +61,7 @@ struct Stats {
     unsigned long long orient_calls;       // occupancy filter: orient3d evaluations
     unsigned long long crossings;          // occupancy filter: plane_z evaluations
     unsigned long long filtered;           // SDF: sub-brick list entries (sphere tests per cell)
+    unsigned long long pairs;              // occupancy: (triangle, column) pairs
 };
 
 enum : int { kPredCompat = 0, kPredExact = 1 };

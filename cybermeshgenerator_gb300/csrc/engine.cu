@@ -192,6 +192,8 @@ int sub_precision(const VoxOpts& o) {
 // serialised by the caller), so repeated single calls do not re-allocate.
 struct Pool {
     Arena a[4];
+    cudaStream_t side = nullptr;  // the second stream of a run, and its fork and join
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 Pool& pool_for_device() {
     static std::mutex mu;
@@ -263,6 +265,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
              bool transient)
     : opts_(opts), stream_(stream) {
     impl_.reset(new Impl(transient ? pool_for_device().a : nullptr));
+    pooled_ = transient;
     bool slab = false;
     for (const HostMesh& m : meshes)
         slab = slab || (m.g.z1 > 0 && (m.g.z0 != 0 || m.g.z1 != m.g.nz));
@@ -295,12 +298,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         // along z only the bricks that overlap the slab
         s.bzo = s.g.z0 / brick;
         s.bnz = (s.g.z1 - 1) / brick + 1 - s.bzo;
-        double sc = 0.0;
-        for (int64_t i = 0; i < m.npts; ++i)
-            for (int a = 0; a < 3; ++a) sc = std::max(sc, std::fabs(m.pts[3 * i + a] - m.g.corner[a]));
-        sc = std::max(sc, m.g.h * std::max(m.g.nx, std::max(m.g.ny, m.g.nz)));
-        s.scale = static_cast<float>(sc * 1.0001);
-        segs_.push_back(s);
+        segs_.push_back(s);  // the scale is found on the device (k_seg_finish)
         tb += m.ntris;
         pb += m.npts;
         ncol_ += static_cast<int64_t>(m.g.nx) * m.g.ny;
@@ -387,6 +385,8 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         near_tri_ = opts_.want_near ? carve<int>(O, nvox_) : nullptr;
         near_reg_ = opts_.want_near ? carve<uint8_t>(O, nvox_) : nullptr;
         err_ = (opts_.want_err && opts_.precision == kPrecMixed) ? carve<float>(O, nvox_) : nullptr;
+        occ_xyz_ = opts_.xyz && opts_.want_occ ? carve<uint8_t>(O, nvox_) : nullptr;
+        sdf32_xyz_ = opts_.xyz && opts_.want_sdf32 ? carve<float>(O, nvox_) : nullptr;
     };
     O.clear_need();
     plan_out();
@@ -397,21 +397,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     if (!opts_.want_occ) occ_ = nullptr;
 
     // ---- upload inputs (indices rebased to the concatenated point array)
-    std::vector<double> hp(static_cast<size_t>(3 * npts_));
-    std::vector<int> ht(static_cast<size_t>(3 * ntris_));
-    int64_t po = 0, to = 0;
-    for (const HostMesh& m : meshes) {
-        std::memcpy(hp.data() + 3 * po, m.pts, sizeof(double) * 3 * m.npts);
-        for (int64_t i = 0; i < 3 * m.ntris; ++i) ht[3 * to + i] = m.tris[i] + static_cast<int>(po);
-        po += m.npts;
-        to += m.ntris;
-    }
-    CMG_CUDA(cudaMemcpyAsync(pts_, hp.data(), sizeof(double) * hp.size(), cudaMemcpyHostToDevice, stream_));
-    CMG_CUDA(cudaMemcpyAsync(tris_, ht.data(), sizeof(int) * ht.size(), cudaMemcpyHostToDevice, stream_));
-    CMG_CUDA(cudaMemcpyAsync(dsegs_, segs_.data(), sizeof(MeshSeg) * segs_.size(),
-                             cudaMemcpyHostToDevice, stream_));
-    CMG_CUDA(cudaStreamSynchronize(stream_));  // host vectors go out of scope
-    h2d_bytes_ = static_cast<int64_t>(sizeof(double) * hp.size() + sizeof(int) * ht.size());
+    upload(meshes);
 
     const int sms = device_sms();
     impl_->grid_exact = 2 * sms;
@@ -424,20 +410,66 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     }
     else impl_->grid_eval = (brick == 4 ? 8 : 3) * sms;
     if (sdf) {  // made here: a graph capture must not create them
-        CMG_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
-        CMG_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
-        CMG_CUDA(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
+        auto make = [](cudaStream_t& side, cudaEvent_t& fork, cudaEvent_t& join) {
+            if (!side) CMG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+            if (!fork) CMG_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+            if (!join) CMG_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+        };
+        if (pooled_) {
+            Pool& p = pool_for_device();
+            make(p.side, p.fork, p.join);
+            side_ = p.side;
+            fork_ = p.fork;
+            join_ = p.join;
+        } else {
+            make(side_, fork_, join_);
+        }
     }
+}
+
+// The meshes' points and triangles to the device. One mesh is copied from where it lies (a
+// pooled batch's caller keeps it until the results are there); several are staged in a
+// page-locked block, where the indices are rebased.
+void Batch::upload(const std::vector<HostMesh>& meshes) {
+    const size_t nb = sizeof(double) * 3 * static_cast<size_t>(npts_), tb = sizeof(int) * 3 * static_cast<size_t>(ntris_);
+    CMG_CUDA(cudaMemcpyAsync(dsegs_, segs_.data(), sizeof(MeshSeg) * segs_.size(),
+                             cudaMemcpyHostToDevice, stream_));
+    in_flight_ = true;
+    if (meshes.size() == 1) {
+        if (nb) CMG_CUDA(cudaMemcpyAsync(pts_, meshes[0].pts, nb, cudaMemcpyHostToDevice, stream_));
+        if (tb) CMG_CUDA(cudaMemcpyAsync(tris_, meshes[0].tris, tb, cudaMemcpyHostToDevice, stream_));
+        if (!pooled_) CMG_CUDA(cudaStreamSynchronize(stream_));
+    } else {
+        HostBuf<char> stage;
+        stage.resize(nb + tb + 1);
+        double* hp = reinterpret_cast<double*>(stage.data());
+        int* ht = reinterpret_cast<int*>(stage.data() + nb);
+        int po = 0;
+        for (const HostMesh& m : meshes) {
+            std::memcpy(hp, m.pts, sizeof(double) * 3 * static_cast<size_t>(m.npts));
+            for (int64_t i = 0; i < 3 * m.ntris; ++i) ht[i] = m.tris[i] + po;
+            hp += 3 * m.npts;
+            ht += 3 * m.ntris;
+            po += static_cast<int>(m.npts);
+        }
+        CMG_CUDA(cudaMemcpyAsync(pts_, stage.data(), nb, cudaMemcpyHostToDevice, stream_));
+        CMG_CUDA(cudaMemcpyAsync(tris_, stage.data() + nb, tb, cudaMemcpyHostToDevice, stream_));
+        CMG_CUDA(cudaStreamSynchronize(stream_));  // the block goes back to the pool
+    }
+    h2d_bytes_ = static_cast<int64_t>(nb + tb);
 }
 
 Batch::~Batch() {
     for (cudaEvent_t& e : ev_)
         if (e) cudaEventDestroy(e);
-    if (fork_) cudaEventDestroy(fork_);
-    if (join_) cudaEventDestroy(join_);
-    if (side_) {
-        if (side_open_) cudaStreamSynchronize(side_);  // pooled arenas are reused next
-        cudaStreamDestroy(side_);
+    if (side_ && side_open_) cudaStreamSynchronize(side_);  // pooled arenas are reused next
+    if (pooled_) {
+        // a call that ended in an error may leave copies of the caller's arrays under way
+        if (in_flight_) cudaStreamSynchronize(stream_);
+    } else {
+        if (fork_) cudaEventDestroy(fork_);
+        if (join_) cudaEventDestroy(join_);
+        if (side_) cudaStreamDestroy(side_);
     }
     if (graph_) cudaGraphExecDestroy(graph_);
     if (impl_ && impl_->graph) cudaGraphDestroy(impl_->graph);
@@ -476,9 +508,50 @@ void Batch::sized_run() {
     }
 }
 
+// Pair and candidate arrays of n entries in their arenas (nothing is allocated here).
+void Batch::plan_pairs(size_t n) {
+    Arena& B = impl_->pairs;
+    B.reset();
+    impl_->col_list = carve<int>(B, n);
+    impl_->hs = carve<double>(B, n);
+    impl_->hv = carve<uint8_t>(B, n);
+    pairs_cap_ = static_cast<int64_t>(n);
+}
+void Batch::plan_cands(size_t n) {
+    const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
+    impl_->cands.reset();
+    impl_->cand = carve<int>(impl_->cands, n);
+    impl_->cand_c = near_list ? carve<float4>(impl_->cands, n) : nullptr;
+    cand_cap_ = static_cast<int64_t>(n);
+}
+
+// Bytes of an arena per entry, and the entries that fit (a few 256-byte roundings aside).
+static constexpr size_t kPairBytes = sizeof(int) + sizeof(double) + 1, kCandBytes = sizeof(int) + sizeof(float4);
+static size_t entries_of(const Arena& a, size_t each) {
+    return a.capacity() > 4096 ? (a.capacity() - 1024) / each : 0;
+}
+
 void Batch::run() {
-    if (needs_sizing()) sized_run();
-    else run_impl(false);
+    if (!needs_sizing()) {
+        run_impl(false);
+    } else if (pooled_ && entries_of(impl_->pairs, kPairBytes) > 0 &&
+               (!(sdf32_ || sdf64_ || near_tri_) || entries_of(impl_->cands, kCandBytes) > 0)) {
+        // A pooled batch runs into what the pool's arenas hold, without a readback between its
+        // passes; a mesh with longer lists than they take is sized and run again (download)
+        plan_pairs(entries_of(impl_->pairs, kPairBytes));
+        plan_cands(entries_of(impl_->cands, kCandBytes));
+        unchecked_ = true;
+        run_impl(false);
+    } else {
+        sized_run();
+    }
+    finish_xyz();
+}
+
+void Batch::finish_xyz() {
+    const GridDesc& g = segs_[0].g;
+    if (occ_xyz_) launch_to_xyz(occ_, g.nx, g.ny, g.z1 - g.z0, occ_xyz_, stream_);
+    if (sdf32_xyz_) launch_to_xyz(sdf32_, g.nx, g.ny, g.z1 - g.z0, sdf32_xyz_, stream_);
 }
 
 void Batch::run_graph() {
@@ -525,30 +598,24 @@ void Batch::run_impl(bool sizing) {
         int64_t P = 0;
         CMG_CUDA(cudaMemcpyAsync(&P, I.pair_off + ntris_, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         CMG_CUDA(cudaStreamSynchronize(s));
-        Arena& B = I.pairs;
-        auto planb = [&]() {
-            B.reset();
-            I.col_list = carve<int>(B, P);
-            I.hs = carve<double>(B, P);
-            I.hv = carve<uint8_t>(B, P);
-        };
-        B.clear_need();
-        planb();
-        if (B.overflowed()) {
-            B.reserve(B.need());
-            planb();
+        I.pairs.clear_need();
+        plan_pairs(static_cast<size_t>(P));
+        if (I.pairs.overflowed()) {
+            pairs_cap_ = -1;  // until the allocation has succeeded
+            // (an eighth to spare: the next pooled call runs into what is there)
+            I.pairs.reserve(I.pairs.need() + (pooled_ ? I.pairs.need() / 8 + 4096 : 0));
+            plan_pairs(static_cast<size_t>(P));
         }
-        pairs_cap_ = P;
     };
     auto occ_tail = [&](cudaStream_t s) {
         const int pair_grid = 4 * device_sms();
         launch_col_pairs(false, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, nullptr, nullptr,
-                         pair_grid, s);
+                         pairs_cap_, stats_, pair_grid, s);
         exclusive_scan(I.colcnt, I.col_off, ncol_, I.scan_tmp, s);
         launch_col_pairs(true, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, I.col_off,
-                         I.col_list, pair_grid, s);
+                         I.col_list, pairs_cap_, stats_, pair_grid, s);
         launch_occ_filter(opts_.predicates, dsegs_, nseg, nrow_, I.soup, I.col_off, I.col_list, occ,
-                          I.flagged, stats_, s);
+                          I.flagged, pairs_cap_, stats_, s);
         launch_occ_exact(opts_.predicates, dsegs_, nseg, I.soup, I.col_off, I.col_list, I.flagged,
                          I.hs, I.hv, occ, stats_, I.grid_exact, s);
         if (timed) CMG_CUDA(cudaEventRecord(ev_[1], s));
@@ -580,18 +647,7 @@ void Batch::run_impl(bool sizing) {
                           I.bin_info, I.bin_ball, I.bin_reach, I.large_list, I.cand_cnt, I.cand_rng, I.cand,
                           I.cand_c, cand_cap_, I.brick_emax, stats_, ss);
     };
-    const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
-    auto plan_cands = [&](size_t n) {
-        I.cands.reset();
-        I.cand = carve<int>(I.cands, n);
-        I.cand_c = near_list ? carve<float4>(I.cands, n) : nullptr;
-        cand_cap_ = static_cast<int64_t>(n);
-    };
-    // the first sizing run walks into whatever the arena holds (a pooled one is seldom empty)
-    if (sizing && cand_cap_ < 0) {
-        const size_t each = near_list ? 20 : 4, have = I.cands.capacity();
-        plan_cands(have > 4096 ? (have - 1024) / each : 0);
-    }
+    if (cand_cap_ < 0) plan_cands(entries_of(I.cands, kCandBytes));
     // reads the walk's total back; lists that did not fit are sized (with an eighth to
     // spare, for points that move) and walked again
     auto prep_size = [&]() {
@@ -603,7 +659,7 @@ void Batch::run_impl(bool sizing) {
         I.cands.clear_need();
         plan_cands(n);
         if (I.cands.overflowed()) {
-            cand_cap_ = 0;  // a failed allocation leaves no list
+            cand_cap_ = -1;  // until the allocation has succeeded
             I.cands.reserve(I.cands.need());
             plan_cands(n);
         }
@@ -693,9 +749,15 @@ int64_t Batch::d2h_bytes() const {
 }
 
 RunInfo Batch::info() {
-    RunInfo r;
-    CMG_CUDA(cudaMemcpyAsync(&r.stats, stats_, sizeof(Stats), cudaMemcpyDeviceToHost, stream_));
+    Stats s;
+    CMG_CUDA(cudaMemcpyAsync(&s, stats_, sizeof(Stats), cudaMemcpyDeviceToHost, stream_));
     CMG_CUDA(cudaStreamSynchronize(stream_));
+    return info_of(s);
+}
+
+RunInfo Batch::info_of(const Stats& s) const {
+    RunInfo r;
+    r.stats = s;
     r.brick = opts_.brick;
     r.grab = opts_.brick == 16 ? opts_.grab : 0;
     r.walk_warps = segs_[0].walk_warps;
@@ -703,12 +765,13 @@ RunInfo Batch::info() {
     r.probe = plain || opts_.brick != 16 ? 0 : std::max(opts_.probe, 0);
     r.ctas = opts_.brick != 16 ? 0 : (plain ? sdf_sub_minb(opts_.ctas) : impl_->grid_eval / device_sms());
     r.cells = nvox_;
-    r.pairs = pairs_cap_;
+    r.pairs = static_cast<int64_t>(r.stats.pairs);
     r.candidates = static_cast<int64_t>(r.stats.candidates);
     return r;
 }
 
-void Batch::download_one(int m, HostResult& r) {
+// Enqueues the copies of mesh m's outputs.
+void Batch::fetch(int m, HostResult& r) {
     const MeshSeg& s = segs_[static_cast<size_t>(m)];
     const int64_t n = slab_cells(s.g);
     auto get = [&](auto* dev, auto& vec) {
@@ -717,19 +780,38 @@ void Batch::download_one(int m, HostResult& r) {
         CMG_CUDA(cudaMemcpyAsync(vec.data(), dev + s.vox_begin, sizeof(vec[0]) * n,
                                  cudaMemcpyDeviceToHost, stream_));
     };
-    get(occ_, r.occ);
-    get(sdf32_, r.sdf32);
+    get(occ_xyz_ ? occ_xyz_ : occ_, r.occ);
+    get(sdf32_xyz_ ? sdf32_xyz_ : sdf32_, r.sdf32);
     get(sdf64_, r.sdf64);
     get(near_tri_, r.near_tri);
     get(near_reg_, r.near_reg);
     get(err_, r.err);
+}
+
+void Batch::download_one(int m, HostResult& r) {
+    fetch(m, r);
     CMG_CUDA(cudaStreamSynchronize(stream_));
 }
 
 void Batch::download(std::vector<HostResult>& out, RunInfo* info) {
     out.resize(segs_.size());
-    for (size_t m = 0; m < segs_.size(); ++m) download_one(static_cast<int>(m), out[m]);
-    if (info) *info = this->info();
+    for (;;) {
+        for (size_t m = 0; m < segs_.size(); ++m) fetch(static_cast<int>(m), out[m]);
+        Stats s;
+        CMG_CUDA(cudaMemcpyAsync(&s, stats_, sizeof(Stats), cudaMemcpyDeviceToHost, stream_));
+        CMG_CUDA(cudaStreamSynchronize(stream_));
+        const bool fitted = static_cast<int64_t>(s.pairs) <= pairs_cap_ && static_cast<int64_t>(s.candidates) <= cand_cap_;
+        if (!unchecked_ || fitted) {
+            unchecked_ = in_flight_ = false;
+            if (info) *info = info_of(s);
+            return;
+        }
+        unchecked_ = false;
+        pairs_cap_ = cand_cap_ = -1;
+        resize_ = true;  // the sizing run, whatever the arenas hold
+        sized_run();
+        finish_xyz();
+    }
 }
 
 // ------------------------------------------------------------------ autotuner

@@ -37,6 +37,8 @@ struct VoxOpts {
     bool want_sdf64 = false;
     bool want_near = false;        // nearest triangle id + Ericson region per cell
     bool want_err = false;         // mixed: stated per-cell FP32 error bound
+    bool xyz = false;              // one mesh: occupancy and float distances are downloaded
+                                   // with x slowest and z fastest (idx = (i*ny + j)*nz + k)
     bool autotune = false;
     int grab = 0;                  // sub-bricks per queue grab (1, 2, 4, 8); 0 = default
     int stage = -1;                // no effect (records are always staged)
@@ -213,6 +215,10 @@ private:
     int64_t npts_ = 0, ntris_ = 0, ncol_ = 0, nrow_ = 0, nvox_ = 0, nbrick_ = 0, nwork_ = 0, nwalk_ = 0;
     int64_t pairs_cap_ = -1, cand_cap_ = -1;
     bool resize_ = false;  // points moved since the workspace was sized
+    bool pooled_ = false;     // the arenas, second stream and events are the device pool's
+    // a pooled run into whatever its arenas held: download() checks that it fitted
+    bool unchecked_ = false;
+    bool in_flight_ = false;  // a pooled batch's inputs may still be being copied
     double* pts_ = nullptr;
     int* tris_ = nullptr;
     MeshSeg* dsegs_ = nullptr;
@@ -222,6 +228,8 @@ private:
     int* near_tri_ = nullptr;
     uint8_t* near_reg_ = nullptr;
     float* err_ = nullptr;
+    uint8_t* occ_xyz_ = nullptr;
+    float* sdf32_xyz_ = nullptr;
     Stats* stats_ = nullptr;
     unsigned long long* queue_ = nullptr;
     cudaGraphExec_t graph_ = nullptr;
@@ -239,6 +247,12 @@ private:
     void run_impl(bool sizing);
     bool needs_sizing() const { return pairs_cap_ < 0 || cand_cap_ < 0 || resize_; }
     void sized_run();
+    void upload(const std::vector<HostMesh>& meshes);
+    void fetch(int m, HostResult& r);
+    void finish_xyz();
+    RunInfo info_of(const Stats& s) const;
+    void plan_pairs(size_t n);
+    void plan_cands(size_t n);
 };
 
 // Sets opts.brick, grab, walk_warps and ctas for a workload by timing the

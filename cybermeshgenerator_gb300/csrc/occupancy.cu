@@ -145,13 +145,15 @@ __global__ void k_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64_t n
 }
 
 // FILL=false: count bucket sizes into the zeroed colcnt; FILL=true: write bucket entries,
-// taking the counts down to zero again.
+// taking the counts down to zero again. More than cap pairs: nothing (st->pairs says so).
 template <bool FILL>
 __global__ void k_col_pairs(const MeshSeg* __restrict__ segs, int nseg, int64_t ntris,
                             const int4* __restrict__ xybox, const int64_t* __restrict__ pair_off,
                             int* __restrict__ colcnt, const int64_t* __restrict__ col_off,
-                            int* __restrict__ col_list) {
+                            int* __restrict__ col_list, int64_t cap, Stats* __restrict__ st) {
     const int64_t npairs = pair_off[ntris];
+    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) st->pairs = static_cast<unsigned long long>(npairs);
+    if (npairs > cap) return;
     for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < npairs;
          p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         int64_t t = last_le(pair_off, ntris, p);
@@ -172,12 +174,12 @@ template <int MODE>
 __global__ void __launch_bounds__(kOccThreads)
 k_occ_filter(const MeshSeg* __restrict__ segs, int nseg, const double* __restrict__ soup,
              const int64_t* __restrict__ col_off, const int* __restrict__ col_list,
-             uint8_t* __restrict__ occ, int64_t* __restrict__ flagged, Stats* __restrict__ st) {
+             uint8_t* __restrict__ occ, int64_t* __restrict__ flagged, int64_t cap, Stats* __restrict__ st) {
     __shared__ double hts[kRowCols][kHCap];
     __shared__ int nbelow[kRowCols][kHCap];
     __shared__ int hcnt[kRowCols];
     __shared__ int cflag[kRowCols];
-    __shared__ unsigned long long* flag_count;
+    if (static_cast<int64_t>(st->pairs) > cap) return;  // the buckets were not written
 
     const int64_t row = blockIdx.x;
     const int si = find_seg<&MeshSeg::row_begin>(segs, nseg, row);
@@ -261,7 +263,6 @@ k_occ_filter(const MeshSeg* __restrict__ segs, int nseg, const double* __restric
             flagged[base + rank] = s.col_begin + static_cast<int64_t>(j) * g.nx + i;
         }
     }
-    (void)flag_count;
 }
 
 // One warp per listed column (grid-stride); scratch hs[e] holds the crossing height
@@ -348,27 +349,27 @@ void launch_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double*
 
 void launch_col_pairs(bool fill, const MeshSeg* segs, int nseg, int64_t ntris, const int4* xybox,
                       const int64_t* pair_off, int* colcnt, const int64_t* col_off, int* col_list,
-                      int grid, cudaStream_t st) {
+                      int64_t cap, Stats* stats, int grid, cudaStream_t st) {
     if (ntris == 0) return;
     if (fill)
         k_col_pairs<true><<<grid, 256, 0, st>>>(segs, nseg, ntris, xybox, pair_off, colcnt, col_off,
-                                                col_list);
+                                                col_list, cap, stats);
     else
         k_col_pairs<false><<<grid, 256, 0, st>>>(segs, nseg, ntris, xybox, pair_off, colcnt, col_off,
-                                                 col_list);
+                                                 col_list, cap, stats);
     CMG_LAUNCH();
 }
 
 void launch_occ_filter(int mode, const MeshSeg* segs, int nseg, int64_t nrows, const double* soup,
                        const int64_t* col_off, const int* col_list, uint8_t* occ, int64_t* flagged,
-                       Stats* stats, cudaStream_t st) {
+                       int64_t cap, Stats* stats, cudaStream_t st) {
     if (nrows == 0) return;
     if (mode == kPredExact)
         k_occ_filter<kPredExact><<<static_cast<unsigned>(nrows), kOccThreads, 0, st>>>(
-            segs, nseg, soup, col_off, col_list, occ, flagged, stats);
+            segs, nseg, soup, col_off, col_list, occ, flagged, cap, stats);
     else
         k_occ_filter<kPredCompat><<<static_cast<unsigned>(nrows), kOccThreads, 0, st>>>(
-            segs, nseg, soup, col_off, col_list, occ, flagged, stats);
+            segs, nseg, soup, col_off, col_list, occ, flagged, cap, stats);
     CMG_LAUNCH();
 }
 

@@ -93,6 +93,11 @@ typedef struct cmg_voxel_stats {
     int ctas;                  /* evaluation CTAs per SM used (16^3 bricks) */
 } cmg_voxel_stats;
 
+/* cmg_plc_voxelize with the array of the handle in the reference binding's order, x slowest
+ * and z fastest: idx = (i*ny + j)*nz + k (the transposition runs on the GPU). */
+cmg_status cmg_plc_voxelize_xyz(const cmg_plc*, int resolution, int mode, int pad,
+                                cmg_voxels** out, char* errbuf, size_t errbuf_len);
+
 /* Defaults: resolution 64, pad 1, occupancy, FP64, compat predicates, band 1. */
 void cmg_voxel_opts_init(cmg_voxel_opts* opts);
 
