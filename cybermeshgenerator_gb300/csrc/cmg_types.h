@@ -1,6 +1,7 @@
 // cmg_types.h — plain data shared by the host engine and the device kernels.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 namespace cmg::gpu {
@@ -25,6 +26,28 @@ inline int64_t slab_cells(const GridDesc& g) {
     return static_cast<int64_t>(g.nx) * g.ny * (g.z1 - g.z0);
 }
 
+// What the column tests take from a grid, the same on both sides: the segment's ends, the
+// power of two that brings the cell edge into [1, 2) (the scale of the FP32 test; 0 for an
+// edge near the ends of FP32's range, which leaves everything to FP64), and the edge's
+// rounded reciprocals (guesses, never results).
+struct OccFrame {
+    double zmin, zmax;
+    double inv;
+    float s, inv32;
+};
+
+inline OccFrame occ_frame(const GridDesc& g) {
+    OccFrame f;
+    f.zmin = g.corner[2] - g.h;
+    const double top = static_cast<double>(g.nz + 1) * g.h;
+    f.zmax = g.corner[2] + top;
+    f.inv = 1.0 / g.h;
+    const int e = std::isnormal(g.h) ? std::ilogb(g.h) : 1000;
+    f.s = e >= -60 && e <= 60 ? std::ldexp(1.0f, -e) : 0.0f;
+    f.inv32 = f.s > 0.0f ? static_cast<float>(f.inv) : 0.0f;
+    return f;
+}
+
 // One mesh of a batch. Every index range is global (into the concatenated
 // arrays of the batch), so kernels over a flattened index space recover the mesh
 // by a binary search on the corresponding *_begin field.
@@ -44,6 +67,7 @@ struct MeshSeg {
     float emax;                     // max centroid-to-vertex distance of binned triangles
     float emax_all;                 // the same over all the mesh's triangles
     float scale;                    // max |coordinate| of the mesh and grid (error bounds)
+    OccFrame f;
 };
 
 // Counters written by the kernels (device memory, one per batch).

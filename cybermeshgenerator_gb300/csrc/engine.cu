@@ -218,6 +218,7 @@ struct Batch::Impl {
           outs(a ? a[3] : own[3]) {}
     // workspace
     double* soup = nullptr;
+    float4* otri = nullptr;  // the column test's FP32 records
     int4* xybox = nullptr;
     int64_t* pairs_n = nullptr;
     int64_t* pair_off = nullptr;
@@ -286,6 +287,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         }
         if (s.g.z0 < 0 || s.g.z0 >= s.g.z1 || s.g.z1 > s.g.nz)
             throw std::invalid_argument("voxelize: cell layers outside the grid");
+        s.f = occ_frame(s.g);
         s.tri_begin = tb;
         s.tri_end = tb + m.ntris;
         s.col_begin = ncol_;
@@ -312,6 +314,8 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     if (nwork_ >= (int64_t(1) << 32)) throw std::invalid_argument("voxelize: grid too large");
     const int nseg = static_cast<int>(segs_.size());
     const bool sdf = opts_.want_sdf32 || opts_.want_sdf64 || opts_.want_near;
+    if (opts_.xyz && (segs_.size() != 1 || slab || (opts_.want_occ && sdf)))
+        throw std::invalid_argument("voxelize: [x][y][z] order is for one mesh's whole grid and one output");
     for (MeshSeg& s : segs_) {
         const int64_t n = static_cast<int64_t>(s.bnx) * s.bny * s.bnz;
         s.walk_warps = brick_walk_warps(nbrick_, n, s.tri_end - s.tri_begin, opts_.walk_warps);
@@ -337,6 +341,7 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         }
         impl_->zero_end = carve<char>(A, 1);
         impl_->soup = carve<double>(A, kSoupStride * ntris_);
+        impl_->otri = carve<float4>(A, 3 * ntris_);
         impl_->xybox = carve<int4>(A, ntris_);
         impl_->pairs_n = carve<int64_t>(A, ntris_ + 1);
         impl_->pair_off = carve<int64_t>(A, ntris_ + 1);
@@ -385,7 +390,6 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
         near_tri_ = opts_.want_near ? carve<int>(O, nvox_) : nullptr;
         near_reg_ = opts_.want_near ? carve<uint8_t>(O, nvox_) : nullptr;
         err_ = (opts_.want_err && opts_.precision == kPrecMixed) ? carve<float>(O, nvox_) : nullptr;
-        occ_xyz_ = opts_.xyz && opts_.want_occ ? carve<uint8_t>(O, nvox_) : nullptr;
         sdf32_xyz_ = opts_.xyz && opts_.want_sdf32 ? carve<float>(O, nvox_) : nullptr;
     };
     O.clear_need();
@@ -550,7 +554,6 @@ void Batch::run() {
 
 void Batch::finish_xyz() {
     const GridDesc& g = segs_[0].g;
-    if (occ_xyz_) launch_to_xyz(occ_, g.nx, g.ny, g.z1 - g.z0, occ_xyz_, stream_);
     if (sdf32_xyz_) launch_to_xyz(sdf32_, g.nx, g.ny, g.z1 - g.z0, sdf32_xyz_, stream_);
 }
 
@@ -576,6 +579,7 @@ void Batch::run_impl(bool sizing) {
     const int nseg = static_cast<int>(segs_.size());
     const bool sdf = opts_.want_sdf32 || opts_.want_sdf64 || opts_.want_near;
     uint8_t* occ = opts_.want_occ ? occ_ : I.occ_internal;
+    const bool occ_xyz = opts_.xyz && opts_.want_occ;  // (the distances read the cells' order)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CMG_CUDA(cudaStreamIsCapturing(st, &cap));
     const bool timed = timing_ && cap == cudaStreamCaptureStatusNone;
@@ -588,7 +592,8 @@ void Batch::run_impl(bool sizing) {
     if (timed) CMG_CUDA(cudaEventRecord(ev_[0], st));
 
     CMG_CUDA(cudaMemsetAsync(stats_, 0, static_cast<size_t>(I.zero_end - reinterpret_cast<char*>(stats_)), st));
-    launch_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.soup, I.xybox, I.pairs_n, st);
+    launch_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.soup, I.otri, I.xybox,
+                    I.pairs_n, st);
 
     // Ray-parity occupancy: (triangle, column) pairs, filter, exact pass. The pair count
     // sizes the pair arena in a sizing run.
@@ -614,10 +619,10 @@ void Batch::run_impl(bool sizing) {
         exclusive_scan(I.colcnt, I.col_off, ncol_, I.scan_tmp, s);
         launch_col_pairs(true, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, I.col_off,
                          I.col_list, pairs_cap_, stats_, pair_grid, s);
-        launch_occ_filter(opts_.predicates, dsegs_, nseg, nrow_, I.soup, I.col_off, I.col_list, occ,
-                          I.flagged, pairs_cap_, stats_, s);
+        launch_occ_filter(opts_.predicates, dsegs_, nseg, nrow_, I.soup, I.otri, I.col_off,
+                          I.col_list, occ, occ_xyz, I.flagged, pairs_cap_, stats_, s);
         launch_occ_exact(opts_.predicates, dsegs_, nseg, I.soup, I.col_off, I.col_list, I.flagged,
-                         I.hs, I.hv, occ, stats_, I.grid_exact, s);
+                         I.hs, I.hv, occ, occ_xyz, stats_, I.grid_exact, s);
         if (timed) CMG_CUDA(cudaEventRecord(ev_[1], s));
     };
     if (!sdf) {
@@ -780,7 +785,7 @@ void Batch::fetch(int m, HostResult& r) {
         CMG_CUDA(cudaMemcpyAsync(vec.data(), dev + s.vox_begin, sizeof(vec[0]) * n,
                                  cudaMemcpyDeviceToHost, stream_));
     };
-    get(occ_xyz_ ? occ_xyz_ : occ_, r.occ);
+    get(occ_, r.occ);
     get(sdf32_xyz_ ? sdf32_xyz_ : sdf32_, r.sdf32);
     get(sdf64_, r.sdf64);
     get(near_tri_, r.near_tri);

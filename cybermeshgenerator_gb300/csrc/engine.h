@@ -37,8 +37,8 @@ struct VoxOpts {
     bool want_sdf64 = false;
     bool want_near = false;        // nearest triangle id + Ericson region per cell
     bool want_err = false;         // mixed: stated per-cell FP32 error bound
-    bool xyz = false;              // one mesh: occupancy and float distances are downloaded
-                                   // with x slowest and z fastest (idx = (i*ny + j)*nz + k)
+    bool xyz = false;              // one mesh's whole grid, occupancy or distances: the array
+                                   // has x slowest and z fastest (idx = (i*ny + j)*nz + k)
     bool autotune = false;
     int grab = 0;                  // sub-bricks per queue grab (1, 2, 4, 8); 0 = default
     int stage = -1;                // no effect (records are always staged)
@@ -228,7 +228,6 @@ private:
     int* near_tri_ = nullptr;
     uint8_t* near_reg_ = nullptr;
     float* err_ = nullptr;
-    uint8_t* occ_xyz_ = nullptr;
     float* sdf32_xyz_ = nullptr;
     Stats* stats_ = nullptr;
     unsigned long long* queue_ = nullptr;

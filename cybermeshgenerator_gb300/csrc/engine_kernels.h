@@ -17,21 +17,23 @@ int device_sms();
 
 // layout.cu: a grid of nx * ny * nz cells from idx = (k*ny + j)*nx + i to (i*ny + j)*nz + k.
 void launch_to_xyz(const float* in, int nx, int ny, int nz, float* out, cudaStream_t st);
-void launch_to_xyz(const uint8_t* in, int nx, int ny, int nz, uint8_t* out, cudaStream_t st);
 
 // occupancy.cu. cap: bucket entries that fit; with more, the buckets and what follows from
-// them are left out and stats->pairs tells the caller.
+// them are left out and stats->pairs tells the caller. otri: three float4 per triangle, the
+// column test's FP32 records; nullptr: every entry is decided in FP64. xyz: one mesh's whole
+// grid, its cells in [x][y][z] order.
 void launch_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts,
-                     const int* tris, double* soup, int4* xybox, int64_t* pairs, cudaStream_t st);
+                     const int* tris, double* soup, float4* otri, int4* xybox, int64_t* pairs,
+                     cudaStream_t st);
 void launch_col_pairs(bool fill, const MeshSeg* segs, int nseg, int64_t ntris, const int4* xybox,
                       const int64_t* pair_off, int* colcnt, const int64_t* col_off, int* col_list,
                       int64_t cap, Stats* stats, int grid, cudaStream_t st);
 void launch_occ_filter(int mode, const MeshSeg* segs, int nseg, int64_t nrows, const double* soup,
-                       const int64_t* col_off, const int* col_list, uint8_t* occ, int64_t* flagged,
-                       int64_t cap, Stats* stats, cudaStream_t st);
+                       const float4* otri, const int64_t* col_off, const int* col_list, uint8_t* occ,
+                       bool xyz, int64_t* flagged, int64_t cap, Stats* stats, cudaStream_t st);
 void launch_occ_exact(int mode, const MeshSeg* segs, int nseg, const double* soup,
                       const int64_t* col_off, const int* col_list, const int64_t* flagged,
-                      double* hs, uint8_t* hv, uint8_t* occ, Stats* stats, int grid,
+                      double* hs, uint8_t* hv, uint8_t* occ, bool xyz, Stats* stats, int grid,
                       cudaStream_t st);
 int occ_row_cols();
 

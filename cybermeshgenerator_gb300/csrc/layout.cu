@@ -1,5 +1,6 @@
 // layout.cu — grids from the cells' layout (z slowest, x fastest) to the reference
-// binding's array order (x slowest, z fastest: its transposed copy).
+// binding's array order (x slowest, z fastest: its transposed copy). Distances only: the
+// occupancy kernels write either order themselves.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -16,10 +17,9 @@ constexpr int kEdge = 32, kRows = 8;
 // One block per row j and 32 x 32 tile of its (k, i) plane, through shared memory, so that
 // both sides move whole 32-value rows. The device does in 0.03 ms what the host's copies took
 // 25 ms for (15M cells of 4 bytes: 120 MB of traffic).
-template <typename T>
-__global__ void __launch_bounds__(kEdge* kRows) k_to_xyz(const T* __restrict__ in, int nx, int ny, int nz,
-                                                         T* __restrict__ out) {
-    __shared__ T tile[kEdge][kEdge + 1];
+__global__ void __launch_bounds__(kEdge* kRows) k_to_xyz(const float* __restrict__ in, int nx, int ny, int nz,
+                                                         float* __restrict__ out) {
+    __shared__ float tile[kEdge][kEdge + 1];
     const unsigned ti = (nx + kEdge - 1) / kEdge, tk = (nz + kEdge - 1) / kEdge;
     const unsigned b = blockIdx.x;
     const int i0 = static_cast<int>(b % ti) * kEdge, k0 = static_cast<int>(b / ti % tk) * kEdge;
@@ -36,20 +36,12 @@ __global__ void __launch_bounds__(kEdge* kRows) k_to_xyz(const T* __restrict__ i
             out[(static_cast<int64_t>(i0 + r) * ny + j) * nz + k0 + lane] = tile[lane][r];
 }
 
-template <typename T>
-void to_xyz(const T* in, int nx, int ny, int nz, T* out, cudaStream_t st) {
-    const int64_t blocks = static_cast<int64_t>((nx + kEdge - 1) / kEdge) * ((nz + kEdge - 1) / kEdge) * ny;
-    k_to_xyz<T><<<static_cast<unsigned>(blocks), kEdge * kRows, 0, st>>>(in, nx, ny, nz, out);
-    CMG_LAUNCH();
-}
-
 }  // namespace
 
 void launch_to_xyz(const float* in, int nx, int ny, int nz, float* out, cudaStream_t st) {
-    to_xyz(in, nx, ny, nz, out, st);
-}
-void launch_to_xyz(const uint8_t* in, int nx, int ny, int nz, uint8_t* out, cudaStream_t st) {
-    to_xyz(in, nx, ny, nz, out, st);
+    const int64_t blocks = static_cast<int64_t>((nx + kEdge - 1) / kEdge) * ((nz + kEdge - 1) / kEdge) * ny;
+    k_to_xyz<<<static_cast<unsigned>(blocks), kEdge * kRows, 0, st>>>(in, nx, ny, nz, out);
+    CMG_LAUNCH();
 }
 
 }  // namespace cmg::gpu

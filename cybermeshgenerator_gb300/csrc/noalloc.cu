@@ -162,6 +162,7 @@ extern "C" cmg_status cmg_gpu_occupancy_static(const double* d_points, int64_t n
         s.g.nz = dims[2];
         s.g.z0 = 0;  // every layer
         s.g.z1 = dims[2];
+        s.f = occ_frame(s.g);
         s.tri_begin = 0;
         s.tri_end = T;
         CMG_CUDA(cudaMemcpyAsync(segs, &s, sizeof(s), cudaMemcpyHostToDevice, st));
@@ -179,7 +180,7 @@ extern "C" cmg_status cmg_gpu_occupancy_static(const double* d_points, int64_t n
             return CMG_ERR_INVALID_INPUT;
         }
 
-        launch_tri_prep(segs, 1, T, d_points, d_triangles, soup, xybox, pairs_n, st);
+        launch_tri_prep(segs, 1, T, d_points, d_triangles, soup, nullptr, xybox, pairs_n, st);
         exclusive_scan(pairs_n, pair_off, T, scan_tmp, st);
         int64_t P = 0;
         CMG_CUDA(cudaMemcpyAsync(&P, pair_off + T, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -197,10 +198,10 @@ extern "C" cmg_status cmg_gpu_occupancy_static(const double* d_points, int64_t n
         launch_col_pairs(false, segs, 1, T, xybox, pair_off, colcnt, nullptr, nullptr, P, stats, grid, st);
         exclusive_scan(colcnt, col_off, ncol, scan_tmp, st);
         launch_col_pairs(true, segs, 1, T, xybox, pair_off, colcnt, col_off, col_list, P, stats, grid, st);
-        launch_occ_filter(predicates, segs, 1, nrows, soup, col_off, col_list, d_occupancy, flagged,
-                          P, stats, st);
+        launch_occ_filter(predicates, segs, 1, nrows, soup, nullptr, col_off, col_list, d_occupancy,
+                          false, flagged, P, stats, st);
         launch_occ_exact(predicates, segs, 1, soup, col_off, col_list, flagged, hs, hv,
-                         d_occupancy, stats, 2 * device_sms(), st);
+                         d_occupancy, false, stats, 2 * device_sms(), st);
         CMG_CUDA(cudaStreamSynchronize(st));
         return CMG_OK;
     } catch (const std::exception& e) {
