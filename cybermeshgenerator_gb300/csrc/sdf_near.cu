@@ -11,7 +11,8 @@
 //      keeps (box_ball) go to a short list in shared memory;
 //   3. as soon as 32 of them wait, each lane loads one's record; those that the disc
 //      test keeps (box_disc) are staged in shared memory, and every cell tests them
-//      (cell_disc); a triangle that some cell needs is evaluated for all 64;
+//      (cell_disc); the (cell, triangle) pairs left are evaluated 32 at a time, one per
+//      lane (a triangle that some cell needs is needed by 8 to 18 of the 64);
 //   4. near-ties (FP32 distance within twice the stated error of the cell's minimum) are
 //      kept as (cell, triangle) pairs, and the FP64 distance in the reference's order is
 //      taken over the pairs, one per lane: for every cell (kPrecExact, the reference's
@@ -43,21 +44,22 @@ constexpr int kWarps = 4;       // independent warps per CTA
 constexpr int kStep = 4;        // list entries per lane and filter step (loads in flight)
 constexpr int kWait = 32 * (kStep + 1);  // entries that can wait for the disc test
 constexpr int kPairs = 256;     // near-tie pairs kept per sub-brick
+constexpr int kSkip = 512;      // of longer lists the probe reads every other step
 constexpr float kItemCost = 1024.f;  // a sub-brick's fixed work, in list entries
 constexpr float kHeavy = 0.25f;      // lists over this part of a warp's share are shared
 constexpr unsigned kAll = 0xffffffffu;
 
 struct WarpMem {
     // staged records, their centroids (radius widened: reach_term) and ids
-    union {
-        TriRec rec[32];
-        struct {  // a shared sub-brick: this warp's FP32 minima
-            float d[64];
-            int t[64];
-        } part;
-    };
+    TriRec rec[32];
     float4 c[32];
     int t[32];
+    // per cell: its FP32 minimum (bits of the squared distance, then the triangle), and the
+    // plane_reach of its bound (-1: not a cell of the grid)
+    unsigned long long best[64];
+    float reach[64];
+    float pos[12];  // cell offsets from the sub-brick centre, per axis
+    unsigned short ev[96];  // (cell, staged triangle) pairs that wait: cell | triangle << 6
     // FP64 results per cell: the smallest squared distance (bits) and, for it, the smallest
     // (triangle << 3) | region
     unsigned long long d[64], win[64];
@@ -176,13 +178,17 @@ __device__ __forceinline__ float plane_reach(float b, float ebr4) {
     return __fmaf_ru(__fadd_ru(b, ebr4), __fadd_ru(kRecNormalErr, 64.f * kU32), b);
 }
 
-// One cell of the lane.
-struct Cell {
-    float z;      // offset along z from the sub-brick centre (x and y are the lane's)
-    float best;   // smallest FP32 squared distance (-1: not a cell of the grid)
-    float reach;  // plane_reach of its bound
-    int t;        // the triangle of `best`
-};
+// A cell's FP32 minimum as one number: the smaller distance, the lower triangle on ties.
+__device__ __forceinline__ unsigned long long near_key(float d2, int t) {
+    return (static_cast<unsigned long long>(__float_as_uint(d2)) << 32) | static_cast<unsigned>(t);
+}
+__device__ __forceinline__ float key_dist(unsigned long long k) { return __uint_as_float(static_cast<unsigned>(k >> 32)); }
+__device__ __forceinline__ int key_tri(unsigned long long k) { return static_cast<int>(static_cast<unsigned>(k)); }
+
+// Lowers a nonnegative float (several lanes may).
+__device__ __forceinline__ void lower(float* at, float v) {
+    atomicMin(reinterpret_cast<unsigned*>(at), __float_as_uint(v));
+}
 
 // What the kernel reads and writes.
 struct Args {
@@ -218,8 +224,8 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
     const unsigned below = (1u << lane) - 1u;
     const int64_t gb = g.work[item >> 6];  // the bricks in order, 64 sub-bricks each
     const MeshSeg& s = g.segs[find_seg<&MeshSeg::brick_begin>(g.segs, g.nseg, gb)];
-    float px, py;
-    Cell A, B;
+    float px, py, zA, zB;  // the lane's two cells, lane and 32 + lane
+    bool okA, okB;         // are cells of the grid and the slab
     // ---- geometry: each lane forms one number per axis in FP64 (the FP64 pipe takes 16 cycles
     //      per warp instruction), the others get it by shuffles
     float hx, hy, hz;
@@ -237,13 +243,15 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         split2(ck, ch, cl);
         px = __shfl_sync(kAll, pv, lane & 3);
         py = __shfl_sync(kAll, pv, 4 + ((lane >> 2) & 3));
-        A.z = __shfl_sync(kAll, pv, 8 + (lane >> 4));
-        B.z = __shfl_sync(kAll, pv, 10 + (lane >> 4));
+        zA = __shfl_sync(kAll, pv, 8 + (lane >> 4));
+        zB = __shfl_sync(kAll, pv, 10 + (lane >> 4));
         hx = __shfl_sync(kAll, hw, 12);
         hy = __shfl_sync(kAll, hw, 13);
         hz = __shfl_sync(kAll, hw, 14);
-        if (lane < 12) M.ctr[lane] = cell_center(s.g.corner[a], lo + i, h);
-        else if (lane < 15) {
+        if (lane < 12) {
+            M.ctr[lane] = cell_center(s.g.corner[a], lo + i, h);
+            M.pos[lane] = pv;
+        } else if (lane < 15) {
             // the list's centroids are relative to the brick's centre, without their lo parts
             const int b0 = lo / s.brick * s.brick;
             const int n = a == 0 ? s.g.nx : (a == 1 ? s.g.ny : s.g.nz);
@@ -255,9 +263,8 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         }
         const int x = q.x0 + (lane & 3), y = q.y0 + ((lane >> 2) & 3), z = q.z0 + (lane >> 4);
         const bool col = x < q.x1 && y < q.y1;
-        // (-1: not a cell of the grid and the slab)
-        A.best = col && z < q.z1 && z >= s.g.z0 && z < s.g.z1 ? FLT_MAX : -1.f;
-        B.best = col && z + 2 < q.z1 && z + 2 >= s.g.z0 && z + 2 < s.g.z1 ? FLT_MAX : -1.f;
+        okA = col && z < q.z1 && z >= s.g.z0 && z < s.g.z1;
+        okB = col && z + 2 < q.z1 && z + 2 >= s.g.z0 && z + 2 < s.g.z1;
     }
     const float emax = s.emax_all;
     {
@@ -274,8 +281,11 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 fmaxf(0.f, __fmaf_ru(fabsf(bh), 512.f * kU32, bh + 16.f * kap + 1e-28f) * (1.f + 8.f * kU32));
             keep2 = far * far * (1.f + 8.f * kU32);
         }
-        M.thr2[lane] = A.best < 0.f ? -1.f : keep2;
-        M.thr2[32 + lane] = B.best < 0.f ? -1.f : keep2;
+        M.thr2[lane] = okA ? keep2 : -1.f;
+        M.thr2[32 + lane] = okB ? keep2 : -1.f;
+        M.reach[lane] = okA ? FLT_MAX : -1.f;
+        M.reach[32 + lane] = okB ? FLT_MAX : -1.f;
+        M.best[lane] = M.best[32 + lane] = near_key(FLT_MAX, INT_MAX);
         M.d[lane] = M.d[32 + lane] = static_cast<unsigned long long>(__double_as_longlong(DBL_MAX));
         M.win[lane] = M.win[32 + lane] = static_cast<unsigned long long>(INT_MAX) << 3;
         __syncwarp();  // the last sub-brick's reads of these are done
@@ -302,7 +312,8 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         float bestc = FLT_MAX, bestp = FLT_MAX;
         int kc = -1, kp = -1;
         const int np = min(nc, g.probe_n);
-        for (int k0 = first + lane; k0 < np; k0 += step) {
+        const int skip = np > kSkip ? 2 * step : step;
+        for (int k0 = first + lane; k0 < np; k0 += skip) {
             float4 e[kStep];
 #pragma unroll
             for (int i = 0; i < kStep; ++i)
@@ -349,34 +360,26 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
 
     // ---- the seed: every cell's first bound, and the box test around its nearest point to
     //      the centre (eps: four stated errors of the FP32 distances, and q's own)
-    A.t = B.t = INT_MAX;
-    A.reach = A.best;  // FLT_MAX, or -1: never reached
-    B.reach = B.best;
     int npair = 0, nfull = 0, neval = 0, nstaged = 0;  // nfull: pairs refined before the end
-    // appends the near-ties of one triangle (both cells of each lane); there is room
-    auto push = [&](int t, float dA, unsigned mA, float dB, unsigned mB) {
-        if ((mA >> lane) & 1u) {
-            const int k = npair + __popc(mA & below);
+    // appends near-ties of triangle t, one of each lane in m; there is room
+    auto push = [&](unsigned m, int t, float d, int cell) {
+        if ((m >> lane) & 1u) {
+            const int k = npair + __popc(m & below);
             M.pt[k] = t;
-            M.pd[k] = dA;
-            M.pc[k] = static_cast<unsigned char>(lane);
+            M.pd[k] = d;
+            M.pc[k] = static_cast<unsigned char>(cell);
         }
-        npair += __popc(mA);
-        if ((mB >> lane) & 1u) {
-            const int k = npair + __popc(mB & below);
-            M.pt[k] = t;
-            M.pd[k] = dB;
-            M.pc[k] = static_cast<unsigned char>(32 + lane);
-        }
-        npair += __popc(mB);
+        npair += __popc(m);
     };
-    auto improve = [&](Cell& c, int cell, float d, int t) {
-        if (d < c.best || (d == c.best && t < c.t)) {
+    // a cell's minimum, and what follows from it, after a triangle's distance
+    auto improve = [&](int cell, float d, int t) {
+        const unsigned long long key = near_key(d, t), was = M.best[cell];
+        if (key >= was) return;
+        atomicMin(&M.best[cell], key);
+        if (d < key_dist(was)) {
             const float4 con = M.con;
-            c.best = d;
-            c.t = t;
-            c.reach = plane_reach(cell_bound_x(d, con.y), con.z);
-            M.thr2[cell] = fminf(near_thr2(d, con.x), con.w);
+            lower(&M.reach[cell], plane_reach(cell_bound_x(d, con.y), con.z));
+            lower(&M.thr2[cell], near_thr2(d, con.x));
         }
     };
     if (seed != INT_MAX) {
@@ -390,12 +393,16 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
             box_test(qx, qy, qz, hx, hy, hz, M.mid[0].w,
                      __fmaf_ru(240.f * kU32, U + 4.f * M.mid[0].w, fmaf(40.f * kU32, con.z, 4.f * con.x)), M.off.w);
         if (lane == 0) M.box = b;
-        const float dA = dist_rec_val(r, px - e.x, py - e.y, A.z - e.z);
-        const float dB = dist_rec_val(r, px - e.x, py - e.y, B.z - e.z);
-        improve(A, lane, dA, seed);
-        improve(B, 32 + lane, dB, seed);
-        const unsigned nA = __ballot_sync(kAll, dA <= M.thr2[lane]), nB = __ballot_sync(kAll, dB <= M.thr2[32 + lane]);
-        if (!COOP || wid == 0) push(seed, dA, nA, dB, nB);
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            const int cell = lane + 32 * half;
+            const bool ok = half ? okB : okA;
+            const float d = dist_rec_val(r, px - e.x, py - e.y, (half ? zB : zA) - e.z);
+            if (ok) improve(cell, d, seed);
+            const unsigned m = __ballot_sync(kAll, ok && d <= M.thr2[cell]);
+            if (!COOP || wid == 0) push(m, seed, d, cell);
+        }
+        neval = 64;
     }
     __syncwarp();
 
@@ -451,62 +458,77 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         }
         __syncwarp();
         nstaged += staged;
-        for (int j = 0; j < staged; ++j) {
-            const float4 c = M.c[j];
-            const TriRec& R = M.rec[j];
-            const float dx = px - c.x, dy = py - c.y, zA = A.z - c.z, zB = B.z - c.z;
-            const PaN pA = pa_n(R, dx, dy, zA), pB = pa_n(R, dx, dy, zB);
-            const float xy = fmaf(dx, dx, dy * dy);
-            // a triangle no nearer than its disc, which lies beyond every cell's bound, is
-            // skipped; the plane's component is the distance's first step
-            if (!__any_sync(kAll, cell_disc(fmaf(zA, zA, xy), pA.n, A.reach, c.w) ||
-                                      cell_disc(fmaf(zB, zB, xy), pB.n, B.reach, c.w)))
-                continue;
-            const float dA = dist_rec_t<false>(R, pA, nullptr), dB = dist_rec_t<false>(R, pB, nullptr);
-            const int t = M.t[j];
-            ++neval;
-            improve(A, lane, dA, t);
-            improve(B, 32 + lane, dB, t);
-            const unsigned nA = __ballot_sync(kAll, dA <= M.thr2[lane]),
-                           nB = __ballot_sync(kAll, dB <= M.thr2[32 + lane]);
-            if (nA | nB) {
-                if (npair + __popc(nA) + __popc(nB) > kPairs) {
-                    npair = prune(M, npair);
-                    if (npair > kPairs - 64) {
-                        refine(M, npair, g.soup);
-                        nfull += npair;
-                        npair = 0;
+        int nev = 0;
+        for (int j = 0; j <= staged; ++j) {
+            if (j < staged) {
+                const float4 c = M.c[j];
+                const TriRec& R = M.rec[j];
+                const float dx = px - c.x, dy = py - c.y, dzA = zA - c.z, dzB = zB - c.z;
+                const float xy = fmaf(dx, dx, dy * dy);
+                // a triangle no nearer than its disc, which lies beyond the cell's bound, is
+                // skipped; the others are evaluated cell by cell
+                const bool a = cell_disc(fmaf(dzA, dzA, xy), pa_n(R, dx, dy, dzA).n, M.reach[lane], c.w);
+                const bool b = cell_disc(fmaf(dzB, dzB, xy), pa_n(R, dx, dy, dzB).n, M.reach[32 + lane], c.w);
+                const unsigned mA = __ballot_sync(kAll, a), mB = __ballot_sync(kAll, b);
+                if (!(mA | mB)) continue;
+                if (a) M.ev[nev + __popc(mA & below)] = static_cast<unsigned short>(lane | j << 6);
+                nev += __popc(mA);
+                if (b) M.ev[nev + __popc(mB & below)] = static_cast<unsigned short>(32 | lane | j << 6);
+                nev += __popc(mB);
+            }
+            while (nev >= 32 || (j == staged && nev > 0)) {
+                __syncwarp();
+                const int n = min(nev, 32);
+                nev -= n;
+                const bool in = lane < n;
+                const int pr = M.ev[nev + (in ? lane : 0)], cell = pr & 63, k = pr >> 6;
+                const float4 c = M.c[k];
+                const int t = M.t[k];
+                const float d = dist_rec_val(M.rec[k], M.pos[cell & 3] - c.x, M.pos[4 + ((cell >> 2) & 3)] - c.y,
+                                             M.pos[8 + (cell >> 4)] - c.z);
+                neval += n;
+                if (in) improve(cell, d, t);
+                __syncwarp();
+                const unsigned m = __ballot_sync(kAll, in && d <= M.thr2[cell]);
+                if (m) {
+                    if (npair + 32 > kPairs) {
+                        npair = prune(M, npair);
+                        if (npair + 32 > kPairs) {
+                            refine(M, npair, g.soup);
+                            nfull += npair;
+                            npair = 0;
+                        }
                     }
+                    push(m, t, d, cell);
                 }
-                push(t, dA, nA, dB, nB);
             }
         }
         __syncwarp();
     }
+    unsigned long long bestA = M.best[lane], bestB = M.best[32 + lane];
     if (COOP) {  // the minima over the warps' parts of the list
-        M.part.d[lane] = A.best;
-        M.part.t[lane] = A.t;
-        M.part.d[32 + lane] = B.best;
-        M.part.t[32 + lane] = B.t;
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < kWarps; ++k) {
-            improve(A, lane, all[k].part.d[lane], all[k].part.t[lane]);
-            improve(B, 32 + lane, all[k].part.d[32 + lane], all[k].part.t[32 + lane]);
+            bestA = min(bestA, all[k].best[lane]);
+            bestB = min(bestB, all[k].best[32 + lane]);
         }
+        const float4 con = M.con;
+        if (okA) M.thr2[lane] = fminf(near_thr2(key_dist(bestA), con.x), con.w);
+        if (okB) M.thr2[32 + lane] = fminf(near_thr2(key_dist(bestB), con.x), con.w);
         __syncwarp();
     }
 
     // ---- 4. FP64 distances of the near-ties: every cell's (exact), or the band cells'
-    const float d32A = sqrtf(A.best), d32B = sqrtf(B.best);
+    const float d32A = sqrtf(key_dist(bestA)), d32B = sqrtf(key_dist(bestB));
     // the mesh's largest triangle radius (not the brick's candidates', which depend on the
     // candidate walk): the bound, and the band it selects, are the same whatever slab of
     // the grid is evaluated
     const float er2 = 2.f * emax + 2.f * M.mid[0].w;
     const float bh = g.band_cells * static_cast<float>(s.g.h);
     const float ebA = 48.f * kU32 * (d32A + er2) + 1e-30f, ebB = 48.f * kU32 * (d32B + er2) + 1e-30f;
-    const bool fineA = A.best >= 0.f && (EXACT || d32A <= bh + ebA);
-    const bool fineB = B.best >= 0.f && (EXACT || d32B <= bh + ebB);
+    const bool fineA = okA && (EXACT || d32A <= bh + ebA);
+    const bool fineB = okB && (EXACT || d32B <= bh + ebB);
     const unsigned maskA = __ballot_sync(kAll, fineA), maskB = __ballot_sync(kAll, fineB);
     if (maskA | maskB) {
         if (!EXACT) {  // the near-ties of the band's cells only
@@ -525,8 +547,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
     }
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
-        const float best = half ? B.best : A.best;
-        if (best < 0.f || (COOP && half != wid)) continue;
+        if (!(half ? okB : okA) || (COOP && half != wid)) continue;
         const int x = M.org[0] + (lane & 3), y = M.org[1] + ((lane >> 2) & 3), z = M.org[2] + (lane >> 4) + 2 * half;
         const int64_t idx = s.vox_begin + (static_cast<int64_t>(z - s.g.z0) * s.g.ny + y) * s.g.nx + x;
         if (half ? fineB : fineA) {
@@ -542,7 +563,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                        static_cast<int>(win >> 3), static_cast<int>(win & 7u));
             if (g.o.errbound) g.o.errbound[idx] = 0.f;
         } else {
-            const int t = half ? B.t : A.t;
+            const int t = key_tri(half ? bestB : bestA);
             int reg = 0;
             if (g.o.near_reg && t != INT_MAX) {
                 // the region of the nearest triangle: its distance again, recentred exactly
@@ -550,7 +571,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const float4 e = recentre(g.tinfo[t], g.tinfo_lo[t], M.mid[0], M.mid[1]);
                 TriRec r;
                 load_rec(g.trec, t, r);
-                dist_rec(r, px - e.x, py - e.y, (half ? B.z : A.z) - e.z, &reg);
+                dist_rec(r, px - e.x, py - e.y, (half ? zB : zA) - e.z, &reg);
             }
             write_cell(g.o, idx, static_cast<double>(half ? d32B : d32A), t, reg);
             if (g.o.errbound) g.o.errbound[idx] = half ? ebB : ebA;
@@ -561,7 +582,12 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
 }
 
 // Registers are budgeted for 5 CTAs (20 warps) per SM: 96 a thread (231x247x256 surface,
-// exact / mixed: 7.0 / 4.5 ms; 4 CTAs at 128: 7.3 / 4.6, 6 at 80: 8.5 / 6.3, spills).
+// exact / mixed: 7.0 / 4.4 ms; 4 CTAs at 128: 7.2 / 4.6, 6 at 80: 8.2 / 6.1, spills).
+// Pairs one per lane instead of triangles for all 64 cells, and the probe's skipping (a seed
+// from half of a long list loosens the bound a little: 4 % more triangles are staged), for
+// 137^3 around 128k triangles, exact: 2.48 -> 2.21 -> 2.12 ms; 118x126x130 around 65k, mixed:
+// 1.40 -> 1.26 -> 1.24; 24 meshes, mixed: 11.2 -> 10.7 -> 10.5; the first grid: 1 to 2 %.
+// A quarter of the list lost 10 %.
 // grab_n: consecutive sub-bricks taken from the queue at once (they share one brick list).
 // probe_n: entries of the brick list the probe scans: all of it unless asked for less (the
 // 128^3 grid around 65k triangles: 1.4 ms; a head of 2048 leaves the sub-bricks with the
@@ -613,8 +639,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
             sub_brick<PREC, false>(g, item + k, M, S, all);
     }
     if (lane == 0) {
-        // a triangle evaluated for a sub-brick counts its 64 cells
-        if (M.evals) atomicAdd(&st->evaluations, 64 * M.evals);
+        if (M.evals) atomicAdd(&st->evaluations, M.evals);
         if (M.filtered) atomicAdd(&st->filtered, M.filtered);
         if (M.evals64) atomicAdd(&st->fp64_evaluations, M.evals64);
         if (M.bandc) atomicAdd(&st->band_voxels, M.bandc);
