@@ -106,33 +106,60 @@ __device__ __noinline__ int prune(WarpMem& M, int n) {
     return kept;
 }
 
-// The FP64 distances of the n pairs, one per lane, into the cells' results: the smallest,
-// by the lowest triangle on ties. A pair that later turns out to lie beyond its cell's
-// final threshold changes nothing: the minimum over more triangles is the same.
+// What a CTA's warps exchange about a shared sub-brick.
+struct Shared {
+    unsigned long long grab;
+    unsigned u[kWarps];
+    int seed[kWarps];
+    int npair[kWarps];
+};
+
+// The FP64 distance of one pair per lane (in: there is one) into the cells' results.
+__device__ __forceinline__ void refine_32(WarpMem& M, const double* __restrict__ soup, int t, int c, bool in) {
+    d3 a, b, cc;
+    load_soup(soup, t, a, b, cc);
+    int reg;
+    const double e2 = ericson_sel(d3{M.ctr[c & 3], M.ctr[4 + ((c >> 2) & 3)], M.ctr[8 + (c >> 4)]}, a, b, cc, &reg);
+    // (a NaN or infinite distance counts for nothing)
+    const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(e2));
+    const bool use = in && e2 <= DBL_MAX;
+    const unsigned long long was = M.d[c];
+    __syncwarp();
+    if (use && bits < was) atomicMin(&M.d[c], bits);
+    __syncwarp();
+    const unsigned long long now = M.d[c];
+    if (now != was) M.win[c] = ~0ull;
+    __syncwarp();
+    if (use && bits == now) atomicMin(&M.win[c], (static_cast<unsigned long long>(t) << 3) | static_cast<unsigned>(reg));
+    __syncwarp();
+}
+
+// The FP64 distances of the n pairs, one per lane: the smallest, by the lowest triangle on
+// ties. A pair that later turns out to lie beyond its cell's final threshold changes
+// nothing: the minimum over more triangles is the same.
 __device__ __noinline__ void refine(WarpMem& M, int n, const double* __restrict__ soup) {
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
     for (int k0 = 0; k0 < n; k0 += 32) {
         const bool in = k0 + lane < n;
         const int k = in ? k0 + lane : n - 1;
-        const int t = M.pt[k], c = M.pc[k];
-        d3 a, b, cc;
-        load_soup(soup, t, a, b, cc);
-        int reg;
-        const double e2 = ericson_sel(d3{M.ctr[c & 3], M.ctr[4 + ((c >> 2) & 3)], M.ctr[8 + (c >> 4)]}, a, b, cc, &reg);
-        // (a NaN or infinite distance counts for nothing)
-        const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(e2));
-        const bool use = in && e2 <= DBL_MAX;
-        const unsigned long long was = M.d[c];
-        __syncwarp();
-        if (use && bits < was) atomicMin(&M.d[c], bits);
-        __syncwarp();
-        const unsigned long long now = M.d[c];
-        if (now != was) M.win[c] = ~0ull;
-        __syncwarp();
-        if (use && bits == now)
-            atomicMin(&M.win[c], (static_cast<unsigned long long>(t) << 3) | static_cast<unsigned>(reg));
-        __syncwarp();
+        refine_32(M, soup, M.pt[k], M.pc[k], in);
+    }
+}
+
+// The same for the pairs of all the CTA's warps (S.npair each): of every 128 in a row, this
+// warp's 32.
+__device__ __noinline__ void refine_shared(WarpMem& M, const WarpMem* all, const Shared& S,
+                                           const double* __restrict__ soup) {
+    const int lane = threadIdx.x & 31;
+    int n = 0;
+    for (int w = 0; w < kWarps; ++w) n += S.npair[w];
+#pragma unroll 1
+    for (int k0 = threadIdx.x & ~31; k0 < n; k0 += 32 * kWarps) {
+        const bool in = k0 + lane < n;
+        int k = in ? k0 + lane : n - 1, w = 0;
+        while (k >= S.npair[w]) k -= S.npair[w++];
+        refine_32(M, soup, all[w].pt[k], all[w].pc[k], in);
     }
 }
 
@@ -205,13 +232,6 @@ struct Args {
     const float4* cand_c;
     float band_cells;
     Out o;
-};
-
-// What a CTA's warps exchange about a shared sub-brick.
-struct Shared {
-    unsigned long long grab;
-    unsigned u[kWarps];
-    int seed[kWarps];
 };
 
 // One sub-brick: by this warp alone, or (COOP) by the CTA's warps together, each over its
@@ -300,7 +320,10 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
     const int nc = static_cast<int>(g.cand_rng[2 * gb + 1] - c0);
     const int* __restrict__ list = g.cand + c0;
     const float4* __restrict__ listc = g.cand_c + c0;
-    const int first = COOP ? wid * 32 * kStep : 0, step = COOP ? kWarps * 32 * kStep : 32 * kStep;
+    // (the warps of a shared sub-brick take every fourth 32 entries)
+    constexpr int kNext = COOP ? 32 * kWarps : 32;
+    const int first = COOP ? wid * 32 : 0;
+    constexpr int step = kNext * kStep;
 
     // ---- 1. probe: per lane, over the list's head, the triangle of the nearest centroid
     //         and the one of the smallest power distance |c|^2 - w^2 (w the radius: large
@@ -317,13 +340,13 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
             float4 e[kStep];
 #pragma unroll
             for (int i = 0; i < kStep; ++i)
-                e[i] = k0 + 32 * i < np ? __ldg(listc + k0 + 32 * i) : make_float4(FLT_MAX, 0.f, 0.f, 0.f);
+                e[i] = k0 + kNext * i < np ? __ldg(listc + k0 + kNext * i) : make_float4(FLT_MAX, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int i = 0; i < kStep; ++i) {
                 const float ex = e[i].x - off.x, ey = e[i].y - off.y, ez = e[i].z - off.z;
                 const float c2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez)), pw = fmaf(-e[i].w, e[i].w, c2);
-                if (c2 < bestc) { bestc = c2; kc = k0 + 32 * i; }
-                if (pw < bestp) { bestp = pw; kp = k0 + 32 * i; }
+                if (c2 < bestc) { bestc = c2; kc = k0 + kNext * i; }
+                if (pw < bestp) { bestp = pw; kp = k0 + kNext * i; }
             }
         }
 #pragma unroll 1
@@ -415,7 +438,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
             float4 e[kStep];
 #pragma unroll
             for (int i = 0; i < kStep; ++i)
-                e[i] = cur + lane + 32 * i < nc ? __ldg(listc + cur + lane + 32 * i)
+                e[i] = cur + lane + kNext * i < nc ? __ldg(listc + cur + lane + kNext * i)
                                                 : make_float4(CUDART_NAN_F, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int i = 0; i < kStep; ++i) {
@@ -424,7 +447,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const bool take = seed != INT_MAX ? ex == ex && box_ball(box, ex, ey, ez, e[i].w, off.w)
                                                   : ex * ex + ey * ey + ez * ez <= FLT_MAX;
                 const unsigned m = __ballot_sync(kAll, take);
-                if (take) M.wait[nwait + __popc(m & below)] = cur + lane + 32 * i;
+                if (take) M.wait[nwait + __popc(m & below)] = cur + lane + kNext * i;
                 nwait += __popc(m);
             }
             cur += step;
@@ -536,7 +559,13 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
             if (!fineB) M.thr2[32 + lane] = -1.f;
         }
         npair = prune(M, npair);
-        if (npair > 0) refine(M, npair, g.soup);
+        if (COOP) {
+            if (lane == 0) S.npair[wid] = npair;
+            __syncthreads();
+            refine_shared(M, all, S, g.soup);
+        } else if (npair > 0) {
+            refine(M, npair, g.soup);
+        }
     }
     const bool full = COOP ? __syncthreads_or(nfull) != 0 : nfull != 0;
     if (lane == 0) {
@@ -597,7 +626,10 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
 // parts are the minimum over the list); the lists get shorter (to within an eighth), so the
 // first light one ends the sharing. With few sub-bricks in all, every one is shared. (128^3 grid around 65k
 // triangles: 3.1 -> 1.4 ms, the warp with the longest list had ended last; 63^3 around 1280
-// triangles, all shared: 0.28 -> 0.19 ms.)
+// triangles, all shared: 0.28 -> 0.19 ms.) Their lists are dealt out by 32 entries, and the
+// pairs for FP64 by 32 pairs, whichever warp found them: with parts of 128 entries and
+// everybody's own pairs, half of a shared sub-brick's time was waiting for the last warp (63^3:
+// 0.19 -> 0.17 ms, 35^3 around 320 triangles: 0.11 -> 0.075 ms).
 template <int PREC>
 __global__ void __launch_bounds__(32 * kWarps, 5)
 k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restrict__ st) {
