@@ -592,6 +592,11 @@ void Batch::run_impl(bool sizing) {
     if (timed) CMG_CUDA(cudaEventRecord(ev_[0], st));
 
     CMG_CUDA(cudaMemsetAsync(stats_, 0, static_cast<size_t>(I.zero_end - reinterpret_cast<char*>(stats_)), st));
+    if (sdf) {
+        CMG_CUDA(cudaEventRecord(fork_, st));
+        CMG_CUDA(cudaStreamWaitEvent(side_, fork_, 0));
+        side_open_ = true;
+    }
     launch_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.soup, I.otri, I.xybox,
                     I.pairs_n, st);
 
@@ -634,13 +639,14 @@ void Batch::run_impl(bool sizing) {
     }
 
     // SDF preparation: triangle bins, brick walk (candidate lists), work order. It reads
-    // the soup, never the occupancy, so it runs on the second stream beside the
-    // occupancy passes. The candidate count sizes the candidate arena in a sizing run.
+    // the points and (the walk) the soup, never the occupancy, so it runs on the second
+    // stream beside the occupancy passes. The candidate count sizes the candidate arena in a sizing run.
     cudaStream_t ss = side_;
     int64_t* tmp = I.scan_tmp_side;
     auto prep_head = [&]() {
         if (timed) CMG_CUDA(cudaEventRecord(ev_[4], ss));
-        launch_sdf_tri_prep(dsegs_, nseg, ntris_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.tnorm, I.tlo,
+        launch_sdf_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.tinfo, I.tinfo_lo, I.trec,
+                            opts_.brick == 16 && sub_precision(opts_) == kPrecFP64 ? I.tnorm : nullptr, I.tlo,
                             I.thi, I.tbin, I.bincnt, I.large_cnt, I.emax_bits, ss);
         exclusive_scan(I.bincnt, I.bin_off, nbrick_, tmp, ss);
         launch_seg_finish(dsegs_, nseg, I.large_cnt, I.emax_bits, ss);
@@ -679,9 +685,8 @@ void Batch::run_impl(bool sizing) {
     // The longer preparation is issued first. In a sizing run each arena is re-planned
     // while the other stream's passes, which do not touch it, keep the device busy.
     CMG_CUDA(cudaEventRecord(fork_, st));
-    CMG_CUDA(cudaStreamWaitEvent(ss, fork_, 0));
-    side_open_ = true;
     prep_head();
+    CMG_CUDA(cudaStreamWaitEvent(ss, fork_, 0));
     walk();
     occ_head(st);
     if (!sizing) prep_tail();

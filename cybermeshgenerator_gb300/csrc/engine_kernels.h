@@ -41,7 +41,7 @@ int occ_row_cols();
 // trec: one kTriRecBytes-byte translation-invariant FP32 record per triangle (sdf::TriRec,
 // the triangle in its own frame).
 constexpr size_t kTriRecBytes = 96;
-void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* soup,
+void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts, const int* tris,
                          float4* tinfo, float4* tinfo_lo, void* trec, float4* tnorm, float4* tlo,
                          float4* thi,
                          int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits,

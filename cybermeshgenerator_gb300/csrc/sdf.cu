@@ -48,9 +48,15 @@ __device__ __forceinline__ float round_up_f(double x) { return __double2float_ru
 
 // ------------------------------------------------------------------ triangle prep
 // tinfo (float4 per triangle): centroid relative to the mesh grid corner (FP32,
-// nearest) and the radius e_t rounded up (plus the rounding of the centroid).
+// nearest) and the radius e_t rounded up (plus the rounding of the centroid). tnorm, for the
+// plain FP64 evaluation, may be null; tlo and thi are written for large triangles, the only
+// ones whose boxes are read.
+// 128k triangles: 320 us with one atomic per triangle on its mesh's largest radius (twice),
+// coordinate scale and bin; 118 us with one per warp, bound by some 300 FP64 instructions a
+// triangle on the narrow pipe (24 meshes: 677 -> 288 us, k_bin_fill 109 -> 12).
 __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64_t ntris,
-                               const double* __restrict__ soup, float4* __restrict__ tinfo,
+                               const double* __restrict__ pts, const int* __restrict__ tris,
+                               float4* __restrict__ tinfo,
                                float4* __restrict__ tinfo_lo, TriRec* __restrict__ trec,
                                float4* __restrict__ tnorm,
                                float4* __restrict__ tlo, float4* __restrict__ thi,
@@ -61,19 +67,22 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
     const int si = find_seg<&MeshSeg::tri_begin>(segs, nseg, t);
     const MeshSeg& s = segs[si];
     d3 a, b, c;
-    load_soup(soup, t, a, b, c);
+    {
+        const double* pa = pts + 3 * static_cast<int64_t>(tris[3 * t]);
+        const double* pb = pts + 3 * static_cast<int64_t>(tris[3 * t + 1]);
+        const double* pc = pts + 3 * static_cast<int64_t>(tris[3 * t + 2]);
+        a = {pa[0], pa[1], pa[2]};
+        b = {pb[0], pb[1], pb[2]};
+        c = {pc[0], pc[1], pc[2]};
+    }
     const double* K = s.g.corner;
     // centroid in FP64 (any rounding is covered by the radius padding below)
     double cx = (a.x + b.x + c.x) / 3.0, cy = (a.y + b.y + c.y) / 3.0, cz = (a.z + b.z + c.z) / 3.0;
     double r2 = 0.0;
     const d3 V[3] = {a, b, c};
-    double lo[3] = {a.x, a.y, a.z}, hi[3] = {a.x, a.y, a.z};
     for (int k = 0; k < 3; ++k) {
         double dx = V[k].x - cx, dy = V[k].y - cy, dz = V[k].z - cz;
         r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
-        lo[0] = fmin(lo[0], V[k].x); hi[0] = fmax(hi[0], V[k].x);
-        lo[1] = fmin(lo[1], V[k].y); hi[1] = fmax(hi[1], V[k].y);
-        lo[2] = fmin(lo[2], V[k].z); hi[2] = fmax(hi[2], V[k].z);
     }
     float4 ci, cl;
     split2(cx - K[0], ci.x, cl.x);
@@ -85,28 +94,25 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
     double pad = 2.0 * kU32 * (fabs(cx - K[0]) + fabs(cy - K[1]) + fabs(cz - K[2])) + 1e-300;
     ci.w = round_up_f(sqrt(r2) * (1.0 + 1e-12) + pad);
     tinfo[t] = ci;
-    tlo[t] = make_float4(__double2float_rd(lo[0] - K[0]), __double2float_rd(lo[1] - K[1]),
-                         __double2float_rd(lo[2] - K[2]), 0.f);
-    thi[t] = make_float4(__double2float_ru(hi[0] - K[0]), __double2float_ru(hi[1] - K[1]),
-                         __double2float_ru(hi[2] - K[2]), 0.f);
     // translation-invariant FP32 record (from FP64)
     double ux = b.x - a.x, uy = b.y - a.y, uz = b.z - a.z;
     double vx = c.x - a.x, vy = c.y - a.y, vz = c.z - a.z;
     double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
     bool degenerate = !(nx * nx + ny * ny + nz * nz > 0.0);
     {
-        double nl = sqrt(nx * nx + ny * ny + nz * nz);
-        double n3[3] = {0.0, 0.0, 0.0};
-        if (nl > 0.0) { n3[0] = nx / nl; n3[1] = ny / nl; n3[2] = nz / nl; }
-        // the FP64 path's plane bound: the unit normal in FP32 and a bound on its distance
-        // from the exact one: the cross product of rounded edges errs by at most
-        // 21 u |u| |v| (as a vector), which turns its direction by at most twice that
-        // over |u x v|; then the normalisation and the FP32 rounding of the components
         const double lu = sqrt(ux * ux + uy * uy + uz * uz), lv = sqrt(vx * vx + vy * vy + vz * vz);
-        const double en = nl > 0.0 ? 50.0 * kU64 * lu * lv / nl + 1.2e-7 : 0.0;
-        if (tnorm)
+        if (tnorm) {
+            double nl = sqrt(nx * nx + ny * ny + nz * nz);
+            double n3[3] = {0.0, 0.0, 0.0};
+            if (nl > 0.0) { n3[0] = nx / nl; n3[1] = ny / nl; n3[2] = nz / nl; }
+            // the FP64 path's plane bound: the unit normal in FP32 and a bound on its distance
+            // from the exact one: the cross product of rounded edges errs by at most
+            // 21 u |u| |v| (as a vector), which turns its direction by at most twice that
+            // over |u x v|; then the normalisation and the FP32 rounding of the components
+            const double en = nl > 0.0 ? 50.0 * kU64 * lu * lv / nl + 1.2e-7 : 0.0;
             tnorm[t] = make_float4(static_cast<float>(n3[0]), static_cast<float>(n3[1]),
                                    static_cast<float>(n3[2]), round_up_f(en));
+        }
         // the mixed path's record in the triangle's frame: u along b - a (else along
         // c - a, else x), v from c - a by two Gram-Schmidt passes (so c = a + cx u +
         // cy v to FP64 rounding however thin the triangle), n = u x v
@@ -160,40 +166,68 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
         r.pad_[0] = r.pad_[1] = r.pad_[2] = 0.f;
         trec[t] = r;
     }
-    // the mesh's coordinate scale max |v - K| (rounded up), per segment, for the
-    // FP32 tolerances; k_seg_finish folds in the grid extent
-    {
-        double m = 0.0;
-        for (int k = 0; k < 3; ++k)
-            m = fmax(m, fmax(fabs(V[k].x - K[0]), fmax(fabs(V[k].y - K[1]), fabs(V[k].z - K[2]))));
-        const unsigned bits = __float_as_uint(round_up_f(m));
-        const unsigned grp = __match_any_sync(__activemask(), si);
-        const unsigned mx = __reduce_max_sync(grp, bits);
-        if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicMax(&emax_bits[nseg + si], mx);
-    }
-    // the largest radius of all the mesh's triangles (the mixed path's error bounds)
-    atomicMax(&emax_bits[2 * nseg + si], __float_as_uint(ci.w));
     // degenerate (zero-area) or larger than two bricks: always considered
     const double bw = static_cast<double>(s.brick) * s.g.h;
-    bool large = degenerate || sqrt(r2) > 2.0 * bw;
+    const bool large = degenerate || sqrt(r2) > 2.0 * bw;
+    // per segment, one set of atomics per warp: the mesh's coordinate scale max |v - K|
+    // (rounded up) for the FP32 tolerances (k_seg_finish folds in the grid extent), the
+    // largest radius of all its triangles (the mixed path's error bounds) and of the binned
+    // ones, and the large ones' count
+    {
+        // (the largest by the bits, off the FP64 pipe; NaNs do not count)
+        unsigned long long m = 0ull;
+        auto most = [&](double v) {
+            const unsigned long long w = static_cast<unsigned long long>(__double_as_longlong(fabs(v)));
+            if (w > m && w <= 0x7ff0000000000000ull) m = w;
+        };
+        for (int k = 0; k < 3; ++k) {
+            most(V[k].x - K[0]);
+            most(V[k].y - K[1]);
+            most(V[k].z - K[2]);
+        }
+        const unsigned bits = __float_as_uint(round_up_f(__longlong_as_double(static_cast<long long>(m))));
+        const unsigned grp = __match_any_sync(__activemask(), si);
+        const unsigned scale = __reduce_max_sync(grp, bits), w = __float_as_uint(ci.w);
+        const unsigned all = __reduce_max_sync(grp, w), binned = __reduce_max_sync(grp, large ? 0u : w);
+        const unsigned n = __reduce_add_sync(grp, large ? 1u : 0u);
+        if ((threadIdx.x & 31) == __ffs(grp) - 1) {
+            atomicMax(&emax_bits[nseg + si], scale);
+            atomicMax(&emax_bits[2 * nseg + si], all);
+            if (binned) atomicMax(&emax_bits[si], binned);
+            if (n) atomicAdd(&large_cnt[si], static_cast<int>(n));
+        }
+    }
     if (large) {
+        tlo[t] = make_float4(__double2float_rd(fmin(a.x, fmin(b.x, c.x)) - K[0]),
+                             __double2float_rd(fmin(a.y, fmin(b.y, c.y)) - K[1]),
+                             __double2float_rd(fmin(a.z, fmin(b.z, c.z)) - K[2]), 0.f);
+        thi[t] = make_float4(__double2float_ru(fmax(a.x, fmax(b.x, c.x)) - K[0]),
+                             __double2float_ru(fmax(a.y, fmax(b.y, c.y)) - K[1]),
+                             __double2float_ru(fmax(a.z, fmax(b.z, c.z)) - K[2]), 0.f);
         tbin[t] = -1;
-        atomicAdd(&large_cnt[si], 1);
         return;
     }
-    atomicMax(&emax_bits[si], __float_as_uint(ci.w));
     // the bin of the centroid among the mesh's bricks (along z those of its slab, from
     // brick layer bzo), clamped: a clamped triangle lies outside the bins' box, and no
     // point inside the box is nearer its clamped position than its own
-    int bx = static_cast<int>(floor((cx - K[0]) / bw));
-    int by = static_cast<int>(floor((cy - K[1]) / bw));
-    int bz = static_cast<int>(floor((cz - K[2]) / bw)) - s.bzo;
+    // (an FP32 product decides where it is clear of the whole numbers by more than its error)
+    const float inv = 1.f / static_cast<float>(bw);
+    auto bin_of = [&](float d32, double d) {
+        const float v = d32 * inv, f = floorf(v), rest = v - f, m = 4e-7f * fabsf(v);
+        if (rest > m && 1.f - rest > m && fabsf(v) < 1e6f) return static_cast<int>(f);
+        return static_cast<int>(floor(d / bw));
+    };
+    int bx = bin_of(ci.x, cx - K[0]);
+    int by = bin_of(ci.y, cy - K[1]);
+    int bz = bin_of(ci.z, cz - K[2]) - s.bzo;
     bx = min(max(bx, 0), s.bnx - 1);
     by = min(max(by, 0), s.bny - 1);
     bz = min(max(bz, 0), s.bnz - 1);
     int64_t bin = s.brick_begin + (static_cast<int64_t>(bz) * s.bny + by) * s.bnx + bx;
     tbin[t] = bin;
-    atomicAdd(&bincnt[bin], 1);
+    // (neighbouring triangles share bins: one atomic per bin and warp, here and in k_bin_fill)
+    const unsigned grp = __match_any_sync(__activemask(), bin);
+    if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&bincnt[bin], __popc(grp));
 }
 
 // Bin -> triangle CSR. bin_info: the triangles' tinfo in the list's order, so that the walks
@@ -205,9 +239,15 @@ __global__ void k_bin_fill(int64_t ntris, const int64_t* __restrict__ tbin,
                            int* __restrict__ large_cur, int* __restrict__ large_list) {
     int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= ntris) return;
+    const int lane = threadIdx.x & 31;
     int64_t b = tbin[t];
     if (b >= 0) {
-        const int64_t at = bin_off[b] + atomicSub(&bincur[b], 1) - 1;  // the counts, taken down to zero
+        const unsigned grp = __match_any_sync(__activemask(), b);
+        const int lead = __ffs(grp) - 1, n = __popc(grp);
+        int left = 0;
+        if (lane == lead) left = atomicSub(&bincur[b], n);  // the counts, taken down to zero
+        left = __shfl_sync(grp, left, lead);
+        const int64_t at = bin_off[b] + left - n + __popc(grp & ((1u << lane) - 1u));
         bin_list[at] = static_cast<int>(t);
         bin_info[at] = tinfo[t];
     } else {
@@ -232,20 +272,31 @@ __global__ void k_bin_balls(int64_t nbins, const int64_t* __restrict__ bin_off,
         return;
     }
     float lx = FLT_MAX, ly = FLT_MAX, lz = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX, hz = -FLT_MAX;
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-        const float4 t = bin_info[e];
-        lx = fminf(lx, t.x); ly = fminf(ly, t.y); lz = fminf(lz, t.z);
-        hx = fmaxf(hx, t.x); hy = fmaxf(hy, t.y); hz = fmaxf(hz, t.z);
+    // (the last entry again beyond the end: four loads in flight in long bins)
+    for (int64_t e = e0 + lane; e - lane < e1; e += 128) {
+        float4 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t[j] = bin_info[min(e + 32 * j, e1 - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            lx = fminf(lx, t[j].x); ly = fminf(ly, t[j].y); lz = fminf(lz, t[j].z);
+            hx = fmaxf(hx, t[j].x); hy = fmaxf(hy, t[j].y); hz = fmaxf(hz, t[j].z);
+        }
     }
     const float cx = 0.5f * (warp_min(lx) - warp_min(-hx)), cy = 0.5f * (warp_min(ly) - warp_min(-hy)),
                 cz = 0.5f * (warp_min(lz) - warp_min(-hz));
     float rc = 0.f, rt = 0.f;
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-        const float4 t = bin_info[e];
-        const float dx = t.x - cx, dy = t.y - cy, dz = t.z - cz;
-        const float d = sqrtf(dx * dx + dy * dy + dz * dz);
-        rc = fmaxf(rc, d);
-        rt = fmaxf(rt, d + t.w);
+    for (int64_t e = e0 + lane; e - lane < e1; e += 128) {
+        float4 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t[j] = bin_info[min(e + 32 * j, e1 - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float dx = t[j].x - cx, dy = t[j].y - cy, dz = t[j].z - cz;
+            const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+            rc = fmaxf(rc, d);
+            rt = fmaxf(rt, d + t[j].w);
+        }
     }
     rc = -warp_min(-rc);
     rt = -warp_min(-rt);
@@ -1136,14 +1187,14 @@ k_count_K(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* soup,
+void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts, const int* tris,
                          float4* tinfo, float4* tinfo_lo, void* trec, float4* tnorm, float4* tlo,
                          float4* thi,
                          int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits,
                          cudaStream_t st) {
     if (ntris == 0) return;
     k_sdf_tri_prep<<<static_cast<unsigned>((ntris + 255) / 256), 256, 0, st>>>(
-        segs, nseg, ntris, soup, tinfo, tinfo_lo, static_cast<TriRec*>(trec), tnorm, tlo, thi, tbin,
+        segs, nseg, ntris, pts, tris, tinfo, tinfo_lo, static_cast<TriRec*>(trec), tnorm, tlo, thi, tbin,
         bincnt, large_cnt, emax_bits);
     CMG_LAUNCH();
 }
