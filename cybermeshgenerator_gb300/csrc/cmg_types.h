@@ -62,7 +62,8 @@ struct MeshSeg {
     int bzo;                        // brick layer of the mesh's first brick (the slab's)
     int brick;                      // brick edge in cells
     int walk_warps;                 // warps per brick of the candidate walk
-    int64_t walk_begin;             // the walk's CTAs
+    int64_t walk_begin;             // the walk's CTAs of the mesh that is this many-th in its order,
+    int64_t walk_seg;               // which is this one (the meshes with the longest lists first)
     int64_t large_begin, large_end; // always-considered triangles (global list)
     float emax;                     // max centroid-to-vertex distance of binned triangles
     float emax_all;                 // the same over all the mesh's triangles

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <new>
 #include <tuple>
 
@@ -316,11 +317,20 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     const bool sdf = opts_.want_sdf32 || opts_.want_sdf64 || opts_.want_near;
     if (opts_.xyz && (segs_.size() != 1 || slab || (opts_.want_occ && sdf)))
         throw std::invalid_argument("voxelize: [x][y][z] order is for one mesh's whole grid and one output");
-    for (MeshSeg& s : segs_) {
-        const int64_t n = static_cast<int64_t>(s.bnx) * s.bny * s.bnz;
-        s.walk_warps = brick_walk_warps(nbrick_, n, s.tri_end - s.tri_begin, opts_.walk_warps);
-        s.walk_begin = nwalk_;
-        nwalk_ += brick_walk_ctas(n, s.walk_warps);
+    // the candidate walk takes the meshes in the order of triangles per brick
+    std::vector<int> turn(segs_.size());
+    std::iota(turn.begin(), turn.end(), 0);
+    const auto bricks = [](const MeshSeg& s) { return static_cast<int64_t>(s.bnx) * s.bny * s.bnz; };
+    const auto density = [&](int i) {
+        return static_cast<double>(segs_[i].tri_end - segs_[i].tri_begin) / static_cast<double>(bricks(segs_[i]));
+    };
+    std::stable_sort(turn.begin(), turn.end(), [&](int a, int b) { return density(a) > density(b); });
+    for (int i = 0; i < nseg; ++i) {
+        MeshSeg& s = segs_[turn[i]];
+        s.walk_warps = brick_walk_warps(nbrick_, bricks(s), s.tri_end - s.tri_begin, opts_.walk_warps);
+        segs_[i].walk_begin = nwalk_;
+        segs_[i].walk_seg = turn[i];
+        nwalk_ += brick_walk_ctas(bricks(s), s.walk_warps);
     }
 
     // ---- fixed workspace

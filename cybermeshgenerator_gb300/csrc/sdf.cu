@@ -510,6 +510,18 @@ __device__ __forceinline__ void for_group_entries(int64_t b0, int64_t b1, int la
 // kernel that gathered every entry of every shell's bins -> 0.56 ms.)
 constexpr int kWalkThreads = 256;
 
+// Brick number k of the mesh when they are taken from the middle of the grid outward, layer
+// by layer and row by row: the lists of the bricks deep inside a closed surface are the
+// longest, and a long one taken last would be waited for (231x247x256: 0.61 -> 0.52 ms; 24
+// meshes, which are taken by triangles per brick besides: 2.20 -> 2.00 ms).
+__device__ __forceinline__ int64_t centre_first(const MeshSeg& s, int64_t k) {
+    auto outward = [](int i, int n) { return n / 2 + ((i & 1) ? -((i + 1) / 2) : i / 2); };
+    const int x = static_cast<int>(k % s.bnx), y = static_cast<int>(k / s.bnx % s.bny),
+              z = static_cast<int>(k / (static_cast<int64_t>(s.bnx) * s.bny));
+    return (static_cast<int64_t>(outward(z, s.bnz)) * s.bny + outward(y, s.bny)) * s.bnx + outward(x, s.bnx);
+}
+
+
 __global__ void __launch_bounds__(kWalkThreads, 3)
 k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
              const double* __restrict__ soup, const float4* __restrict__ tinfo,
@@ -525,12 +537,14 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
     __shared__ int s_c[kWarps];
     __shared__ long long s_off[kWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const MeshSeg& s = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
+    const MeshSeg& turn = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
+    const MeshSeg& s = segs[turn.walk_seg];
     const int W = s.walk_warps;
     const int slot = wid / W, sub = wid % W;  // brick within the CTA, warp within the brick
     const int first = slot * W;               // the brick's first warp
-    const int64_t lb = (blockIdx.x - s.walk_begin) * (kWarps / W) + slot;
+    int64_t lb = (blockIdx.x - turn.walk_begin) * (kWarps / W) + slot;
     if (lb >= static_cast<int64_t>(s.bnx) * s.bny * s.bnz) return;  // uniform over the brick's warps
+    lb = centre_first(s, lb);
     const int64_t gb = s.brick_begin + lb;
     auto brick_sync = [&]() {
         if (W == 1) __syncwarp();
