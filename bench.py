@@ -69,7 +69,7 @@ def workload():
     return W.sh_sphere(nlon=256, nlat=128, seed=3)
 
 
-def kernel_source_sha(files=("sdf_sub.cu", "cmg_sdf.cuh")):
+def kernel_source_sha(files=("sdf_near.cu", "cmg_sdf.cuh")):
     """SHA-256 (16 hex digits) of the evaluation kernel's code (the sources with their
     // comments and blank lines taken out), recorded in its ncu summary so that the bench
     line takes DRAM traffic only from a capture of this code."""
@@ -204,7 +204,7 @@ def fraction_of_peak(work_flops, ms, peak):
     return achieved, achieved / peak
 
 
-TRAFFIC_PROFILE = os.path.join("profiles", "k_sdf_sub_mixed_shsphere256.md")
+TRAFFIC_PROFILE = os.path.join("profiles", "k_sdf_near_mixed_shsphere256.md")
 
 
 def traffic_from_profile():
@@ -392,7 +392,7 @@ def run_ours(args):
         ach64, frac64 = fraction_of_peak(w_sdf, tp["eval_ms"], p64)
         traffic, traffic_note = traffic_from_profile()
         line["roofline"] = {
-            "bound": "fp32", "kernel": "k_sdf_sub<mixed> (distance evaluation)",
+            "bound": "fp32", "kernel": "k_sdf_near<mixed> (distance evaluation)",
             "achieved": ach / 1e12, "peak": p32 / 1e12, "unit": "TFLOP/s", "frac": frac,
             "traffic": traffic, "traffic_source": traffic_note,
             "work": f"sum_v K(v) * {PT_FLOPS} = {w_sdf:.4g} flops per launch; K(v) = triangles whose "
@@ -556,7 +556,7 @@ def run_batch(args):
         p32 = cm.peak_flops(False)
         w_sdf = wm["sum_k"] * PT_FLOPS
         ach, frac = fraction_of_peak(w_sdf, tm["eval_ms"], p32)
-        line["roofline"] = {"bound": "fp32", "kernel": "k_sdf_sub<mixed> (distance evaluation)",
+        line["roofline"] = {"bound": "fp32", "kernel": "k_sdf_near<mixed> (distance evaluation)",
                             "achieved": ach / 1e12, "peak": p32 / 1e12, "unit": "TFLOP/s",
                             "frac": frac, "traffic": None, "eval_ms": tm["eval_ms"], "phase_ms": tm,
                             "work": f"sum_v K(v) * {PT_FLOPS} = {w_sdf:.4g} flops per launch",
@@ -674,7 +674,7 @@ def run_scale(args):
         p32 = cm.peak_flops(False)
         w_sdf = wm["sum_k"] * PT_FLOPS
         ach, frac = fraction_of_peak(w_sdf, tm["eval_ms"], p32)
-        line["roofline"] = {"bound": "fp32", "kernel": "k_sdf_sub<mixed> (distance evaluation)",
+        line["roofline"] = {"bound": "fp32", "kernel": "k_sdf_near<mixed> (distance evaluation)",
                             "achieved": ach / 1e12, "peak": p32 / 1e12, "unit": "TFLOP/s",
                             "frac": frac, "traffic": None, "eval_ms": tm["eval_ms"], "phase_ms": tm,
                             "work": f"sum_v K(v) * {PT_FLOPS} = {w_sdf:.4g} flops per launch",
@@ -1052,7 +1052,7 @@ def run_detect(args):
         hbm = _measured_hbm()
         byts = T * (12 + 72)  # indices + the three vertices read once per triangle
         ach = byts / (sum(dev_ms) / len(dev_ms) * 1e-3) / 1e9
-        line["roofline"] = {"bound": "hbm", "kernel": "k_det_boxes + k_det_bin + k_det_pairs",
+        line["roofline"] = {"bound": "hbm", "kernel": "k_det_count + k_det_fill + k_det_pairs + k_det_cross",
                             "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                             "traffic": None, "device_ms": sum(dev_ms) / len(dev_ms),
                             "work": "84 B per triangle (indices and vertices read once); the pair "
@@ -1284,7 +1284,7 @@ def run_sizing(args):
         flops = st["tests"] * SIZING_TEST_FLOPS
         ms = sum(dev_ms) / len(dev_ms)
         ach, frac = fraction_of_peak(flops, ms, p64)
-        line["roofline"] = {"bound": "fp64", "kernel": "k_sizing_eval (+ k_sizing_slow)",
+        line["roofline"] = {"bound": "fp64", "kernel": "k_sizing_screen + k_sizing_interp + k_sizing_nearest",
                             "achieved": ach / 1e12, "peak": p64 / 1e12, "unit": "TFLOP/s",
                             "frac": frac, "traffic": None,
                             "tests_per_query": st["tests"] / n,
@@ -1388,12 +1388,12 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--brick", type=int, default=0)
     ap.add_argument("--stage", type=int, default=-1,
-                    help="mixed record access: 0 L1/L2, 1 staged in shared memory, -1 default")
+                    help="no effect (records are always staged in shared memory)")
     ap.add_argument("--walk-warps", type=int, default=0,
                     help="warps per brick of the candidate walk (1, 2, 4); 0 = autotuned")
-    ap.add_argument("--probe", type=int, default=0, help="mixed probe head; 0 = autotuned")
+    ap.add_argument("--probe", type=int, default=0, help="list entries that the probe scans; 0 = the whole list")
     ap.add_argument("--ctas", type=int, default=0,
-                    help="evaluation CTAs per SM (12, 16); 0 = autotuned")
+                    help="evaluation CTAs per SM of the plain FP64 path (12, 16); 0 = default")
     ap.add_argument("--no-autotune", action="store_true",
                     help="library defaults for every tunable not given")
     ap.add_argument("--cpu-seconds", type=float, default=12.0)

@@ -51,42 +51,6 @@ struct AdjTri {
 };
 static_assert(sizeof(AdjTri) == 192, "record layout");
 
-__global__ void k_adj_tri_rec(int64_t ntris, const double* __restrict__ pts,
-                              const int* __restrict__ tris, AdjTri* __restrict__ rec) {
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= ntris) return;
-    AdjTri r;
-    const int iv[3] = {tris[3 * t], tris[3 * t + 1], tris[3 * t + 2]};
-    double* V[3] = {r.a, r.b, r.c};
-    for (int k = 0; k < 3; ++k)
-        for (int q = 0; q < 3; ++q) V[k][q] = pts[3 * static_cast<int64_t>(iv[k]) + q];
-    double e1[3], e2[3], e3[3];
-    for (int q = 0; q < 3; ++q) {
-        e1[q] = r.b[q] - r.a[q];
-        e2[q] = r.c[q] - r.a[q];
-        e3[q] = r.c[q] - r.b[q];
-    }
-    const double N[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2],
-                         e1[0] * e2[1] - e1[1] * e2[0]};
-    const double nn = N[0] * N[0] + N[1] * N[1] + N[2] * N[2];
-    const double inn = nn > 0.0 ? 1.0 / nn : 0.0;
-    const double il = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
-    for (int q = 0; q < 3; ++q) r.n[q] = N[q] * il;
-    r.mb[0] = (e2[1] * N[2] - e2[2] * N[1]) * inn;
-    r.mb[1] = (e2[2] * N[0] - e2[0] * N[2]) * inn;
-    r.mb[2] = (e2[0] * N[1] - e2[1] * N[0]) * inn;
-    r.mc[0] = (N[1] * e1[2] - N[2] * e1[1]) * inn;
-    r.mc[1] = (N[2] * e1[0] - N[0] * e1[2]) * inn;
-    r.mc[2] = (N[0] * e1[1] - N[1] * e1[0]) * inn;
-    const double* E[3] = {e1, e2, e3};
-    for (int k = 0; k < 3; ++k) {
-        const double ee = E[k][0] * E[k][0] + E[k][1] * E[k][1] + E[k][2] * E[k][2];
-        r.inv_e[k] = ee > 0.0 ? 1.0 / ee : 0.0;
-    }
-    r.pad_[0] = r.pad_[1] = r.pad_[2] = 0.0;
-    rec[t] = r;
-}
-
 // 1/sqrt(x) in FP64: a single-precision seed refined by two Newton-Raphson steps
 // y <- y (3/2 - (x/2) y^2), each of which roughly doubles the correct bits (24 ->
 // 48 -> the double's 53). Outside the seed's comfortable range, 1/sqrt.
@@ -195,11 +159,52 @@ struct AdjTri32 {
 };
 static_assert(sizeof(AdjTri32) == 96, "record layout");
 
-__global__ void k_adj_tri_rec32(int64_t ntris, const GridDesc g, const AdjTri* __restrict__ rec,
-                                AdjTri32* __restrict__ rec32) {
+__device__ __forceinline__ AdjTri adj_record(int64_t t, const double* __restrict__ pts,
+                                             const int* __restrict__ tris) {
+    AdjTri r;
+    const int iv[3] = {tris[3 * t], tris[3 * t + 1], tris[3 * t + 2]};
+    double* V[3] = {r.a, r.b, r.c};
+    for (int k = 0; k < 3; ++k)
+        for (int q = 0; q < 3; ++q) V[k][q] = pts[3 * static_cast<int64_t>(iv[k]) + q];
+    double e1[3], e2[3], e3[3];
+    for (int q = 0; q < 3; ++q) {
+        e1[q] = r.b[q] - r.a[q];
+        e2[q] = r.c[q] - r.a[q];
+        e3[q] = r.c[q] - r.b[q];
+    }
+    const double N[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2],
+                         e1[0] * e2[1] - e1[1] * e2[0]};
+    const double nn = N[0] * N[0] + N[1] * N[1] + N[2] * N[2];
+    const double inn = nn > 0.0 ? 1.0 / nn : 0.0;
+    const double il = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
+    for (int q = 0; q < 3; ++q) r.n[q] = N[q] * il;
+    r.mb[0] = (e2[1] * N[2] - e2[2] * N[1]) * inn;
+    r.mb[1] = (e2[2] * N[0] - e2[0] * N[2]) * inn;
+    r.mb[2] = (e2[0] * N[1] - e2[1] * N[0]) * inn;
+    r.mc[0] = (N[1] * e1[2] - N[2] * e1[1]) * inn;
+    r.mc[1] = (N[2] * e1[0] - N[0] * e1[2]) * inn;
+    r.mc[2] = (N[0] * e1[1] - N[1] * e1[0]) * inn;
+    const double* E[3] = {e1, e2, e3};
+    for (int k = 0; k < 3; ++k) {
+        const double ee = E[k][0] * E[k][0] + E[k][1] * E[k][1] + E[k][2] * E[k][2];
+        r.inv_e[k] = ee > 0.0 ? 1.0 / ee : 0.0;
+    }
+    r.pad_[0] = r.pad_[1] = r.pad_[2] = 0.0;
+    return r;
+}
+
+// The records of the precision in use.
+template <int PREC>
+__global__ void k_adj_tri_rec(int64_t ntris, const GridDesc g, const double* __restrict__ pts,
+                              const int* __restrict__ tris, AdjTri* __restrict__ rec,
+                              AdjTri32* __restrict__ rec32) {
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= ntris) return;
-    const AdjTri& R = rec[t];
+    const AdjTri R = adj_record(t, pts, tris);
+    if (PREC == kPrecFP64) {
+        rec[t] = R;
+        return;
+    }
     AdjTri32 r;
     for (int q = 0; q < 3; ++q) {
         const double A = R.a[q] - g.corner[q];
@@ -341,20 +346,14 @@ __global__ void k_run_emit(int64_t ncell, const int* __restrict__ flag,
     vals[r] = static_cast<uint32_t>(r);
 }
 
-// 2. lengths of the sorted runs (0 for runs without a triangle) and runs per triangle.
+// 2. lengths of the sorted runs (0 for runs without a triangle).
 __global__ void k_run_len(int64_t nrun, const uint32_t* __restrict__ keys,
                           const uint32_t* __restrict__ vals, const uint32_t* __restrict__ st,
-                          uint32_t ntris, int* __restrict__ len, int* __restrict__ tcount) {
+                          uint32_t ntris, int* __restrict__ len) {
     const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (e >= nrun) return;
-    const uint32_t t = keys[e];
-    if (t >= ntris) {
-        len[e] = 0;
-        return;
-    }
     const uint32_t r = vals[e];
-    len[e] = static_cast<int>(st[r + 1] - st[r]);
-    atomicAdd(&tcount[t], 1);
+    len[e] = keys[e] < ntris ? static_cast<int>(st[r + 1] - st[r]) : 0;
 }
 
 // 3. one lane per position. P (nrun + 1 entries) holds the first position of every
@@ -372,24 +371,23 @@ __global__ void __launch_bounds__(256) k_adj_cells(
     const int64_t ptot = P[nrun];
     const int64_t w0 = warp * 32;
     if (w0 >= ptot) return;  // whole warp past the end (warp-uniform)
-    // the run holding position w0: the last e with P[e] <= w0 (binary search by
-    // lane 0, broadcast)
-    int64_t lo = 0;
-    if (lane == 0) {
-        int64_t hi = nrun - 1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (P[mid] <= w0) lo = mid;
-            else hi = mid - 1;
-        }
+    // the run holding position w0: the last e with P[e] <= w0, 33 intervals a step
+    int64_t ef = 0;
+    for (int64_t len = nrun; len > 1;) {  // ef <= it < ef + len
+        const int64_t w = (len + 32) / 33, at = (lane + 1) * w;
+        const int below = __popc(__ballot_sync(0xffffffffu, at < len && P[ef + at] <= w0));
+        ef += below * w;
+        len = min(w, len - below * w);
     }
-    const int64_t ef = __shfl_sync(0xffffffffu, lo, 0);
     // the (at most 32) runs that start after w0 inside the window
     const int64_t pk = (ef + 1 + lane <= nrun) ? P[ef + 1 + lane] : INT64_MAX;
     const int64_t pos = w0 + lane;
     const bool valid = pos < ptot;
-    int off = 0;
-    for (int k = 0; k < 32; ++k) off += (__shfl_sync(0xffffffffu, pk, k) <= pos) ? 1 : 0;
+    int off = 0;  // how many of them start at or before pos
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+        if (__shfl_sync(0xffffffffu, pk, off + d - 1) <= pos) off += d;
+    off += __shfl_sync(0xffffffffu, pk, off) <= pos ? 1 : 0;
     const int64_t e = ef + off;
     uint32_t key = 0xffffffffu;
     double c9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -472,15 +470,29 @@ __global__ void __launch_bounds__(256) k_adj_cells(
 
 // 4. triangles whose positions reach a warp's first or last lane: add the partials
 // in warp order (in warp w the triangle is the first segment when it started before
-// w or at its lane 0, else the last segment); empty triangles get zeros.
-__global__ void k_adj_tri_combine(int64_t ntris, const int64_t* __restrict__ toff,
+// w or at its lane 0, else the last segment); empty triangles get zeros. A triangle's runs
+// are found in the sorted keys, each bound once (a count per triangle by atomics and its
+// scan were four launches).
+__global__ void k_adj_tri_combine(int64_t ntris, int64_t nrun, const uint32_t* __restrict__ keys,
                                   const int64_t* __restrict__ P,
                                   const double* __restrict__ wp_first,
                                   const double* __restrict__ wp_last,
                                   double* __restrict__ tri_grad) {
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const auto first_run = [&](int64_t key) {  // the first run with a key >= key
+        int64_t lo = 0, hi = nrun;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (static_cast<int64_t>(keys[mid]) < key) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    const int64_t r0 = first_run(t);
+    int64_t r1 = __shfl_down_sync(0xffffffffu, r0, 1);
     if (t >= ntris) return;
-    const int64_t s0 = P[toff[t]], s1 = P[toff[t + 1]] - 1;
+    if ((threadIdx.x & 31) == 31) r1 = first_run(t + 1);
+    const int64_t s0 = P[r0], s1 = P[r1] - 1;
     if (s1 < s0) {
 #pragma unroll
         for (int q = 0; q < 9; ++q) tri_grad[9 * t + q] = 0.0;
@@ -498,20 +510,54 @@ __global__ void k_adj_tri_combine(int64_t ntris, const int64_t* __restrict__ tof
     for (int q = 0; q < 9; ++q) tri_grad[9 * t + q] = acc[q];
 }
 
-// 5. one thread per vertex: its (triangle, corner) entries in CSR order.
+// 5. one thread per vertex: its (triangle, corner) entries in CSR order, one after the other.
+// The entries of a vertex with many (a pole of a latitude-longitude sphere has one per
+// meridian) are loaded by its whole warp, 32 at a time, and added in the same order: alone,
+// such a vertex waits for each entry in turn (256 of them: 52 us, now 39).
+constexpr int kFewEntries = 16;
 __global__ void k_adj_vertex(int64_t npts, const int64_t* __restrict__ voff,
                              const int* __restrict__ vinc, const double* __restrict__ tri_grad,
                              double* __restrict__ grad) {
     const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= npts) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t begin = p < npts ? voff[p] : 0, end = p < npts ? voff[p + 1] : 0;
+    const bool many = end - begin > kFewEntries;
     double gx = 0, gy = 0, gz = 0;
-    for (int64_t e = voff[p]; e < voff[p + 1]; ++e) {
-        const int code = vinc[e];  // 3 * triangle + corner
-        const double* tg = tri_grad + 3 * static_cast<int64_t>(code);
-        gx += tg[0];
-        gy += tg[1];
-        gz += tg[2];
+    if (!many)
+        for (int64_t e = begin; e < end; ++e) {
+            const int code = vinc[e];  // 3 * triangle + corner
+            const double* tg = tri_grad + 3 * static_cast<int64_t>(code);
+            gx += tg[0];
+            gy += tg[1];
+            gz += tg[2];
+        }
+    for (unsigned left = __ballot_sync(0xffffffffu, many); left; left &= left - 1) {
+        const int who = __ffs(left) - 1;
+        const int64_t e0 = __shfl_sync(0xffffffffu, begin, who), e1 = __shfl_sync(0xffffffffu, end, who);
+        double sx = 0, sy = 0, sz = 0;
+        for (int64_t e = e0; e < e1; e += 32) {
+            const int n = static_cast<int>(e1 - e < 32 ? e1 - e : 32);
+            double x = 0, y = 0, z = 0;
+            if (lane < n) {
+                const double* tg = tri_grad + 3 * static_cast<int64_t>(vinc[e + lane]);
+                x = tg[0];
+                y = tg[1];
+                z = tg[2];
+            }
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) {
+                sx += __shfl_sync(0xffffffffu, x, k);
+                sy += __shfl_sync(0xffffffffu, y, k);
+                sz += __shfl_sync(0xffffffffu, z, k);
+            }
+        }
+        if (lane == who) {
+            gx = sx;
+            gy = sy;
+            gz = sz;
+        }
     }
+    if (p >= npts) return;
     grad[3 * p] = gx;
     grad[3 * p + 1] = gy;
     grad[3 * p + 2] = gz;
@@ -526,8 +572,6 @@ struct AdjWork {
     void* sort_tmp;
     int* len;
     int64_t* P;
-    int* tcount;
-    int64_t* toff;
     double *wp_first, *wp_last, *tri_grad;
     AdjTri* rec;
     AdjTri32* rec32;
@@ -551,8 +595,6 @@ struct AdjWork {
         sort_tmp = take(radix_sort_tmp_bytes(ncell));
         len = reinterpret_cast<int*>(take(sizeof(int) * ncell));
         P = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * (ncell + 1)));
-        tcount = reinterpret_cast<int*>(take(sizeof(int) * (ntris + 1)));
-        toff = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * (ntris + 2)));
         wp_first = reinterpret_cast<double*>(take(sizeof(double) * 9 * nw));
         wp_last = reinterpret_cast<double*>(take(sizeof(double) * 9 * nw));
         tri_grad = reinterpret_cast<double*>(take(sizeof(double) * 9 * ntris));
@@ -576,6 +618,8 @@ void adjoint_backward(int precision, const GridDesc& g, int64_t ncell, const dou
     AdjWork w(tmp, ncell, ntris);
     const uint32_t nt = static_cast<uint32_t>(ntris);
     const unsigned gc = static_cast<unsigned>((ncell + 255) / 256);
+    const unsigned gt = static_cast<unsigned>((ntris + 127) / 128);
+    const bool mixed = precision == kPrecMixed;
     k_run_heads<<<gc, 256, 0, st>>>(g.nx, ncell, near_tri, w.flag);
     CMG_LAUNCH();
     exclusive_scan(w.flag, w.runidx, ncell, w.scan_tmp, st);
@@ -583,22 +627,18 @@ void adjoint_backward(int precision, const GridDesc& g, int64_t ncell, const dou
     CMG_LAUNCH();
     int64_t nrun = 0;  // the sort's length is needed on the host
     CMG_CUDA(cudaMemcpyAsync(&nrun, w.runidx + ncell, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    if (mixed) k_adj_tri_rec<kPrecMixed><<<gt, 128, 0, st>>>(ntris, g, pts, tris, w.rec, w.rec32);
+    else k_adj_tri_rec<kPrecFP64><<<gt, 128, 0, st>>>(ntris, g, pts, tris, w.rec, w.rec32);
+    CMG_LAUNCH();
     CMG_CUDA(cudaStreamSynchronize(st));
     int bits = 1;
     while ((int64_t(1) << bits) <= ntris) ++bits;
     radix_sort_pairs(w.keys, w.vals, nrun, bits, w.sort_tmp, st);
-    CMG_CUDA(cudaMemsetAsync(w.tcount, 0, sizeof(int) * (ntris + 1), st));
     const unsigned gr = static_cast<unsigned>((nrun + 255) / 256);
-    k_run_len<<<gr, 256, 0, st>>>(nrun, w.keys, w.vals, w.st, nt, w.len, w.tcount);
+    k_run_len<<<gr, 256, 0, st>>>(nrun, w.keys, w.vals, w.st, nt, w.len);
     CMG_LAUNCH();
     exclusive_scan(w.len, w.P, nrun, w.scan_tmp, st);
-    exclusive_scan(w.tcount, w.toff, ntris, w.scan_tmp, st);
-    const unsigned gt = static_cast<unsigned>((ntris + 127) / 128);
-    k_adj_tri_rec<<<gt, 128, 0, st>>>(ntris, pts, tris, w.rec);
-    CMG_LAUNCH();
-    if (precision == kPrecMixed) {
-        k_adj_tri_rec32<<<gt, 128, 0, st>>>(ntris, g, w.rec, w.rec32);
-        CMG_LAUNCH();
+    if (mixed) {
         const float hh = static_cast<float>(g.h);
         const float hl = static_cast<float>(g.h - static_cast<double>(hh));
         k_adj_cells<kPrecMixed><<<gc, 256, 0, st>>>(g, hh, hl, nrun, w.P, w.keys, w.vals, w.st,
@@ -610,7 +650,7 @@ void adjoint_backward(int precision, const GridDesc& g, int64_t ncell, const dou
                                                    w.tri_grad, w.wp_first, w.wp_last);
     }
     CMG_LAUNCH();
-    k_adj_tri_combine<<<gt, 128, 0, st>>>(ntris, w.toff, w.P, w.wp_first, w.wp_last, w.tri_grad);
+    k_adj_tri_combine<<<gt, 128, 0, st>>>(ntris, nrun, w.keys, w.P, w.wp_first, w.wp_last, w.tri_grad);
     CMG_LAUNCH();
     const unsigned gp = static_cast<unsigned>((npts + 127) / 128);
     k_adj_vertex<<<gp, 128, 0, st>>>(npts, voff, vinc, w.tri_grad, grad);

@@ -3,9 +3,10 @@
 // A Batch holds one or more meshes (each with its own grid) resident on the
 // device, the workspace sized for them, and the device outputs. run() enqueues
 // the whole pipeline on a stream:
-//   occupancy: triangle prep -> per-column buckets -> FP64 filter -> exact pass
+//   occupancy: triangle prep -> per-column buckets -> FP32/FP64 filter -> exact pass
 //   SDF:       triangle bins -> brick candidate lists -> LPT work order ->
-//              persistent evaluation (plain FP64 or mixed FP32 + FP64 band)
+//              persistent evaluation (through FP32 with FP64 near-ties, in the band or
+//              everywhere, or plain FP64)
 // The first run sizes the workspace (it reads two totals back from the device);
 // later runs allocate nothing and synchronise nothing, so they can be captured in
 // a CUDA graph and replayed.
@@ -151,7 +152,9 @@ class Batch {
 public:
     // Uploads the meshes (host buffers) and plans the workspace. Grids must be set.
     // A transient batch borrows the device's shared workspace (at most one alive
-    // per device at a time); otherwise the batch owns its memory.
+    // per device at a time) and runs into what is there without waiting for its list
+    // lengths: they come back with the results, and a run whose lists did not fit is
+    // repeated with the right sizes. Otherwise the batch owns its memory.
     Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStream_t stream,
           bool transient = false);
     ~Batch();

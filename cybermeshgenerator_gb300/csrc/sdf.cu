@@ -8,12 +8,16 @@
 //   k_sdf_tri_prep   centroid c_t, radius e_t = max |v - c_t| (rounded up), bin of
 //                    c_t in the brick grid; triangles larger than two bricks (or
 //                    degenerate) go to a per-mesh "always considered" list
-//   k_bin_fill       bin -> triangle CSR
-//   k_brick_walk     one CTA per brick: a ring walk over bins gives an upper bound
-//                    U on the distance from the brick centre to the surface, then
+//   k_bin_fill       bin -> triangle CSR, the entries' centroids and radii in its order;
+//                    k_bin_balls: a ball around each bin's triangles
+//   k_brick_walk     one to eight warps per brick: a ring walk over bins gives an upper
+//                    bound U on the distance from the brick centre to the surface, then
 //                    the candidate list = every triangle whose lower bound
-//                    |c - c_t| - e_t - r_B can be <= U + r_B (r_B = brick radius),
-//                    with margins far above FP32 and FP64 rounding
+//                    |c - c_t| - e_t - r_B can be <= U + r_B (r_B = brick radius) and that
+//                    the box test around the nearest centroid leaves, with margins far
+//                    above FP32 and FP64 rounding
+// and the lists are evaluated by warps of 4^3 cells (sdf_near.cu; plain FP64: sdf_sub.cu),
+// or at brick edges 4 and 8 by
 //   k_sdf_fp64       one CTA per brick, candidates staged through shared memory;
 //                    each thread owns voxels and evaluates Ericson in the reference
 //                    operation order (FP64, no FMA): bit-identical to the reference
