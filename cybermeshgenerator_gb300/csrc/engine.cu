@@ -663,10 +663,11 @@ void Batch::run_impl(bool sizing) {
         launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.tinfo, I.bin_list, I.bin_info, nbrick_,
                         I.bin_ball, I.bin_reach, dsegs_, nseg, I.large_cnt + nseg, I.large_list, ss);
     };
+    const bool eight = std::any_of(segs_.begin(), segs_.end(), [](const MeshSeg& s) { return s.walk_warps == 8; });
     auto walk = [&]() {
         launch_brick_walk(dsegs_, nseg, nwalk_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off, I.bin_list,
                           I.bin_info, I.bin_ball, I.bin_reach, I.large_list, I.cand_cnt, I.cand_rng, I.cand,
-                          I.cand_c, cand_cap_, I.brick_emax, stats_, ss);
+                          I.cand_c, cand_cap_, I.brick_emax, stats_, eight, ss);
     };
     if (cand_cap_ < 0) plan_cands(entries_of(I.cands, kCandBytes));
     // reads the walk's total back; lists that did not fit are sized (with an eighth to

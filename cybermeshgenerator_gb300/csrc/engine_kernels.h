@@ -58,12 +58,13 @@ void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsi
 // cand (cap entries), in no particular order; stats->candidates (zero before) gets the
 // total. A total above cap leaves lists out: the caller sizes cand and walks again.
 // cand_c (null: not wanted): per candidate, its centroid from the brick's centre and radius.
+// eight: whether some mesh has eight-warp bricks.
 void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double* soup,
                        const float4* tinfo, const float4* tlo, const float4* thi,
                        const int64_t* bin_off, const int* bin_list, const float4* bin_info,
                        const float4* bin_ball, const float* bin_reach, const int* large_list,
                        int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
-                       float* brick_emax, Stats* stats, cudaStream_t st);
+                       float* brick_emax, Stats* stats, bool eight, cudaStream_t st);
 // Warps per brick the walk uses for a mesh of a batch of nbricks in all (walk_warps when it
 // is 1, 2 or 4, else by the counts), and its CTAs for that.
 int brick_walk_warps(int64_t nbricks, int64_t mesh_bricks, int64_t mesh_tris, int walk_warps);

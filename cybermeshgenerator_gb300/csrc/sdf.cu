@@ -460,9 +460,7 @@ __device__ __forceinline__ float aabb_dist(float cx, float cy, float cz, float4 
 // warp takes 32 x R entries per round (R loads in flight per lane, across bin
 // boundaries); f(e, ok) gets the R entry positions of this lane and whether each
 // exists. The trip count is warp-uniform, so f may use warp votes.
-constexpr int kWalkRounds = 4;
-
-template <class F>
+template <int kWalkRounds, class F>
 __device__ __forceinline__ void for_group_entries(int64_t b0, int64_t b1, int lane, F&& f) {
     const int len = static_cast<int>(b1 - b0);
     int inc = len;
@@ -511,7 +509,8 @@ __device__ __forceinline__ void for_group_entries(int64_t b0, int64_t b1, int la
 // one per warp, and each warp writes its own entries after those of the warps before it;
 // the bound is reduced over the brick's warps after each shell (a named barrier per brick).
 // (231x247x256 surface, 65k triangles, W = 4: 0.57 + 0.87 ms for a counting and a writing
-// kernel that gathered every entry of every shell's bins -> 0.56 ms.)
+// kernel that gathered every entry of every shell's bins -> 0.56 ms -> 0.52 ms in the order
+// below.)
 constexpr int kWalkThreads = 256;
 
 // Brick number k of the mesh when they are taken from the middle of the grid outward, layer
@@ -526,22 +525,21 @@ __device__ __forceinline__ int64_t centre_first(const MeshSeg& s, int64_t k) {
 }
 
 
-__global__ void __launch_bounds__(kWalkThreads, 3)
-k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
-             const double* __restrict__ soup, const float4* __restrict__ tinfo,
-             const float4* __restrict__ tlo, const float4* __restrict__ thi,
-             const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
-             const float4* __restrict__ bin_info, const float4* __restrict__ bin_ball,
-             const float* __restrict__ bin_reach, const int* __restrict__ large_list,
-             int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
-             float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
-             Stats* __restrict__ st) {
+template <int kWalkRounds>
+__device__ __forceinline__ void brick_walk(const MeshSeg& turn, const MeshSeg* __restrict__ segs, int nseg,
+           const double* __restrict__ soup, const float4* __restrict__ tinfo,
+           const float4* __restrict__ tlo, const float4* __restrict__ thi,
+           const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
+           const float4* __restrict__ bin_info, const float4* __restrict__ bin_ball,
+           const float* __restrict__ bin_reach, const int* __restrict__ large_list,
+           int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
+           float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
+           Stats* __restrict__ st) {
     constexpr int kWarps = kWalkThreads / 32;
     __shared__ float4 s_q[kWarps];
     __shared__ int s_c[kWarps];
     __shared__ long long s_off[kWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const MeshSeg& turn = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
     const MeshSeg& s = segs[turn.walk_seg];
     const int W = s.walk_warps;
     const int slot = wid / W, sub = wid % W;  // brick within the CTA, warp within the brick
@@ -625,7 +623,7 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
                     b1 = bin_off[bin + 1];
                 }
             }
-            for_group_entries(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
+            for_group_entries<kWalkRounds>(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
                 float4 t[kWalkRounds];
 #pragma unroll
                 for (int j = 0; j < kWalkRounds; ++j)
@@ -665,8 +663,8 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
         const float d2 = fmaf(x, x, fmaf(y, y, z * z)), l = lim + w;  // |v - c| - w >= d - r_B - w
         return !(d2 > l * l * (1.f + 16.f * kU32)) && (!boxed || box_ball(box, x, y, z, w, tol));
     };
-    // walks this warp's groups of every shell; f(take, entry, info) per entry, in walk order,
-    // called by the whole warp
+    // walks this warp's groups of every shell; f(take, entry, info) per kWalkRounds entries of
+    // each lane, in walk order, called by the whole warp
     auto walk = [&](auto&& f) {
         for (int r = 0; r <= rmax; ++r) {
             if (r > 0 && (r - 1) * bw - emax > lim) break;
@@ -683,14 +681,16 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
                         b1 = bin_off[bin + 1];
                     }
                 }
-                for_group_entries(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
+                for_group_entries<kWalkRounds>(b0, b1, lane, [&](const int64_t* e, const bool* ok) {
                     float4 t[kWalkRounds];
 #pragma unroll
                     for (int j = 0; j < kWalkRounds; ++j)
                         t[j] = ok[j] ? bin_info[e[j]] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    bool take[kWalkRounds];
 #pragma unroll
                     for (int j = 0; j < kWalkRounds; ++j)
-                        f(ok[j] && reaches(t[j].x - q.cx, t[j].y - q.cy, t[j].z - q.cz, t[j].w), e[j], t[j]);
+                        take[j] = ok[j] && reaches(t[j].x - q.cx, t[j].y - q.cy, t[j].z - q.cz, t[j].w);
+                    f(take, e, t);
                 });
             }
         }
@@ -711,9 +711,12 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
         }
     };
     int mine = 0;
-    auto count = [&](bool take, auto, const float4&) { mine += __popc(__ballot_sync(0xffffffffu, take)); };
-    if (sub == 0) walk_large(count);
-    walk(count);
+    auto count = [&](bool take) { mine += __popc(__ballot_sync(0xffffffffu, take)); };
+    if (sub == 0) walk_large([&](bool take, int, const float4&) { count(take); });
+    walk([&](const bool* take, const int64_t*, const float4*) {
+#pragma unroll
+        for (int j = 0; j < kWalkRounds; ++j) count(take[j]);
+    });
     // ---- 3. the list's place, and the entries
     if (lane == 0) s_c[wid] = mine;
     brick_sync();
@@ -749,7 +752,13 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
         at += __popc(m);
     };
     if (sub == 0) walk_large(put);
-    walk([&](bool take, int64_t e, const float4& ti) { put(take, take ? bin_list[e] : 0, ti); });
+    walk([&](const bool* take, const int64_t* e, const float4* ti) {
+        int id[kWalkRounds];  // (loaded together)
+#pragma unroll
+        for (int j = 0; j < kWalkRounds; ++j) id[j] = take[j] ? bin_list[e[j]] : 0;
+#pragma unroll
+        for (int j = 0; j < kWalkRounds; ++j) put(take[j], id[j], ti[j]);
+    });
     {
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
         bemax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bemax)));
@@ -761,6 +770,30 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
         }
         if (sub == 0 && lane == 0) brick_emax[gb] = bemax;
     }
+}
+
+// Eight-warp bricks have long walks of full groups and take eight entries per lane and round,
+// the others four; a launch with eight-warp bricks has 122 registers and two CTAs per SM, one
+// without 80 and three, which leaves room for the occupancy passes beside it. (137^3 around
+// 128k triangles 0.43 -> 0.36 ms, 118x126x130 around 65k 0.40 -> 0.32, 24 meshes 1.98 ->
+// 1.68 with eight; 231x247x256, four warps: 0.46 alone with two CTAs against 0.52 with three,
+// but the whole call 0.4 % slower.)
+template <bool EIGHT>
+__global__ void __launch_bounds__(kWalkThreads, EIGHT ? 2 : 3)
+k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
+             const double* __restrict__ soup, const float4* __restrict__ tinfo,
+             const float4* __restrict__ tlo, const float4* __restrict__ thi,
+             const int64_t* __restrict__ bin_off, const int* __restrict__ bin_list,
+             const float4* __restrict__ bin_info, const float4* __restrict__ bin_ball,
+             const float* __restrict__ bin_reach, const int* __restrict__ large_list,
+             int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
+             float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
+             Stats* __restrict__ st) {
+    const MeshSeg& turn = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
+    if (EIGHT && segs[turn.walk_seg].walk_warps == 8)
+        brick_walk<8>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st);
+    else
+        brick_walk<4>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st);
 }
 
 // ------------------------------------------------------------------ evaluation
@@ -1254,11 +1287,15 @@ void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double
                        const int64_t* bin_off, const int* bin_list, const float4* bin_info,
                        const float4* bin_ball, const float* bin_reach, const int* large_list,
                        int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
-                       float* brick_emax, Stats* stats, cudaStream_t st) {
+                       float* brick_emax, Stats* stats, bool eight, cudaStream_t st) {
     if (ctas == 0) return;
-    k_brick_walk<<<static_cast<unsigned>(ctas), kWalkThreads, 0, st>>>(
-        segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list,
-        cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, stats);
+    auto go = [&](auto kernel) {
+        kernel<<<static_cast<unsigned>(ctas), kWalkThreads, 0, st>>>(
+            segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list,
+            cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, stats);
+    };
+    if (eight) go(k_brick_walk<true>);
+    else go(k_brick_walk<false>);
     CMG_LAUNCH();
 }
 
