@@ -41,8 +41,12 @@ namespace {
 using namespace sdf;
 
 constexpr int kWarps = 4;       // independent warps per CTA
-constexpr int kStep = 4;        // list entries per lane and filter step (loads in flight)
-constexpr int kWait = 32 * (kStep + 1);  // entries that can wait for the disc test
+// List entries per lane and scan step (loads in flight): the exact kernel's FP64 part leaves
+// fewer registers (231x247x256, mixed / exact, ms: 4 entries 4.41 / 6.95, 5: 4.39 / 6.97, 6:
+// 4.36 / 7.10, 8: 4.45 / 7.38).
+template <int PREC>
+constexpr int kSteps = PREC == kPrecMixed ? 6 : 4;
+constexpr int kWait = 32 * (kSteps<kPrecMixed> + 1);  // entries that can wait for the disc test
 constexpr int kPairs = 256;     // near-tie pairs kept per sub-brick
 constexpr int kSkip = 512;      // of longer lists the probe reads every other step
 constexpr float kItemCost = 1024.f;  // a sub-brick's fixed work, in list entries
@@ -240,6 +244,7 @@ template <int PREC, bool COOP>
 __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, WarpMem& M, Shared& S,
                                           const WarpMem* all) {
     constexpr bool EXACT = PREC == kPrecExact;
+    constexpr int kStep = kSteps<PREC>;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     const int64_t gb = g.work[item >> 6];  // the bricks in order, 64 sub-bricks each
