@@ -1732,12 +1732,11 @@ void sizing_eval_device(SizingField* S, const double* q, int64_t n, double* out,
         S->slow_cap = cap;
     }
     const int64_t tcells = int64_t(S->f.tg.n[0]) * S->f.tg.n[1] * S->f.tg.n[2];
-    if (!S->nslow) {
-        S->nslow = S->alloc<int>(3);
-        S->kcnt = S->alloc<int>(tcells + 1);
-        S->koff = S->alloc<int64_t>(tcells + 2);
-        S->kscan = S->alloc<int64_t>(scan_tmp_elems(tcells + 1));
-    }
+    // (each asked for by itself: the one that could not be had is had by a later call)
+    if (!S->nslow) S->nslow = S->alloc<int>(3);
+    if (!S->kcnt) S->kcnt = S->alloc<int>(tcells + 1);
+    if (!S->koff) S->koff = S->alloc<int64_t>(tcells + 2);
+    if (!S->kscan) S->kscan = S->alloc<int64_t>(scan_tmp_elems(tcells + 1));
     CMG_CUDA(cudaMemsetAsync(S->nslow, 0, 3 * sizeof(int), st));
     CMG_CUDA(cudaMemsetAsync(S->ctr, 0, sizeof(EvalCounters), st));
     // A counting sort passes once over the cells and twice over the queries, the radix sort
