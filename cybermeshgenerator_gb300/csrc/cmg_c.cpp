@@ -169,7 +169,7 @@ cmg::gpu::HostVec<int> fan(const cmg_plc& p) {
 bool make_grid(const double* pts, size_t n, int resolution, int pad, GridDesc& g) {
     // eight points at a time, each coordinate its own minimum and maximum, all starting from the
     // first point (independent comparisons, which the compiler runs as vectors); the minimum
-    // of those in order is the minimum in order
+    // of those is the minimum in order, but for a zero's sign (below)
     constexpr size_t kB = 24;
     double pl[kB], ph[kB];
     for (size_t j = 0; j < kB; ++j) pl[j] = ph[j] = pts[j % 3];
@@ -204,6 +204,11 @@ bool make_grid(const double* pts, size_t n, int resolution, int pad, GridDesc& g
         int core = std::max(1, static_cast<int>(std::ceil(e / g.h)));
         double covered = core * g.h;
         g.corner[a] = lo[a] - (covered - e) / 2.0 - pad * g.h;
+        if (g.corner[a] == 0.0 && lo[a] == 0.0) {  // the first least point's zero
+            size_t k = a;
+            while (pts[k] != 0.0) k += 3;
+            g.corner[a] = pts[k] - (covered - e) / 2.0 - pad * g.h;
+        }
         *dims[a] = core + 2 * pad;
     }
     return true;
