@@ -437,6 +437,24 @@ cmg_status voxelize_host(const double* pts, int64_t npts, const int* tris, int64
 }  // namespace cmg::gpu
 
 namespace {
+// Runs append, which adds facets to the PLC's arrays; where memory runs out on the way, the
+// arrays are cut back to what they held.
+template <typename F>
+cmg_status add_facets(cmg_plc& p, F&& append) {
+    const size_t indices = p.fidx.size(), facets = p.foff.size() - 1;
+    const bool triangles = p.triangles;
+    try {
+        append();
+    } catch (...) {
+        p.fidx.resize(indices);
+        p.foff.resize(facets + 1);
+        p.markers.resize(facets);
+        p.triangles = triangles;
+        return CMG_ERR_INTERNAL;
+    }
+    return CMG_OK;
+}
+
 // Blocks handed out by cmg_host_alloc: capacity and whether page-locked.
 struct HostBlocks {
     std::mutex mu;
@@ -467,29 +485,23 @@ cmg_status cmg_plc_set_points(cmg_plc* plc, const double* xyz, size_t count) {
 cmg_status cmg_plc_add_facet(cmg_plc* plc, const int* idx, size_t count, int marker) {
     if (!plc || (!idx && count)) return CMG_ERR_INVALID_INPUT;
     if (count < 3) return CMG_ERR_INVALID_INPUT;
-    try {
+    return add_facets(*plc, [&] {
         plc->triangles = plc->triangles && count == 3;
         plc->fidx.insert(plc->fidx.end(), idx, idx + count);
         plc->foff.push_back(plc->fidx.size());
         plc->markers.push_back(marker);
-    } catch (...) {
-        return CMG_ERR_INTERNAL;
-    }
-    return CMG_OK;
+    });
 }
 
 cmg_status cmg_plc_add_triangles(cmg_plc* plc, const int* idx, size_t count, int marker) {
     if (!plc || (!idx && count)) return CMG_ERR_INVALID_INPUT;
-    try {
+    return add_facets(*plc, [&] {
         plc->fidx.insert(plc->fidx.end(), idx, idx + 3 * count);
         const size_t base = plc->foff.back();
         plc->foff.reserve(plc->foff.size() + count);
         for (size_t f = 1; f <= count; ++f) plc->foff.push_back(base + 3 * f);
         plc->markers.insert(plc->markers.end(), count, marker);
-    } catch (...) {
-        return CMG_ERR_INTERNAL;
-    }
-    return CMG_OK;
+    });
 }
 
 cmg_status cmg_plc_add_hole(cmg_plc* plc, double x, double y, double z) {
