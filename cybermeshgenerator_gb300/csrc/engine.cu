@@ -506,14 +506,17 @@ void Batch::update_points_device(const double* d_pts) {
     resize_ = true;
 }
 
-// A sizing pass: reads the list totals back, grows the list arenas if needed and
-// drops the captured graph when a grown arena moved the buffers it refers to.
+// A sizing pass: reads the list totals back, grows the list arenas if needed and drops the
+// captured graph when the buffers or the list lengths that it was captured with (its kernels
+// leave out longer lists) are no longer those in use.
 void Batch::sized_run() {
-    const size_t pc = impl_->pairs.capacity(), cc = impl_->cands.capacity();
-    const int64_t cap = cand_cap_;
+    const auto plan = [&] {
+        return std::make_tuple(impl_->pairs.capacity(), impl_->cands.capacity(), pairs_cap_, cand_cap_);
+    };
+    const auto before = plan();
     run_impl(true);
     resize_ = false;
-    if ((impl_->pairs.capacity() != pc || impl_->cands.capacity() != cc || cand_cap_ != cap) && graph_) {
+    if (plan() != before && graph_) {
         CMG_CUDA(cudaStreamSynchronize(stream_));
         CMG_CUDA(cudaGraphExecDestroy(graph_));
         graph_ = nullptr;
