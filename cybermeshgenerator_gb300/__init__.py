@@ -294,9 +294,19 @@ def _to_xyz(flat: np.ndarray, dims) -> np.ndarray:
     return flat.reshape((nz, ny, nx)).transpose(2, 1, 0).copy()
 
 
+#: voxelize()'s grids up to this size are copied out of the call's page-locked block (a block
+#: is 64 KiB at least and may be 1 MiB larger than the grid; the copy takes 5 us)
+_COPY_BYTES = 128 << 10
+#: page-locked memory that living grids of voxelize() may hold; those beyond it are copies
+_KEEP_BYTES = 4 << 30
+
+
 def voxelize(plc: PLC, resolution: int = 64, mode="occupancy", pad: int = 1) -> VoxelGrid:
     """Voxelize a PLC (reference semantics: resolution cells on the longest axis,
-    pad margin cells; "occupancy"/0 -> uint8, "sdf"/1 -> float32)."""
+    pad margin cells; "occupancy"/0 -> uint8, "sdf"/1 -> float32). A grid above 128 KiB
+    views the page-locked block that the device wrote it to, which goes back to the pool
+    of such blocks when the array goes; living grids hold up to 4 GiB of locked memory
+    this way, and further ones are copies in the caller's own memory."""
     if not isinstance(plc, PLC):
         raise TypeError("plc must be a PLC")
     code, name = _mode(mode)
@@ -304,13 +314,15 @@ def voxelize(plc: PLC, resolution: int = 64, mode="occupancy", pad: int = 1) -> 
     err = ctypes.create_string_buffer(256)
     _check(_clib.cmg_plc_voxelize_xyz(plc._handle, int(resolution), code, int(pad), ctypes.byref(out),
                                      err, 256), err)
-    # the array views the handle's page-locked block (no host copy: the device wrote it in
-    # this order), which lives as long as the array
+    # the array views the handle's page-locked block where it may (no host copy: the device
+    # wrote it in this order), which then lives as long as the array
     h, owner = out.value, _Owner(out.value)
     dims, origin, spacing = _geometry(h)
     fn, dtype = (_clib.cmg_voxels_occupancy, np.uint8) if code == 0 else (_clib.cmg_voxels_distance, np.float32)
     ptr = ctypes.cast(fn(h), ctypes.c_void_p).value
     grid = np.asarray(_View(owner, ptr, dims[0] * dims[1] * dims[2], dtype)).reshape(dims)
+    if grid.nbytes <= _COPY_BYTES or not _clib.cmg_voxels_keep(h, _KEEP_BYTES):
+        grid = grid.copy()
     return VoxelGrid(grid=grid, origin=origin, spacing=spacing, mode=name)
 
 

@@ -151,6 +151,7 @@ def _bind(lib: ctypes.CDLL) -> None:
     sig("cmg_plc_voxelize", I, [V, I, I, I, c_void_pp, S, Z])
     sig("cmg_plc_voxelize_xyz", I, [V, I, I, I, c_void_pp, S, Z])
     sig("cmg_voxels_destroy", None, [V])
+    sig("cmg_voxels_keep", I, [V, Z])
     sig("cmg_voxels_dims", None, [V, c_int_p, c_int_p, c_int_p])
     sig("cmg_voxels_origin", None, [V, c_double_p, c_double_p, c_double_p])
     sig("cmg_voxels_spacing", D, [V])

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cctype>
 #include <climits>
 #include <cmath>
@@ -66,7 +67,11 @@ struct cmg_options {
 
 struct cmg_mesh {};
 
+// Page-locked bytes of the handles that callers keep for their arrays (cmg_voxels_keep).
+static std::atomic<size_t> g_kept_bytes{0};
+
 struct cmg_voxels {
+    ~cmg_voxels() { g_kept_bytes -= kept; }
     double corner[3] = {0, 0, 0};
     double origin[3] = {0, 0, 0};
     double spacing = 0;
@@ -74,6 +79,7 @@ struct cmg_voxels {
     int z0 = 0, z1 = 0, nz_grid = 0;  // the slab [z0, z1) of the grid's nz_grid layers
     cmg::gpu::HostResult r;
     cmg_voxel_stats stats{};
+    size_t kept = 0;  // this handle's share of g_kept_bytes
 };
 
 struct cmg_batch {
@@ -593,6 +599,19 @@ cmg_status cmg_plc_voxelize_ex(const cmg_plc* in, const cmg_voxel_opts* opts, cm
 }
 
 void cmg_voxels_destroy(cmg_voxels* v) { delete v; }
+
+int cmg_voxels_keep(cmg_voxels* v, size_t limit) {
+    if (!v) return 0;
+    if (v->kept) return 1;
+    const size_t n = v->r.occ.locked_bytes() + v->r.sdf32.locked_bytes() + v->r.sdf64.locked_bytes() +
+                     v->r.near_tri.locked_bytes() + v->r.near_reg.locked_bytes() + v->r.err.locked_bytes();
+    size_t held = g_kept_bytes.load();
+    do {
+        if (held > limit || n > limit - held) return 0;
+    } while (!g_kept_bytes.compare_exchange_weak(held, held + n));
+    v->kept = n;
+    return 1;
+}
 
 void cmg_voxels_dims(const cmg_voxels* v, int* nx, int* ny, int* nz) {
     if (nx) *nx = v ? v->nx : 0;

@@ -87,6 +87,7 @@ public:
     const T* data() const { return p_; }
     size_t size() const { return n_; }
     bool empty() const { return n_ == 0; }
+    size_t locked_bytes() const { return pinned_ ? cap_ : 0; }  // page-locked, the whole block
     T& operator[](size_t i) { return p_[i]; }
     const T& operator[](size_t i) const { return p_[i]; }
     const T* begin() const { return p_; }
