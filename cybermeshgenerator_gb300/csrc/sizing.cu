@@ -1254,7 +1254,8 @@ __global__ void __launch_bounds__(128) k_sizing_rest(Field F, const double* __re
                                                      EvalCounters* __restrict__ ctr) {
     unsigned inside = 0, tests = 0, boxed = 0;
     const int nr = left[0];
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nr; e += gridDim.x * blockDim.x) {
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < nr;
+         e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t pos = rest[e], i = order[pos];
         const P3 p{q[3 * i], q[3 * i + 1], q[3 * i + 2]};
         const Q32 q32 = make_q32(p);
@@ -1333,7 +1334,8 @@ __global__ void __launch_bounds__(128) k_sizing_nearest(Field F, const double* _
                                                         EvalCounters* __restrict__ ctr) {
     const int nl = left[1];
     unsigned nearest = 0;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nl; e += gridDim.x * blockDim.x) {
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < nl;
+         e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t i = order[lost[e]];
         const P3 p{q[3 * i], q[3 * i + 1], q[3 * i + 2]};
         const Q32 q32 = make_q32(p);
