@@ -1769,14 +1769,15 @@ void sizing_eval_device(SizingField* S, const double* q, int64_t n, double* out,
         S->f, q, S->skey, S->order, n, S->hits, S->rest, S->lost, left, out, which, S->ctr);
     CMG_LAUNCH();
     // (their lists' lengths are known on the device only)
-    const unsigned few = static_cast<unsigned>(std::min<int64_t>((n + 127) / 128, 152 * 16));
+    const unsigned sms = device_sms();
+    const unsigned few = static_cast<unsigned>(std::min<int64_t>((n + 127) / 128, sms * 16));
     k_sizing_rest<<<few, 128, 0, st>>>(S->f, q, S->skey, S->order, S->hits, S->rest, S->lost, left, out, which,
                                        S->ctr);
     CMG_LAUNCH();
     k_sizing_nearest<<<few, 128, 0, st>>>(S->f, q, S->order, S->lost, left, out, which, S->ctr);
     CMG_LAUNCH();
     // the slow queries are the tail of the sorted order
-    k_sizing_slow<<<152 * 4, kThreads, 0, st>>>(S->f, q, S->order, n, S->nslow, out, which, S->ctr);
+    k_sizing_slow<<<sms * 4, kThreads, 0, st>>>(S->f, q, S->order, n, S->nslow, out, which, S->ctr);
     CMG_LAUNCH();
 }
 
