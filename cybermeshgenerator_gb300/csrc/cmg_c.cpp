@@ -277,7 +277,6 @@ cmg::gpu::VoxOpts to_vox(const cmg_voxel_opts& o, int outputs) {
     v.want_err = outputs & CMG_OUT_ERROR_BOUND;
     v.autotune = o.autotune != 0;
     v.grab = o.grab;
-    v.stage = o.stage;
     v.walk_warps = o.walk_warps;
     v.probe = o.probe;
     v.ctas = o.ctas;

@@ -40,12 +40,6 @@ __device__ __forceinline__ SubGeo sub_geo(const MeshSeg& s, int64_t lb, int sub)
 __device__ __forceinline__ float span_centre(int x0, int x1, float h) {
     return __fmul_rn(__fmul_rn(0.5f, static_cast<float>(x0 + x1)), h);
 }
-// The centre (as span_centre) of the brick that holds cell (x, y, z).
-__device__ __forceinline__ float3 brick_centre(const MeshSeg& s, int x, int y, int z, float h) {
-    const int B = s.brick, bx = x / B * B, by = y / B * B, bz = z / B * B;
-    return make_float3(span_centre(bx, min(bx + B, s.g.nx), h), span_centre(by, min(by + B, s.g.ny), h),
-                       span_centre(bz, min(bz + B, s.g.nz), h));
-}
 // Position error of FP32 centroids without their lo parts, over a mesh of that scale.
 __device__ __forceinline__ float list_tol(float scale) { return fmaf(8.f * 5.9604645e-8f, scale, 1e-30f); }
 

@@ -417,7 +417,6 @@ Batch::Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStrea
     impl_->grid_exact = 2 * sms;
     // persistent evaluation grid: resident CTAs per SM for the chosen kernel
     if (opts_.grab <= 0) opts_.grab = 1;
-    if (opts_.stage < 0) opts_.stage = 0;
     if (brick == 16) {
         const int prec = sub_precision(opts_);
         impl_->grid_eval = !sdf ? sms : (prec == kPrecFP64 ? sdf_sub_grid(opts_.ctas) : sdf_near_grid(prec));
@@ -850,7 +849,7 @@ void Batch::download(std::vector<HostResult>& out, RunInfo* info) {
 // workload shape.
 namespace {
 struct Tuned {
-    int brick, grab, walk_warps, probe, ctas;
+    int brick, grab, walk_warps, ctas;
 };
 }  // namespace
 
@@ -873,7 +872,6 @@ void autotune(const std::vector<HostMesh>& meshes, VoxOpts& opts, cudaStream_t s
         opts.brick = t.brick;
         opts.grab = t.grab;
         opts.walk_warps = t.walk_warps;
-        opts.probe = t.probe;
         opts.ctas = t.ctas;
     };
     {
@@ -892,7 +890,6 @@ void autotune(const std::vector<HostMesh>& meshes, VoxOpts& opts, cudaStream_t s
         o.brick = t.brick;
         o.grab = t.grab;
         o.walk_warps = t.walk_warps;
-        o.probe = t.probe;
         o.ctas = t.ctas;
         o.autotune = false;
         Batch bt(meshes, o, stream);
@@ -910,7 +907,7 @@ void autotune(const std::vector<HostMesh>& meshes, VoxOpts& opts, cudaStream_t s
         }
         return best;
     };
-    Tuned cur{16, 1, 0, 0, 0};
+    Tuned cur{16, 1, 0, 0};
     float cur_ms = time_one(cur);
     auto try_set = [&](Tuned t) {
         const float ms = time_one(t);
@@ -919,8 +916,8 @@ void autotune(const std::vector<HostMesh>& meshes, VoxOpts& opts, cudaStream_t s
             cur_ms = ms;
         }
     };
-    try_set({16, 2, 0, 0, 0});
-    try_set({8, 1, 0, 0, 0});
+    try_set({16, 2, 0, 0});
+    try_set({8, 1, 0, 0});
     const Tuned step1 = cur;
     for (int w : {1, 2, 4}) {
         Tuned t = step1;

@@ -42,7 +42,6 @@ struct VoxOpts {
                                    // has x slowest and z fastest (idx = (i*ny + j)*nz + k)
     bool autotune = false;
     int grab = 0;                  // sub-bricks per queue grab (1, 2, 4, 8); 0 = default
-    int stage = -1;                // no effect (records are always staged)
     int walk_warps = 0;            // warps per brick in the candidate walk (1, 2, 4); 0 =
                                    // by the brick count
     int probe = 0;                 // FP32 pass: brick-list head the probe scans; 0 = all of it
