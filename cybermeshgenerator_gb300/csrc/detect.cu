@@ -9,9 +9,13 @@
 //      overlap; the points are rounded to a grid of 2^30 steps, triangles are binned on
 //      a uniform grid of cells by their boxes there, and a pair is examined only in the
 //      cell that holds the low corner of the intersection of the two boxes, so each
-//      candidate pair is seen exactly once;
-//   2. middle phase: pairs whose rounded boxes overlap and that share no vertex are dropped when FP32 certifies that one triangle lies on one side of
-//      the other's plane; nothing of it is FP64;
+//      candidate pair is seen exactly once. (Here the answer can differ from the
+//      reference's: among triangles with coplanar or touching parts, or flat to the
+//      rounding of a determinant, its orientation test also names some pairs whose boxes
+//      are apart, which share no point; these are left out.)
+//   2. middle phase: pairs whose rounded boxes overlap and that share no vertex are dropped
+//      when FP32 certifies that one triangle lies on one side of the other's plane; nothing
+//      of it is FP64;
 //   3. narrow phase, for the pairs left (few, on full warps): the exact boxes, then the
 //      same orientation decisions as the reference (o3d_fast in its order, the exact
 //      sign when it is zero);
@@ -197,9 +201,13 @@ __device__ __forceinline__ float max_abs(const V3& a) { return fmaxf(fabsf(a.x),
 // Whether the corners (a, b, c) certainly have one nonzero orientation with respect to the
 // plane through (p, q, r): the reference's rounded determinants have that sign too. In
 // fixed-point units each difference is off by at most 1 (two roundings of 1/2, a little
-// more with the FP64 product's) and then by u = 2^-24 of itself; with D the largest, the
-// determinants are off by 18 D^2 (1.001 + uD) + 30 u D^3, and the rounded FP64 ones by
-// 5e-15 D^3 (while none of their products leaves FP64's normal range: DetGrid::fx > 0).
+// more with the FP64 product's) and then by u = 2^-24 of itself, d = 1.001 + uD in all with D
+// the largest. A 3x3 matrix M that changes of up to d in its entries make singular has
+// |det M| <= 12 d D^2, all orders included: with v the singular one's null vector, its largest
+// entry 1, M v has entries of at most 3d and can stand in M for that entry's column, and 4 is
+// the largest determinant of entries within 1. The FP32 evaluation adds 30 u D^3, the
+// reference's rounded determinants 5e-15 D^3 (while none of their products leaves FP64's
+// normal range: DetGrid::fx > 0).
 __device__ __forceinline__ bool one_side(const int4& p, const int4& q, const int4& r, const int4& a,
                                          const int4& b, const int4& c) {
     const V3 e = fixed_diff(q, p), f = fixed_diff(r, p);
