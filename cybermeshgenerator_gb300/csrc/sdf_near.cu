@@ -184,7 +184,8 @@ __device__ __forceinline__ float reach_term(float w, float r) {
 // distance is within two stated errors of the cell's FP32 minimum m = sqrt(d2) and its
 // true distance d one more, so d <= m + 3 E(d), E(d) = 48u (d + 2e + 2r), which gives
 // 3 E(d) <= 144.1u m + 288.2u (e + r); with the square root's rounding,
-// sqrt(d2)(1 + 160u) + kapx, kapx = RU(300u (e + r)), covers it. So the FP32 pass
+// sqrt(d2)(1 + 160u) + kapx, kapx = RU(300u (e + r) + 4 kTinyDist), covers it (each of the
+// errors has kTinyDist besides, the ends of FP32's range). So the FP32 pass
 // evaluates every triangle that can be the FP32 minimum or a near-tie of it, whatever
 // order the candidates come in: the cell ends with the exact (FP32 distance, triangle
 // id) minimum over all triangles, independent of which candidates the walk listed.
@@ -193,7 +194,8 @@ __device__ __forceinline__ float cell_bound_x(float d2, float kapx) {
 }
 
 // The near-tie threshold of a cell whose FP32 minimum is sqrt(d2), squared and rounded
-// up: at least (m + 2 eb)^2, eb = 48u (m + 2e + 2r) the stated bound (kap = 98u (e + r)).
+// up: at least (m + 2 eb)^2, eb = 48u (m + 2e + 2r) + kTinyDist the stated bound (kap =
+// 98u (e + r) + kTinyDist).
 __device__ __forceinline__ float near_thr2(float d2, float kap) {
     const float thr = __fmaf_ru(sqrt_approx(d2), 1.f + 100.f * kU32, __fmul_ru(2.f, kap));
     return __fmul_ru(thr, thr);
@@ -297,13 +299,13 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         // the stated FP32 error of a distance near d is 48u (d + 2e + 2r); kap carries its
         // constant part, kapx that of the cells' bounds (three of them)
         const float er = __fadd_ru(emax, r);
-        const float kap = __fmul_ru(98.f * kU32, er);
+        const float kap = __fmaf_ru(98.f * kU32, er, kTinyDist);
         // mixed: near-ties beyond what a band cell can reach are not kept
         float keep2 = FLT_MAX;
         if (!EXACT) {
             const float bh = g.band_cells * static_cast<float>(s.g.h);
             const float far =
-                fmaxf(0.f, __fmaf_ru(fabsf(bh), 512.f * kU32, bh + 16.f * kap + 1e-28f) * (1.f + 8.f * kU32));
+                fmaxf(0.f, __fmaf_ru(fabsf(bh), 512.f * kU32, bh + 16.f * kap) * (1.f + 8.f * kU32));
             keep2 = far * far * (1.f + 8.f * kU32);
         }
         M.thr2[lane] = okA ? keep2 : -1.f;
@@ -317,7 +319,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         if (lane == 0) {
             M.mid[0].w = r;
             M.off.w = list_tol(s.scale);
-            M.con = make_float4(kap, __fmul_ru(300.f * kU32, er), __fmul_ru(4.f, er), keep2);
+            M.con = make_float4(kap, __fmaf_ru(300.f * kU32, er, 4.f * kTinyDist), __fmul_ru(4.f, er), keep2);
         }
         __syncwarp();
     }
@@ -364,7 +366,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const float4 e = recentre(g.tinfo[t], g.tinfo_lo[t], M.mid[0], M.mid[1]);
                 const float dc = sqrt_approx(fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)));
                 const float d = sqrt_approx(dist_rec_val(r, -e.x, -e.y, -e.z));
-                const float ub = d * (1.f + 32.f * kU32) + 32.f * kU32 * (dc + 2.f * e.w);
+                const float ub = d * (1.f + 32.f * kU32) + (32.f * kU32 * (dc + 2.f * e.w) + kTinyDist);
                 if (ub < U || (ub == U && t < seed)) { U = ub; seed = t; }
             }
         }
@@ -554,7 +556,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
     // the grid is evaluated
     const float er2 = 2.f * emax + 2.f * M.mid[0].w;
     const float bh = g.band_cells * static_cast<float>(s.g.h);
-    const float ebA = 48.f * kU32 * (d32A + er2) + 1e-30f, ebB = 48.f * kU32 * (d32B + er2) + 1e-30f;
+    const float ebA = 48.f * kU32 * (d32A + er2) + kTinyDist, ebB = 48.f * kU32 * (d32B + er2) + kTinyDist;
     const bool fineA = okA && (EXACT || d32A <= bh + ebA);
     const bool fineB = okB && (EXACT || d32B <= bh + ebB);
     const unsigned maskA = __ballot_sync(kAll, fineA), maskB = __ballot_sync(kAll, fineB);
