@@ -534,15 +534,17 @@ void Batch::plan_pairs(size_t n) {
     pairs_cap_ = static_cast<int64_t>(n);
 }
 void Batch::plan_cands(size_t n) {
-    const bool near_list = opts_.brick == 16 && sub_precision(opts_) != kPrecFP64;
     impl_->cands.reset();
     impl_->cand = carve<int>(impl_->cands, n);
-    impl_->cand_c = near_list ? carve<float4>(impl_->cands, n) : nullptr;
+    impl_->cand_c = near_list() ? carve<float4>(impl_->cands, n) : nullptr;
     cand_cap_ = static_cast<int64_t>(n);
 }
 
 // Bytes of an arena per entry, and the entries that fit (a few 256-byte roundings aside).
-static constexpr size_t kPairBytes = sizeof(int) + sizeof(double) + 1, kCandBytes = sizeof(int) + sizeof(float4);
+static constexpr size_t kPairBytes = sizeof(int) + sizeof(double) + 1;
+// The warp-per-sub-brick evaluation's lists carry the candidates' centroids and radii.
+bool Batch::near_list() const { return opts_.brick == 16 && sub_precision(opts_) != kPrecFP64; }
+size_t Batch::cand_bytes() const { return sizeof(int) + (near_list() ? sizeof(float4) : 0); }
 static size_t entries_of(const Arena& a, size_t each) {
     return a.capacity() > 4096 ? (a.capacity() - 1024) / each : 0;
 }
@@ -551,11 +553,11 @@ void Batch::run() {
     if (!needs_sizing()) {
         run_impl(false);
     } else if (pooled_ && entries_of(impl_->pairs, kPairBytes) > 0 &&
-               (!(sdf32_ || sdf64_ || near_tri_) || entries_of(impl_->cands, kCandBytes) > 0)) {
+               (!(sdf32_ || sdf64_ || near_tri_) || entries_of(impl_->cands, cand_bytes()) > 0)) {
         // A pooled batch runs into what the pool's arenas hold, without a readback between its
         // passes; a mesh with longer lists than they take is sized and run again (download)
         plan_pairs(entries_of(impl_->pairs, kPairBytes));
-        plan_cands(entries_of(impl_->cands, kCandBytes));
+        plan_cands(entries_of(impl_->cands, cand_bytes()));
         unchecked_ = true;
         run_impl(false);
     } else {
@@ -671,7 +673,7 @@ void Batch::run_impl(bool sizing) {
                           I.bin_info, I.bin_ball, I.bin_reach, I.large_list, I.cand_cnt, I.cand_rng, I.cand,
                           I.cand_c, cand_cap_, I.brick_emax, stats_, eight, ss);
     };
-    if (cand_cap_ < 0) plan_cands(entries_of(I.cands, kCandBytes));
+    if (cand_cap_ < 0) plan_cands(entries_of(I.cands, cand_bytes()));
     // reads the walk's total back; lists that did not fit are sized (with an eighth to
     // spare, for points that move) and walked again
     auto prep_size = [&]() {

@@ -255,6 +255,8 @@ private:
     RunInfo info_of(const Stats& s) const;
     void plan_pairs(size_t n);
     void plan_cands(size_t n);
+    bool near_list() const;
+    size_t cand_bytes() const;
 };
 
 // Sets opts.brick, grab, walk_warps and ctas for a workload by timing the
