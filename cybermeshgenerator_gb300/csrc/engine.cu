@@ -540,6 +540,28 @@ void Batch::plan_cands(size_t n) {
     cand_cap_ = static_cast<int64_t>(n);
 }
 
+// The same for the lengths known, growing their arena (each with an eighth to spare: the next
+// pooled call runs into what is there, and points move).
+void Batch::size_pairs(int64_t n) {
+    Arena& B = impl_->pairs;
+    B.clear_need();
+    plan_pairs(static_cast<size_t>(n));
+    if (!B.overflowed()) return;
+    pairs_cap_ = -1;  // until the allocation has succeeded
+    B.reserve(B.need() + (pooled_ ? B.need() / 8 + 4096 : 0));
+    plan_pairs(static_cast<size_t>(n));
+}
+void Batch::size_cands(int64_t n) {
+    Arena& B = impl_->cands;
+    const size_t room = static_cast<size_t>(n + n / 8);
+    B.clear_need();
+    plan_cands(room);
+    if (!B.overflowed()) return;
+    cand_cap_ = -1;  // until the allocation has succeeded
+    B.reserve(B.need());
+    plan_cands(room);
+}
+
 // Bytes of an arena per entry, and the entries that fit (a few 256-byte roundings aside).
 static constexpr size_t kPairBytes = sizeof(int) + sizeof(double) + 1;
 // The warp-per-sub-brick evaluation's lists carry the candidates' centroids and radii.
@@ -555,7 +577,8 @@ void Batch::run() {
     } else if (pooled_ && entries_of(impl_->pairs, kPairBytes) > 0 &&
                (!(sdf32_ || sdf64_ || near_tri_) || entries_of(impl_->cands, cand_bytes()) > 0)) {
         // A pooled batch runs into what the pool's arenas hold, without a readback between its
-        // passes; a mesh with longer lists than they take is sized and run again (download)
+        // passes; a mesh with longer lists than they take is not evaluated, and run again with
+        // the lengths it found (download)
         plan_pairs(entries_of(impl_->pairs, kPairBytes));
         plan_cands(entries_of(impl_->cands, cand_bytes()));
         unchecked_ = true;
@@ -622,22 +645,15 @@ void Batch::run_impl(bool sizing) {
         int64_t P = 0;
         CMG_CUDA(cudaMemcpyAsync(&P, I.pair_off + ntris_, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         CMG_CUDA(cudaStreamSynchronize(s));
-        I.pairs.clear_need();
-        plan_pairs(static_cast<size_t>(P));
-        if (I.pairs.overflowed()) {
-            pairs_cap_ = -1;  // until the allocation has succeeded
-            // (an eighth to spare: the next pooled call runs into what is there)
-            I.pairs.reserve(I.pairs.need() + (pooled_ ? I.pairs.need() / 8 + 4096 : 0));
-            plan_pairs(static_cast<size_t>(P));
-        }
+        size_pairs(P);
     };
     auto occ_tail = [&](cudaStream_t s) {
         const int pair_grid = 4 * device_sms();
         launch_col_pairs(false, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, nullptr, nullptr,
-                         pairs_cap_, stats_, pair_grid, s);
+                         pairs_cap_, stats_, queue_, pair_grid, s);
         exclusive_scan(I.colcnt, I.col_off, ncol_, I.scan_tmp, s);
         launch_col_pairs(true, dsegs_, nseg, ntris_, I.xybox, I.pair_off, I.colcnt, I.col_off,
-                         I.col_list, pairs_cap_, stats_, pair_grid, s);
+                         I.col_list, pairs_cap_, stats_, queue_, pair_grid, s);
         launch_occ_filter(opts_.predicates, dsegs_, nseg, nrow_, I.soup, I.otri, I.col_off,
                           I.col_list, occ, occ_xyz, I.flagged, pairs_cap_, stats_, s);
         launch_occ_exact(opts_.predicates, dsegs_, nseg, I.soup, I.col_off, I.col_list, I.flagged,
@@ -671,25 +687,18 @@ void Batch::run_impl(bool sizing) {
     auto walk = [&]() {
         launch_brick_walk(dsegs_, nseg, nwalk_, I.soup, I.tinfo, I.tlo, I.thi, I.bin_off, I.bin_list,
                           I.bin_info, I.bin_ball, I.bin_reach, I.large_list, I.cand_cnt, I.cand_rng, I.cand,
-                          I.cand_c, cand_cap_, I.brick_emax, stats_, eight, ss);
+                          I.cand_c, cand_cap_, I.brick_emax, stats_, queue_, eight, ss);
     };
     if (cand_cap_ < 0) plan_cands(entries_of(I.cands, cand_bytes()));
-    // reads the walk's total back; lists that did not fit are sized (with an eighth to
-    // spare, for points that move) and walked again
+    // reads the walk's total back; lists that did not fit are sized and walked again
     auto prep_size = [&]() {
         unsigned long long C = 0;
         CMG_CUDA(cudaMemcpyAsync(&C, &stats_->candidates, sizeof(C), cudaMemcpyDeviceToHost, ss));
         CMG_CUDA(cudaStreamSynchronize(ss));
         if (static_cast<int64_t>(C) <= cand_cap_) return;
-        const size_t n = static_cast<size_t>(C + C / 8);
-        I.cands.clear_need();
-        plan_cands(n);
-        if (I.cands.overflowed()) {
-            cand_cap_ = -1;  // until the allocation has succeeded
-            I.cands.reserve(I.cands.need());
-            plan_cands(n);
-        }
+        size_cands(static_cast<int64_t>(C));
         CMG_CUDA(cudaMemsetAsync(&stats_->candidates, 0, sizeof(C), ss));
+        CMG_CUDA(cudaMemsetAsync(queue_, 0, sizeof(*queue_), ss));  // (closed by the first walk)
         walk();
     };
     auto prep_tail = [&]() {
@@ -831,10 +840,10 @@ void Batch::download(std::vector<HostResult>& out, RunInfo* info) {
             if (info) *info = info_of(s);
             return;
         }
-        unchecked_ = false;
-        pairs_cap_ = cand_cap_ = -1;
-        resize_ = true;  // the sizing run, whatever the arenas hold
-        sized_run();
+        // (both totals are counted whether or not the lists fit)
+        if (static_cast<int64_t>(s.pairs) > pairs_cap_) size_pairs(static_cast<int64_t>(s.pairs));
+        if (static_cast<int64_t>(s.candidates) > cand_cap_) size_cands(static_cast<int64_t>(s.candidates));
+        run_impl(false);
         finish_xyz();
     }
 }

@@ -255,6 +255,8 @@ private:
     RunInfo info_of(const Stats& s) const;
     void plan_pairs(size_t n);
     void plan_cands(size_t n);
+    void size_pairs(int64_t n);
+    void size_cands(int64_t n);
     bool near_list() const;
     size_t cand_bytes() const;
 };

@@ -18,8 +18,12 @@ int device_sms();
 // layout.cu: a grid of nx * ny * nz cells from idx = (k*ny + j)*nx + i to (i*ny + j)*nz + k.
 void launch_to_xyz(const float* in, int nx, int ny, int nz, float* out, cudaStream_t st);
 
+// A work queue's count beyond every item: an evaluation that starts there does nothing.
+constexpr unsigned long long kQueueClosed = 1ull << 40;
+
 // occupancy.cu. cap: bucket entries that fit; with more, the buckets and what follows from
-// them are left out and stats->pairs tells the caller. otri: three float4 per triangle, the
+// them are left out, the evaluation's queue (if any) is closed and stats->pairs tells the
+// caller. otri: three float4 per triangle, the
 // column test's FP32 records; nullptr: every entry is decided in FP64. xyz: one mesh's whole
 // grid, its cells in [x][y][z] order.
 void launch_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts,
@@ -27,7 +31,7 @@ void launch_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double*
                      cudaStream_t st);
 void launch_col_pairs(bool fill, const MeshSeg* segs, int nseg, int64_t ntris, const int4* xybox,
                       const int64_t* pair_off, int* colcnt, const int64_t* col_off, int* col_list,
-                      int64_t cap, Stats* stats, int grid, cudaStream_t st);
+                      int64_t cap, Stats* stats, unsigned long long* queue, int grid, cudaStream_t st);
 void launch_occ_filter(int mode, const MeshSeg* segs, int nseg, int64_t nrows, const double* soup,
                        const float4* otri, const int64_t* col_off, const int* col_list, uint8_t* occ,
                        bool xyz, int64_t* flagged, int64_t cap, Stats* stats, cudaStream_t st);
@@ -56,7 +60,8 @@ void launch_seg_finish(MeshSeg* segs, int nseg, const int* large_cnt, const unsi
                        cudaStream_t st);
 // Candidate lists: per brick its count, and its range [cand_rng[2 b], cand_rng[2 b + 1]) in
 // cand (cap entries), in no particular order; stats->candidates (zero before) gets the
-// total. A total above cap leaves lists out: the caller sizes cand and walks again.
+// total. A total above cap leaves lists out and closes the evaluation's queue: the caller
+// sizes cand and walks again.
 // cand_c (null: not wanted): per candidate, its centroid from the brick's centre and radius.
 // eight: whether some mesh has eight-warp bricks.
 void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double* soup,
@@ -64,7 +69,8 @@ void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double
                        const int64_t* bin_off, const int* bin_list, const float4* bin_info,
                        const float4* bin_ball, const float* bin_reach, const int* large_list,
                        int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
-                       float* brick_emax, Stats* stats, bool eight, cudaStream_t st);
+                       float* brick_emax, Stats* stats, unsigned long long* queue, bool eight,
+                       cudaStream_t st);
 // Warps per brick the walk uses for a mesh of a batch of nbricks in all (walk_warps when it
 // is 1, 2 or 4, else by the counts), and its CTAs for that.
 int brick_walk_warps(int64_t nbricks, int64_t mesh_bricks, int64_t mesh_tris, int walk_warps);

@@ -195,9 +195,10 @@ extern "C" cmg_status cmg_gpu_occupancy_static(const double* d_points, int64_t n
 
         const int grid = 4 * device_sms();
         CMG_CUDA(cudaMemsetAsync(colcnt, 0, sizeof(int) * ncol, st));
-        launch_col_pairs(false, segs, 1, T, xybox, pair_off, colcnt, nullptr, nullptr, P, stats, grid, st);
+        launch_col_pairs(false, segs, 1, T, xybox, pair_off, colcnt, nullptr, nullptr, P, stats, nullptr, grid, st);
         exclusive_scan(colcnt, col_off, ncol, scan_tmp, st);
-        launch_col_pairs(true, segs, 1, T, xybox, pair_off, colcnt, col_off, col_list, P, stats, grid, st);
+        launch_col_pairs(true, segs, 1, T, xybox, pair_off, colcnt, col_off, col_list, P, stats, nullptr, grid,
+                         st);
         launch_occ_filter(predicates, segs, 1, nrows, soup, nullptr, col_off, col_list, d_occupancy,
                           false, flagged, P, stats, st);
         launch_occ_exact(predicates, segs, 1, soup, col_off, col_list, flagged, hs, hv,

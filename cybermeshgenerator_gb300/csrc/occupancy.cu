@@ -252,9 +252,13 @@ template <bool FILL>
 __global__ void k_col_pairs(const MeshSeg* __restrict__ segs, int nseg, int64_t ntris,
                             const int4* __restrict__ xybox, const int64_t* __restrict__ pair_off,
                             int* __restrict__ colcnt, const int64_t* __restrict__ col_off,
-                            int* __restrict__ col_list, int64_t cap, Stats* __restrict__ st) {
+                            int* __restrict__ col_list, int64_t cap, Stats* __restrict__ st,
+                            unsigned long long* __restrict__ queue) {
     const int64_t npairs = pair_off[ntris];
-    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) st->pairs = static_cast<unsigned long long>(npairs);
+    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) {
+        st->pairs = static_cast<unsigned long long>(npairs);
+        if (npairs > cap && queue) atomicMax(queue, kQueueClosed);
+    }
     if (npairs > cap) return;
     const int lane = threadIdx.x & 31;
     for (int64_t p0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); p0 < npairs;
@@ -527,14 +531,14 @@ void launch_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double*
 
 void launch_col_pairs(bool fill, const MeshSeg* segs, int nseg, int64_t ntris, const int4* xybox,
                       const int64_t* pair_off, int* colcnt, const int64_t* col_off, int* col_list,
-                      int64_t cap, Stats* stats, int grid, cudaStream_t st) {
+                      int64_t cap, Stats* stats, unsigned long long* queue, int grid, cudaStream_t st) {
     if (ntris == 0) return;
     if (fill)
         k_col_pairs<true><<<grid, 256, 0, st>>>(segs, nseg, ntris, xybox, pair_off, colcnt, col_off,
-                                                col_list, cap, stats);
+                                                col_list, cap, stats, queue);
     else
         k_col_pairs<false><<<grid, 256, 0, st>>>(segs, nseg, ntris, xybox, pair_off, colcnt, col_off,
-                                                 col_list, cap, stats);
+                                                 col_list, cap, stats, queue);
     CMG_LAUNCH();
 }
 

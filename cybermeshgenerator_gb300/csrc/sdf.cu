@@ -534,7 +534,7 @@ __device__ __forceinline__ void brick_walk(const MeshSeg& turn, const MeshSeg* _
            const float* __restrict__ bin_reach, const int* __restrict__ large_list,
            int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
            float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
-           Stats* __restrict__ st) {
+           Stats* __restrict__ st, unsigned long long* __restrict__ queue) {
     constexpr int kWarps = kWalkThreads / 32;
     __shared__ float4 s_q[kWarps];
     __shared__ int s_c[kWarps];
@@ -735,7 +735,10 @@ __device__ __forceinline__ void brick_walk(const MeshSeg& turn, const MeshSeg* _
     }
     brick_sync();
     int64_t at = s_off[first];
-    if (at + total > cap) return;  // uniform over the brick: the lists are sized and walked again
+    if (at + total > cap) {  // uniform over the brick: the lists are sized and walked again
+        if (sub == 0 && lane == 0) atomicMax(queue, kQueueClosed);
+        return;
+    }
     at += before;
     float bemax = 0.f;
     // a list entry: the triangle and, for the warp-per-sub-brick evaluation, its centroid from
@@ -788,12 +791,12 @@ k_brick_walk(const MeshSeg* __restrict__ segs, int nseg,
              const float* __restrict__ bin_reach, const int* __restrict__ large_list,
              int* __restrict__ cand_cnt, int64_t* __restrict__ cand_rng, int* __restrict__ cand,
              float4* __restrict__ cand_c, int64_t cap, float* __restrict__ brick_emax,
-             Stats* __restrict__ st) {
+             Stats* __restrict__ st, unsigned long long* __restrict__ queue) {
     const MeshSeg& turn = segs[find_seg<&MeshSeg::walk_begin>(segs, nseg, blockIdx.x)];
     if (EIGHT && segs[turn.walk_seg].walk_warps == 8)
-        brick_walk<8>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st);
+        brick_walk<8>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st, queue);
     else
-        brick_walk<4>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st);
+        brick_walk<4>(turn, segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list, cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, st, queue);
 }
 
 // ------------------------------------------------------------------ evaluation
@@ -1287,12 +1290,13 @@ void launch_brick_walk(const MeshSeg* segs, int nseg, int64_t ctas, const double
                        const int64_t* bin_off, const int* bin_list, const float4* bin_info,
                        const float4* bin_ball, const float* bin_reach, const int* large_list,
                        int* cand_cnt, int64_t* cand_rng, int* cand, float4* cand_c, int64_t cap,
-                       float* brick_emax, Stats* stats, bool eight, cudaStream_t st) {
+                       float* brick_emax, Stats* stats, unsigned long long* queue, bool eight,
+                       cudaStream_t st) {
     if (ctas == 0) return;
     auto go = [&](auto kernel) {
         kernel<<<static_cast<unsigned>(ctas), kWalkThreads, 0, st>>>(
             segs, nseg, soup, tinfo, tlo, thi, bin_off, bin_list, bin_info, bin_ball, bin_reach, large_list,
-            cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, stats);
+            cand_cnt, cand_rng, cand, cand_c, cap, brick_emax, stats, queue);
     };
     if (eight) go(k_brick_walk<true>);
     else go(k_brick_walk<false>);

@@ -1,7 +1,13 @@
 """Single calls run into what the device's shared workspace holds. A call like the one before
-it fits, whatever its lists' entries take: it enqueues what a batch's run enqueues, once."""
+it fits, whatever its lists' entries take: it enqueues what a batch's run enqueues, once. A call
+whose lists are longer is run again with the lengths it has found, so twice in all."""
+import os
+import subprocess
+import sys
+
 import pytest
 
+from conftest import ROOT
 from cybermeshgenerator_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +35,48 @@ def test_a_repeated_call_runs_once(cm, size):
             return cm.voxelize_ex(plc, resolution=size[1], pad=1, outputs=3, **kw)
         call()
         assert launches(call) == once[name] and launches(call) == once[name], name
+
+
+GROWING = r"""
+import sys
+import numpy as np
+import cybermeshgenerator_gb300 as cm
+from cybermeshgenerator_gb300 import workloads as W
+kw = eval(sys.argv[1])
+
+def launches(f):
+    n = cm.gpu_launches()
+    r = f()
+    return cm.gpu_launches() - n, r
+
+def call(plc, res):
+    return cm.voxelize_ex(plc, resolution=res, pad=1, outputs=3, **kw)
+
+small = cm.PLC.from_arrays(*W.jittered_icosphere(1, 0.03, seed=1))
+for res in (24, 24):
+    n, _ = launches(lambda: call(small, res))
+# (triangles, cells): more of both, more pairs only, more candidates only
+for subdiv, res in ((3, 40), (4, 40), (1, 200), (4, 60), (5, 100)):
+    plc = cm.PLC.from_arrays(*W.jittered_icosphere(subdiv, 0.03, seed=subdiv))
+    b = cm.Batch([plc], [res], [1], outputs=3, **kw)
+    b.run().sync()
+    once, _ = launches(lambda: b.run().sync())
+    want = b.result(0)
+    first, got = launches(lambda: call(plc, res))
+    again, same = launches(lambda: call(plc, res))
+    print(kw, subdiv, res, once, first, again)
+    # (one more: an almost empty workspace is sized on the way, with a second walk)
+    assert first in (once, once + 1, 2 * once) and again == once
+    for r in (got, same):
+        assert np.array_equal(r.occupancy, want.occupancy)
+        assert np.array_equal(r.sdf32.view(np.uint32), want.sdf32.view(np.uint32))
+        assert r.stats["candidates"] == want.stats["candidates"] and r.stats["bucket_entries"] == want.stats["bucket_entries"]
+assert first == 2 * once  # the largest had not been seen
+"""
+
+
+@pytest.mark.parametrize("name", sorted(OPTIONS))
+def test_a_growing_call_runs_twice(cm, name):
+    r = subprocess.run([sys.executable, "-c", GROWING, repr(OPTIONS[name])], cwd=ROOT, text=True,
+                       capture_output=True, timeout=300, env=dict(os.environ))
+    assert r.returncode == 0, r.stdout + r.stderr
