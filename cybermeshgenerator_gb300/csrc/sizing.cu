@@ -1008,7 +1008,25 @@ __global__ void __launch_bounds__(kThreads) k_query_keys(Field F, const double* 
     const uint32_t k = static_cast<uint32_t>(
         cell < 0 ? static_cast<int64_t>(F.tg.n[0]) * F.tg.n[1] * F.tg.n[2] : cell);
     key[i] = k;
-    val[i] = count ? static_cast<uint32_t>(atomicAdd(&count[k], 1)) : static_cast<uint32_t>(i);
+    if (!count) {
+        val[i] = static_cast<uint32_t>(i);
+        return;
+    }
+    // where neighbours share a cell, one atomic per cell and warp: queries that crowd into a few
+    // cells would queue up (1M in one cell of 25k: the call 1004 us with an atomic each, 344 so)
+    const int lane = threadIdx.x & 31;
+    const unsigned live = __activemask();
+    const uint32_t next = __shfl_down_sync(live, k, 1);
+    if (!__any_sync(live, lane < 31 && next == k)) {
+        val[i] = static_cast<uint32_t>(atomicAdd(&count[k], 1));
+        return;
+    }
+    const unsigned grp = __match_any_sync(live, k);
+    const int lead = __ffs(grp) - 1;
+    int at = 0;
+    if (lane == lead) at = atomicAdd(&count[k], __popc(grp));
+    at = __shfl_sync(grp, at, lead);
+    val[i] = static_cast<uint32_t>(at + __popc(grp & ((1u << lane) - 1u)));
 }
 
 // The counting sort's order (within a cell by the atomics' order, which no result shows).
@@ -1744,8 +1762,8 @@ void sizing_eval_device(SizingField* S, const double* q, int64_t n, double* out,
     // A counting sort passes once over the cells and twice over the queries, the radix sort
     // up to four times over the queries and never over the cells: for 1M queries in 85k cells
     // 620 us against 692 (the call), for 1000 in 85k 257 against 293. With hundreds of queries
-    // a cell its atomics queue up (1M in 3k cells: 565 us against 502), and far more cells than
-    // queries are read in vain.
+    // in every cell its atomics queue up (1M in 3k cells, one atomic per query: 565 us against
+    // 502), and far more cells than queries are read in vain.
     if (64 * tcells >= n && tcells <= 2 * n + (int64_t(1) << 20)) {
         uint32_t* key = reinterpret_cast<uint32_t*>(S->sort_tmp);
         uint32_t* place = key + n;
