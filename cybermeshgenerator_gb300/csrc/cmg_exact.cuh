@@ -517,11 +517,9 @@ static __device__ __noinline__ int orient3d_homogeneous(const d3& a, const d3& b
     return sum(nu, u, nv, v, out);
 }
 
-// Exact sign of orient3d(a, b, c, d).
-static __device__ __noinline__ int orient3d_sign(const d3& a, const d3& b, const d3& c, const d3& d) {
+// Exact sign of orient3d(a, b, c, d) where integers do not hold it.
+static __device__ __noinline__ int orient3d_expanded(const d3& a, const d3& b, const d3& c, const d3& d) {
     {
-        int sg;
-        if (orient3d_int(a, b, c, d, &sg) || orient3d_wide(a, b, c, d, &sg)) return sg;
         double det;
         if (orient3d_certified(a, b, c, d, &det)) return det > 0.0 ? 1 : (det < 0.0 ? -1 : 0);
     }
@@ -546,6 +544,13 @@ static __device__ __noinline__ int orient3d_sign(const d3& a, const d3& b, const
     double e[96];
     int n = orient3d_homogeneous(a, b, c, d, e);
     return sign_of(n, e);
+}
+
+// Exact sign of orient3d(a, b, c, d).
+static __device__ __noinline__ int orient3d_sign(const d3& a, const d3& b, const d3& c, const d3& d) {
+    int sg;
+    if (orient3d_int(a, b, c, d, &sg) || orient3d_wide(a, b, c, d, &sg)) return sg;
+    return orient3d_expanded(a, b, c, d);
 }
 
 // acc += s * w * x (w a short expansion, x up to 96 components); acc holds cap

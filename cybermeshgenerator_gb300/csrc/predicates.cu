@@ -631,8 +631,9 @@ __global__ void __launch_bounds__(kThreads) k_pred_fp64(Soa s, Seg L,
     }
 }
 
-// The queries left: wide integers (near-ties span some 70 bits), then an FP64 evaluation in
-// which no operation rounded, then expansions (counted).
+// The queries left, which the FP64 pass has tried as integers: wide integers (near-ties span
+// some 70 bits), then an FP64 evaluation in which no operation rounded, then expansions
+// (counted).
 template <int NPT>
 __global__ void __launch_bounds__(64) k_pred_exact(Soa s, const int64_t* __restrict__ in,
                                                    const unsigned long long* __restrict__ nin,
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(64) k_pred_exact(Soa s, const int64_t* __restr
         int sg;
         if (NPT == 4) {
             if (!exact::orient3d_wide(a, b, c, d, &sg)) {
-                sg = exact::orient3d_sign(a, b, c, d);
+                sg = exact::orient3d_expanded(a, b, c, d);
                 atomicAdd(nexp, 1ull);
             }
         } else {
