@@ -223,24 +223,29 @@ __device__ __forceinline__ bool one_side(const int4& p, const int4& q, const int
 
 constexpr int kPairThreads = 128;
 
-// One thread per cell entry x of n: the pairs with the entries x + 1 .. x + n / 2, round the
-// cell's end (each pair once, and the lanes of a cell run equally long). Pairs whose boxes
-// meet wait in the warp's list until a full warp examines them; what FP32 leaves goes to
-// `open`, nopen of them (more than cap are counted but not stored).
+// Pairs left by the middle phase that are listed at once (8 GB); a search that leaves more
+// takes the cell entries in parts.
+constexpr unsigned long long kOpenMost = 1ull << 30;
+
+// One thread per cell entry of [first, last), x of the n in its cell: the pairs with the
+// entries x + 1 .. x + n / 2, round the cell's end (each pair once, and the lanes of a cell run
+// equally long). Pairs whose boxes meet wait in the warp's list until a full warp examines
+// them; what FP32 leaves goes to `open`, nopen of them (more than cap are counted but not
+// stored).
 //
 // One thread per entry testing boxes, cells and orientations in FP64 took 3.02 ms for 512k
 // facets (the FP64 pipe 78 % busy, 13 lanes in use): now 80 us, and 40 us for the pairs left.
 __global__ void __launch_bounds__(kPairThreads)
-k_det_pairs(int64_t nentries, bool certify, const int2* __restrict__ list, const int64_t* __restrict__ celloff,
+k_det_pairs(int64_t first, int64_t last, bool certify, const int2* __restrict__ list, const int64_t* __restrict__ celloff,
             const StepBox* __restrict__ fbox, const int* __restrict__ tris, const int4* __restrict__ fpts,
             int2* __restrict__ open, unsigned long long* __restrict__ nopen, unsigned long long cap) {
     __shared__ int2 s_q[kPairThreads / 32][64];
     int2* queue = s_q[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int64_t e = static_cast<int64_t>(blockIdx.x) * kPairThreads + threadIdx.x;
+    const int64_t e = first + static_cast<int64_t>(blockIdx.x) * kPairThreads + threadIdx.x;
     int2 me = make_int2(0, 0);
     int64_t begin = 0, n = 0;
-    if (e < nentries) {
+    if (e < last) {
         me = list[e];
         begin = celloff[me.y & 0xffffff];
         n = celloff[(me.y & 0xffffff) + 1] - begin;
@@ -616,7 +621,8 @@ void self_intersections(const double* h_pts, int64_t npts, const int* h_fidx, in
     CMG_LAUNCH();
     unsigned long long cap = 1 << 16;
     unsigned long long open_cap = std::max<unsigned long long>(1 << 16, static_cast<unsigned long long>(ntris));
-    for (int attempt = 0; attempt < 3; ++attempt) {  // (once more for each list that was too short)
+    int64_t part = nent;  // cell entries searched at a time
+    for (int attempt = 0; attempt < 64; ++attempt) {  // (once more for each list that was too short)
         long long* out;
         int2* open;
         unsigned long long* counts;  // pairs left by the middle phase, crossing pairs
@@ -627,22 +633,35 @@ void self_intersections(const double* h_pts, int64_t npts, const int* h_fidx, in
             counts = A_out.take<unsigned long long>(2);
         });
         CMG_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), st));
-        if (nent > 0) {
-            k_det_pairs<<<static_cast<unsigned>((nent + kPairThreads - 1) / kPairThreads), kPairThreads, 0, st>>>(
-                nent, G.fx > 0.0, list, celloff, fbox, tris, fpts, open, counts, open_cap);
+        unsigned long long h_counts[2] = {0, 0};
+        for (int64_t e0 = 0; e0 < nent && h_counts[0] <= open_cap; e0 += part) {
+            const int64_t e1 = std::min(nent, e0 + part);
+            if (e0 > 0) CMG_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned long long), st));
+            k_det_pairs<<<static_cast<unsigned>((e1 - e0 + kPairThreads - 1) / kPairThreads), kPairThreads, 0, st>>>(
+                e0, e1, G.fx > 0.0, list, celloff, fbox, tris, fpts, open, counts, open_cap);
             CMG_LAUNCH();
             k_det_cross<<<4 * device_sms(), 64, 0, st>>>(open, counts, open_cap, tris, d_pts, out, counts + 1,
                                                          cap);
             CMG_LAUNCH();
+            if (e1 < nent) {
+                CMG_CUDA(cudaMemcpyAsync(h_counts, counts, sizeof(h_counts), cudaMemcpyDeviceToHost, st));
+                CMG_CUDA(cudaStreamSynchronize(st));
+            }
         }
         CMG_CUDA(cudaEventRecord(ev[1], st));
-        unsigned long long h_counts[2] = {0, 0};
         CMG_CUDA(cudaMemcpyAsync(h_counts, counts, sizeof(h_counts), cudaMemcpyDeviceToHost, st));
         CMG_CUDA(cudaStreamSynchronize(st));
         CMG_CUDA(cudaEventElapsedTime(&g_last_ms, ev[0], ev[1]));
         const unsigned long long found = h_counts[1];
         if (h_counts[0] > open_cap) {
-            open_cap = h_counts[0];
+            if (h_counts[0] <= kOpenMost || part <= kPairThreads) {
+                open_cap = h_counts[0];
+            } else {
+                // fewer entries at a time, by the pairs they left, with a half to spare
+                open_cap = std::max(open_cap, kOpenMost);
+                const double share = 0.5 * static_cast<double>(open_cap) / static_cast<double>(h_counts[0]);
+                part = std::max<int64_t>(kPairThreads, static_cast<int64_t>(share * static_cast<double>(part)));
+            }
             continue;
         }
         if (found <= cap) {
