@@ -294,16 +294,16 @@ def _to_xyz(flat: np.ndarray, dims) -> np.ndarray:
     return flat.reshape((nz, ny, nx)).transpose(2, 1, 0).copy()
 
 
-#: voxelize()'s grids up to this size are copied out of the call's page-locked block (a block
-#: is 64 KiB at least and may be 1 MiB larger than the grid; the copy takes 5 us)
-_COPY_BYTES = 128 << 10
+#: voxelize()'s grids up to this size are copied out of the call's page-locked block (which is
+#: 64 KiB at least; a copy takes 1 us per 10 KB, which a call of 70 us and more can bear here)
+_COPY_BYTES = 16 << 10
 #: page-locked memory that living grids of voxelize() may hold; those beyond it are copies
 _KEEP_BYTES = 4 << 30
 
 
 def voxelize(plc: PLC, resolution: int = 64, mode="occupancy", pad: int = 1) -> VoxelGrid:
     """Voxelize a PLC (reference semantics: resolution cells on the longest axis,
-    pad margin cells; "occupancy"/0 -> uint8, "sdf"/1 -> float32). A grid above 128 KiB
+    pad margin cells; "occupancy"/0 -> uint8, "sdf"/1 -> float32). A grid above 16 KiB
     views the page-locked block that the device wrote it to, which goes back to the pool
     of such blocks when the array goes; living grids hold up to 4 GiB of locked memory
     this way, and further ones are copies in the caller's own memory."""

@@ -55,6 +55,8 @@ cudaError_t device_alloc_raw(void** p, size_t bytes) {
 // ------------------------------------------------------------------ host block pool
 namespace {
 
+constexpr size_t kBlockUnit = size_t{64} << 10;  // blocks are multiples of it
+
 struct HostPool {
     static constexpr size_t kCachedCap = size_t{4} << 30;  // idle pinned bytes kept
     std::mutex mu;
@@ -74,7 +76,7 @@ void* host_block_acquire(size_t bytes, size_t* cap, bool* pinned) {
     {
         std::lock_guard<std::mutex> lk(P.mu);
         auto it = P.idle.lower_bound(bytes);
-        if (it != P.idle.end() && it->first <= 2 * bytes + (size_t{1} << 20)) {
+        if (it != P.idle.end() && it->first <= 2 * bytes + kBlockUnit) {
             void* p = it->second;
             *cap = it->first;
             *pinned = true;
@@ -83,7 +85,7 @@ void* host_block_acquire(size_t bytes, size_t* cap, bool* pinned) {
             return p;
         }
     }
-    const size_t c = (bytes + 65535) & ~size_t{65535};
+    const size_t c = (bytes + kBlockUnit - 1) / kBlockUnit * kBlockUnit;
     void* p = nullptr;
     if (cudaHostAlloc(&p, c, cudaHostAllocDefault) == cudaSuccess && p) {
         *cap = c;

@@ -99,7 +99,7 @@ cmg_status cmg_plc_voxelize_xyz(const cmg_plc*, int resolution, int mode, int pa
                                 cmg_voxels** out, char* errbuf, size_t errbuf_len);
 
 /* A handle's arrays lie in page-locked blocks of a pool that all calls share; a block may be
- * up to twice the array's size and 1 MiB larger. For a caller that would leave the arrays
+ * up to twice the array's size and 64 KiB larger. For a caller that would leave the arrays
  * where they are beyond its next calls: 1 when the process then keeps `limit` bytes or less
  * this way (the handle's blocks count until cmg_voxels_destroy), else 0: copy what is kept
  * and destroy the handle. Blocks that are not page-locked do not count. Thread-safe but for

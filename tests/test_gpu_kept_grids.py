@@ -28,9 +28,31 @@ def limit(cm, monkeypatch):
 
 def test_small_grids_are_the_callers_own(cm):
     plc = cm.PLC.from_arrays(*W.jittered_icosphere(1, 0.02, seed=1))
-    held = [cm.voxelize(plc, 14 + k % 16, mode, 1).grid for k in range(64) for mode in ("sdf", "occupancy")]
+    held = [cm.voxelize(plc, 4 + k % 10, mode, 1).grid for k in range(64) for mode in ("sdf", "occupancy")]
     for g in held:
-        assert g.nbytes <= 128 << 10 and g.flags.owndata and g.base is None
+        assert g.nbytes <= 16 << 10 and g.flags.owndata and g.base is None
+
+
+def test_a_block_is_no_larger_than_twice_its_grid_and_64_KiB(cm):
+    """Small grids after large ones, kept: what they lock by the library's own count."""
+    from cybermeshgenerator_gb300 import _lib
+    L = _lib.load()
+    gc.collect()
+    big = cm.PLC.from_arrays(*W.jittered_icosphere(2, 0.02, seed=5))
+    for r in (40, 90, 60, 30):
+        cm.voxelize(big, r, "sdf", 1)  # idle blocks of many sizes
+    err = ctypes.create_string_buffer(256)
+    held, room = [], 0
+    for r in range(12, 40):
+        out = ctypes.c_void_p()
+        assert L.cmg_plc_voxelize_xyz(big._handle, r, 1, 1, ctypes.byref(out), err, 256) == 0
+        dims = [ctypes.c_int() for _ in range(3)]
+        L.cmg_voxels_dims(out.value, *(ctypes.byref(d) for d in dims))
+        room += 2 * 4 * int(np.prod([d.value for d in dims])) + (64 << 10)
+        assert L.cmg_voxels_keep(out.value, room) == 1, r
+        held.append(out.value)
+    for h in held:
+        L.cmg_voxels_destroy(h)
 
 
 def test_kept_grids_hold_a_bounded_amount(cm, limit):
@@ -40,8 +62,8 @@ def test_kept_grids_hold_a_bounded_amount(cm, limit):
     limit(8 * size)
     held = [cm.voxelize(plc, 70, "sdf", 1).grid for _ in range(24)]
     n = sum(_in_place(g) for g in held)
-    # a block holds its grid and may be as large again and 1 MiB more
-    assert 8 * size // (2 * size + (1 << 20)) <= n <= 8
+    # a block holds its grid and may be as large again and 64 KiB more
+    assert 8 * size // (2 * size + (64 << 10)) <= n <= 8
     for g in held:
         assert g.tobytes() == want and g.flags.c_contiguous and g.flags.writeable
     held[0][...] = 0
