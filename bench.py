@@ -285,7 +285,7 @@ def cpu_baselines(pts, tris, dims_grid, seconds):
 
 def tunables(args):
     """Options of the SDF pipeline: the library's autotuner (brick edge, queue grab,
-    walk warps, probe head, evaluation CTAs per SM, timed on this input) unless a
+    walk warps and, for plain FP64, evaluation CTAs per SM, timed on this input) unless a
     brick edge or a tunable is given on the command line or --no-autotune is set."""
     fixed = {k: v for k, v in (("brick", args.brick), ("walk_warps", args.walk_warps),
                                 ("probe", args.probe), ("ctas", args.ctas)) if v}

@@ -303,8 +303,8 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // at the origin (its second-order part |p|^2 - (n . p)^2 is at most r^2). n = 0 (a
 // degenerate triangle) leaves the ball test. Rounding: every term is formed from c, q, n and
 // the box with relative errors that sum to less than 40u (|c|^2 + |q|^2 + r^2), the
-// normal's own error nerr to less than 6 nerr (|c|^2 + r^2); `mul` and `add` widen both
-// sides by more. A comparison with a NaN keeps the triangle.
+// normal's own error nerr to less than 6 nerr (|c|^2 + r^2); `add` and the tests' own part of
+// |c|^2 widen the right side by more. A comparison with a NaN keeps the triangle.
 struct BoxTest {
     float qx, qy, qz, q2;
     float hx, hy, hz, r2;

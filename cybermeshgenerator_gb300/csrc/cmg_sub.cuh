@@ -42,9 +42,10 @@ __device__ __forceinline__ float span_centre(int x0, int x1, float h) {
 }
 // What the ends of FP32's range take from a distance: below 1e-38 a square is rounded to
 // multiples of 1.4e-45 (its root moves by up to 1.1e-19), and the reciprocal of a squared
-// edge below 3e-39 is infinite (a nearest point moves along an edge of up to 6e-20). Every
-// bound of an FP32 distance holds this much besides its relative part, so that meshes of
-// that size keep all their candidates; at 1e-6 and above it rounds away.
+// edge below 3e-39 is infinite (a nearest point moves along an edge of up to 6e-20). The
+// bounds of the candidate walk and of the warp-per-sub-brick evaluation hold this much besides
+// their relative parts, so that meshes of that size keep all their candidates; at 1e-6 and
+// above it rounds away.
 constexpr float kTinyDist = 2e-19f;
 // Position error of FP32 centroids without their lo parts, over a mesh of that scale.
 __device__ __forceinline__ float list_tol(float scale) { return fmaf(8.f * 5.9604645e-8f, scale, kTinyDist); }

@@ -7,7 +7,7 @@
 //   1. probe: over the head of the brick list, the lanes' nearest triangles by
 //      bounding sphere; their FP32 distances give the seed triangle, an upper bound U on
 //      the sub-brick centre's distance and a surface point q near it;
-//   2. filter: the brick list in steps of 128; the entries that the ball test around q
+//   2. filter: the brick list in steps of 192 (exact: 128); the entries that the ball test around q
 //      keeps (box_ball) go to a short list in shared memory;
 //   3. as soon as 32 of them wait, each lane loads one's record; those that the disc
 //      test keeps (box_disc) are staged in shared memory, and every cell tests them

@@ -317,9 +317,9 @@ void cmg_sdf_plan_destroy(cmg_sdf_plan*);
 typedef struct cmg_pred_stats {
     int64_t queries;
     int64_t fp64_queries;      /* not certified by the FP32 filter */
-    int64_t exact_queries;     /* resolved in exact arithmetic (an FP64 evaluation in
+    int64_t exact_queries;     /* resolved in exact arithmetic (integers, or what follows) */
+    int64_t expansion_queries; /* of which wide integers did not hold (an FP64 evaluation in
                                   which no operation rounded, or expansions) */
-    int64_t expansion_queries; /* of which needed expansion arithmetic */
     float fp32_pass_ms;        /* device time of the FP32 certification pass (CUDA events) */
     int32_t tma_reruns;        /* FP32 passes rerun with per-thread loads after a bulk-copy
                                   wait ran out (expected 0) */
@@ -334,7 +334,10 @@ typedef struct cmg_pred_stats {
  * read by the device directly where it accesses pageable host memory
  * (cudaDevAttrPageableMemoryAccess), in chunks of 2^24 queries, and otherwise copied
  * in chunks of 2^22 through two device buffer sets (the environment variable
- * CMG_HOST_STREAM=copy forces the copies). The call returns when the signs are
+ * CMG_HOST_STREAM=copy forces the copies). Device columns are copied on chip in 16-byte
+ * words: of a column that starts 8 bytes off a 16-byte boundary the value before it is read
+ * too, and of one that ends there the value after it (never beyond the 16-byte word that
+ * holds a value of the column; neither is used). The call returns when the signs are
  * written. stats may be NULL (fp32_pass_ms: summed over the chunks). No counterpart
  * in the reference beyond the scalar predicate it applies per query. */
 cmg_status cmg_orient3d_stream(const double* const* coords, int64_t n, int mode, int where,
