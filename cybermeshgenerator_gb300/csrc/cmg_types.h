@@ -79,6 +79,7 @@ struct Stats {
     unsigned long long exact_calls;        // orient3d resolved in exact arithmetic
     unsigned long long height_overflow;    // columns whose crossings overflowed shared memory
     unsigned long long candidates;         // SDF candidate (brick, triangle) pairs
+    unsigned long long thin;               // SDF: triangles without a face in their FP32 record
     unsigned long long evaluations;        // SDF (voxel, triangle) distance evaluations
     unsigned long long fp64_evaluations;   // of which in FP64
     unsigned long long band_voxels;        // mixed precision: voxels refined in FP64

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -197,6 +198,7 @@ struct Pool {
     Arena a[4];
     cudaStream_t side = nullptr;  // the second stream of a run, and its fork and join
     cudaEvent_t fork = nullptr, join = nullptr;
+    bool thin = false;  // the last call's meshes had triangles without a face: a guess for the next
 };
 Pool& pool_for_device() {
     static std::mutex mu;
@@ -508,11 +510,11 @@ void Batch::update_points_device(const double* d_pts) {
 }
 
 // A sizing pass: reads the list totals back, grows the list arenas if needed and drops the
-// captured graph when the buffers or the list lengths that it was captured with (its kernels
-// leave out longer lists) are no longer those in use.
+// captured graph when the buffers, the list lengths (its kernels leave out longer lists) or the
+// evaluation kernel that it was captured with are no longer those in use.
 void Batch::sized_run() {
     const auto plan = [&] {
-        return std::make_tuple(impl_->pairs.capacity(), impl_->cands.capacity(), pairs_cap_, cand_cap_);
+        return std::make_tuple(impl_->pairs.capacity(), impl_->cands.capacity(), pairs_cap_, cand_cap_, thin_);
     };
     const auto before = plan();
     run_impl(true);
@@ -584,6 +586,7 @@ void Batch::run() {
         plan_pairs(entries_of(impl_->pairs, kPairBytes));
         plan_cands(entries_of(impl_->cands, cand_bytes()));
         unchecked_ = true;
+        thin_ = pool_for_device().thin;
         run_impl(false);
     } else {
         sized_run();
@@ -679,7 +682,7 @@ void Batch::run_impl(bool sizing) {
         if (timed) CMG_CUDA(cudaEventRecord(ev_[4], ss));
         launch_sdf_tri_prep(dsegs_, nseg, ntris_, pts_, tris_, I.tinfo, I.tinfo_lo, I.trec,
                             opts_.brick == 16 && sub_precision(opts_) == kPrecFP64 ? I.tnorm : nullptr, I.tlo,
-                            I.thi, I.tbin, I.bincnt, I.large_cnt, I.emax_bits, ss);
+                            I.thi, I.tbin, I.bincnt, I.large_cnt, I.emax_bits, stats_, ss);
         exclusive_scan(I.bincnt, I.bin_off, nbrick_, tmp, ss);
         launch_seg_finish(dsegs_, nseg, I.large_cnt, I.emax_bits, ss);
         launch_bin_fill(ntris_, I.tbin, I.bin_off, I.bincnt, I.tinfo, I.bin_list, I.bin_info, nbrick_,
@@ -694,9 +697,12 @@ void Batch::run_impl(bool sizing) {
     if (cand_cap_ < 0) plan_cands(entries_of(I.cands, cand_bytes()));
     // reads the walk's total back; lists that did not fit are sized and walked again
     auto prep_size = [&]() {
-        unsigned long long C = 0;
-        CMG_CUDA(cudaMemcpyAsync(&C, &stats_->candidates, sizeof(C), cudaMemcpyDeviceToHost, ss));
+        unsigned long long found[2] = {0, 0};
+        static_assert(offsetof(Stats, thin) == offsetof(Stats, candidates) + sizeof(found[0]), "read together");
+        CMG_CUDA(cudaMemcpyAsync(found, &stats_->candidates, sizeof(found), cudaMemcpyDeviceToHost, ss));
         CMG_CUDA(cudaStreamSynchronize(ss));
+        const unsigned long long C = found[0];
+        thin_ = found[1] > 0;
         if (static_cast<int64_t>(C) <= cand_cap_) return;
         size_cands(static_cast<int64_t>(C));
         CMG_CUDA(cudaMemsetAsync(&stats_->candidates, 0, sizeof(C), ss));
@@ -730,7 +736,7 @@ void Batch::run_impl(bool sizing) {
                        I.tinfo_lo, I.trec, I.tnorm, I.cand_rng, I.cand, occ, sdf32_, sdf64_,
                        near_tri_, near_reg_, stats_, I.grid_eval, st);
     else if (opts_.brick == 16)
-        launch_sdf_near(sub_precision(opts_), opts_.grab, opts_.probe, dsegs_, nseg,
+        launch_sdf_near(sub_precision(opts_), thin_, opts_.grab, opts_.probe, dsegs_, nseg,
                         I.work, nwork_, queue_, I.soup, I.tinfo, I.tinfo_lo, I.trec, I.cand_rng,
                         I.cand, I.cand_c, opts_.band, occ, sdf32_, sdf64_, near_tri_, near_reg_, err_, stats_,
                         I.grid_eval, st);
@@ -836,13 +842,16 @@ void Batch::download(std::vector<HostResult>& out, RunInfo* info) {
         Stats s;
         CMG_CUDA(cudaMemcpyAsync(&s, stats_, sizeof(Stats), cudaMemcpyDeviceToHost, stream_));
         CMG_CUDA(cudaStreamSynchronize(stream_));
-        const bool fitted = static_cast<int64_t>(s.pairs) <= pairs_cap_ && static_cast<int64_t>(s.candidates) <= cand_cap_;
+        const bool fitted = static_cast<int64_t>(s.pairs) <= pairs_cap_ && static_cast<int64_t>(s.candidates) <= cand_cap_ &&
+                            (thin_ || s.thin == 0 || !near_list());
         if (!unchecked_ || fitted) {
             unchecked_ = in_flight_ = false;
+            if (pooled_ && (sdf32_ || sdf64_ || near_tri_)) pool_for_device().thin = s.thin > 0;
             if (info) *info = info_of(s);
             return;
         }
-        // (both totals are counted whether or not the lists fit)
+        // (all totals are counted whether or not the lists fit)
+        thin_ = s.thin > 0;
         if (static_cast<int64_t>(s.pairs) > pairs_cap_) size_pairs(static_cast<int64_t>(s.pairs));
         if (static_cast<int64_t>(s.candidates) > cand_cap_) size_cands(static_cast<int64_t>(s.candidates));
         run_impl(false);

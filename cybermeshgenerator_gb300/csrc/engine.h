@@ -153,8 +153,8 @@ public:
     // Uploads the meshes (host buffers) and plans the workspace. Grids must be set.
     // A transient batch borrows the device's shared workspace (at most one alive
     // per device at a time) and runs into what is there without waiting for its list
-    // lengths: they come back with the results, and a run whose lists did not fit is
-    // repeated with the right sizes. Otherwise the batch owns its memory.
+    // lengths: they come back with the results, and a run whose lists did not fit (or whose
+    // meshes need the evaluation for triangles without a face) is repeated. Otherwise the batch owns its memory.
     Batch(const std::vector<HostMesh>& meshes, const VoxOpts& opts, cudaStream_t stream,
           bool transient = false);
     ~Batch();
@@ -221,6 +221,7 @@ private:
     bool pooled_ = false;     // the arenas, second stream and events are the device pool's
     // a pooled run into whatever its arenas held: download() checks that it fitted
     bool unchecked_ = false;
+    bool thin_ = false;       // some triangle has no face in its record (Stats::thin), or may have
     bool in_flight_ = false;  // a pooled batch's inputs may still be being copied
     double* pts_ = nullptr;
     int* tris_ = nullptr;

@@ -48,7 +48,7 @@ constexpr size_t kTriRecBytes = 96;
 void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts, const int* tris,
                          float4* tinfo, float4* tinfo_lo, void* trec, float4* tnorm, float4* tlo,
                          float4* thi,
-                         int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits,
+                         int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits, Stats* stats,
                          cudaStream_t st);
 // The bins' triangles (bin_list) with their centroids and radii in that order (bin_info),
 // and per bin a ball around them (bin_ball, bin_reach).
@@ -101,9 +101,10 @@ void launch_sdf_sub(int grab, int ctas, const MeshSeg* segs, int nseg, const uin
 
 // sdf_near.cu: mixed precision and exact FP64 through the FP32 pass, a warp per
 // sub-brick. probe: head of the brick list scanned for the seed (<= 0: all of it). cand_c:
-// the candidates' centroids and radii (launch_brick_walk).
+// the candidates' centroids and radii (launch_brick_walk). thin: some triangle has no face in
+// its record (stats->thin); the results do not depend on a true that need not be.
 int sdf_near_grid(int precision);
-void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, int nseg,
+void launch_sdf_near(int precision, bool thin, int grab, int probe, const MeshSeg* segs, int nseg,
                      const uint32_t* work, int64_t nwork, unsigned long long* queue,
                      const double* soup, const float4* tinfo, const float4* tinfo_lo,
                      const void* trec, const int64_t* cand_rng, const int* cand, const float4* cand_c,

@@ -65,7 +65,8 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
                                float4* __restrict__ tnorm,
                                float4* __restrict__ tlo, float4* __restrict__ thi,
                                int64_t* __restrict__ tbin, int* __restrict__ bincnt,
-                               int* __restrict__ large_cnt, unsigned* __restrict__ emax_bits) {
+                               int* __restrict__ large_cnt, unsigned* __restrict__ emax_bits,
+                               Stats* __restrict__ st) {
     int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= ntris) return;
     const int si = find_seg<&MeshSeg::tri_begin>(segs, nseg, t);
@@ -103,6 +104,7 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
     double vx = c.x - a.x, vy = c.y - a.y, vz = c.z - a.z;
     double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
     bool degenerate = !(nx * nx + ny * ny + nz * nz > 0.0);
+    bool thin;  // without a face in its FP32 record: the reference's distance may be none (NaN)
     {
         const double lu = sqrt(ux * ux + uy * uy + uz * uz), lv = sqrt(vx * vx + vy * vy + vz * vz);
         if (tnorm) {
@@ -166,13 +168,15 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
         const double l1 = (ccx - bx) * (ccx - bx) + ccy * ccy, l2 = ccx * ccx + ccy * ccy;
         r.inv1 = l1 > 0.0 ? static_cast<float>(1.0 / l1) : 0.f;
         r.inv2 = l2 > 0.0 ? static_cast<float>(1.0 / l2) : 0.f;
-        r.ok = bx > 0.0 && ccy > 0.0 ? 1.f : 0.f;
+        thin = !(bx > 0.0 && ccy > 0.0);
+        r.ok = thin ? 0.f : 1.f;
         r.pad_[0] = r.pad_[1] = r.pad_[2] = 0.f;
         trec[t] = r;
     }
-    // degenerate (zero-area) or larger than two bricks: always considered
+    // degenerate (zero-area), thin or larger than two bricks: always considered
     const double bw = static_cast<double>(s.brick) * s.g.h;
-    const bool large = degenerate || sqrt(r2) > 2.0 * bw;
+    const bool large = degenerate || thin || sqrt(r2) > 2.0 * bw;
+    if (thin) atomicAdd(&st->thin, 1ull);
     // per segment, one set of atomics per warp: the mesh's coordinate scale max |v - K|
     // (rounded up) for the FP32 tolerances (k_seg_finish folds in the grid extent), the
     // largest radius of all its triangles (the mixed path's error bounds) and of the binned
@@ -204,7 +208,8 @@ __global__ void k_sdf_tri_prep(const MeshSeg* __restrict__ segs, int nseg, int64
     if (large) {
         tlo[t] = make_float4(__double2float_rd(fmin(a.x, fmin(b.x, c.x)) - K[0]),
                              __double2float_rd(fmin(a.y, fmin(b.y, c.y)) - K[1]),
-                             __double2float_rd(fmin(a.z, fmin(b.z, c.z)) - K[2]), 0.f);
+                             __double2float_rd(fmin(a.z, fmin(b.z, c.z)) - K[2]),
+                             degenerate || thin ? 1.f : 0.f);
         thi[t] = make_float4(__double2float_ru(fmax(a.x, fmax(b.x, c.x)) - K[0]),
                              __double2float_ru(fmax(a.y, fmax(b.y, c.y)) - K[1]),
                              __double2float_ru(fmax(a.z, fmax(b.z, c.z)) - K[2]), 0.f);
@@ -594,8 +599,11 @@ __device__ __forceinline__ void brick_walk(const MeshSeg& turn, const MeshSeg* _
     };
     // ---- 1. the bound. UL: from the large triangles; U: that or the nearest centroid's
     float UL = FLT_MAX;
-    for (int64_t e = s.large_begin + 32 * sub + lane; e < s.large_end; e += 32 * W)
-        UL = fminf(UL, large_upper(soup, large_list[e], s.g.corner, q.cx, q.cy, q.cz, tol));
+    for (int64_t e = s.large_begin + 32 * sub + lane; e < s.large_end; e += 32 * W) {
+        const int t = large_list[e];
+        if (tlo[t].w == 0.f)  // (a thin triangle's distance may be none: it bounds nothing)
+            UL = fminf(UL, large_upper(soup, t, s.g.corner, q.cx, q.cy, q.cz, tol));
+    }
     {
         float4 p = make_float4(0.f, 0.f, 0.f, UL);
         int none = INT_MAX;
@@ -1244,12 +1252,12 @@ k_count_K(const MeshSeg* __restrict__ segs, int nseg, int64_t nbricks,
 void launch_sdf_tri_prep(const MeshSeg* segs, int nseg, int64_t ntris, const double* pts, const int* tris,
                          float4* tinfo, float4* tinfo_lo, void* trec, float4* tnorm, float4* tlo,
                          float4* thi,
-                         int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits,
+                         int64_t* tbin, int* bincnt, int* large_cnt, unsigned* emax_bits, Stats* stats,
                          cudaStream_t st) {
     if (ntris == 0) return;
     k_sdf_tri_prep<<<static_cast<unsigned>((ntris + 255) / 256), 256, 0, st>>>(
         segs, nseg, ntris, pts, tris, tinfo, tinfo_lo, static_cast<TriRec*>(trec), tnorm, tlo, thi, tbin,
-        bincnt, large_cnt, emax_bits);
+        bincnt, large_cnt, emax_bits, stats);
     CMG_LAUNCH();
 }
 

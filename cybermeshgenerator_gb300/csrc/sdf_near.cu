@@ -52,6 +52,7 @@ constexpr int kSkip = 512;      // of longer lists the probe reads every other s
 constexpr float kItemCost = 1024.f;  // a sub-brick's fixed work, in list entries
 constexpr float kHeavy = 0.25f;      // lists over this part of a warp's share are shared
 constexpr unsigned kAll = 0xffffffffu;
+constexpr float kKept = -2.f;  // the distance of a near-tie pair that no threshold drops
 
 struct WarpMem {
     // staged records, their centroids (radius widened: reach_term) and ids
@@ -242,7 +243,14 @@ struct Args {
 
 // One sub-brick: by this warp alone, or (COOP) by the CTA's warps together, each over its
 // part of the list. item: sub-brick of the queue.
-template <int PREC, bool COOP>
+//
+// THIN: the meshes have triangles without a face in their records (repeated or collinear
+// corners, or thinner than a billionth). For those the reference's FP64 operations may give no
+// number (0 / 0; the triangle then counts for nothing) or one that is not the distance. So they
+// are no seeds, lower no cell's minimum and bound (nor the walk's), and every one that might be
+// nearest to a cell goes to FP64, which decides. Meshes without any, by far the most, keep the
+// kernel without it (2 % faster in mixed precision).
+template <int PREC, bool THIN, bool COOP>
 __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, WarpMem& M, Shared& S,
                                           const WarpMem* all) {
     constexpr bool EXACT = PREC == kPrecExact;
@@ -363,6 +371,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const int t = list[at];
                 TriRec r;
                 load_rec(g.trec, t, r);
+                if (THIN && !(r.ok > 0.f)) continue;
                 const float4 e = recentre(g.tinfo[t], g.tinfo_lo[t], M.mid[0], M.mid[1]);
                 const float dc = sqrt_approx(fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)));
                 const float d = sqrt_approx(dist_rec_val(r, -e.x, -e.y, -e.z));
@@ -483,7 +492,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const int pos = __popc(m & below);
                 M.rec[pos] = r;
                 M.c[pos] = make_float4(e.x, e.y, e.z, reach_term(e.w, M.mid[0].w));
-                M.t[pos] = t;
+                M.t[pos] = THIN && !(r.ok > 0.f) ? ~t : t;
             }
         }
         __syncwarp();
@@ -517,9 +526,12 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                 const float d = dist_rec_val(M.rec[k], M.pos[cell & 3] - c.x, M.pos[4 + ((cell >> 2) & 3)] - c.y,
                                              M.pos[8 + (cell >> 4)] - c.z);
                 neval += n;
-                if (in) improve(cell, d, t);
+                const bool face = !THIN || t >= 0;
+                if (in && face) improve(cell, d, t);
                 __syncwarp();
-                const unsigned m = __ballot_sync(kAll, in && d <= M.thr2[cell]);
+                float thr = M.thr2[cell];
+                if (!EXACT && !face) thr = near_thr2(key_dist(M.best[cell]), M.con.x);  // beyond the band too
+                const unsigned m = __ballot_sync(kAll, in && d <= thr);
                 if (m) {
                     if (npair + 32 > kPairs) {
                         npair = prune(M, npair);
@@ -529,7 +541,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
                             npair = 0;
                         }
                     }
-                    push(m, t, d, cell);
+                    push(m, face ? t : ~t, EXACT || face ? d : kKept, cell);
                 }
             }
         }
@@ -560,7 +572,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
     const bool fineA = okA && (EXACT || d32A <= bh + ebA);
     const bool fineB = okB && (EXACT || d32B <= bh + ebB);
     const unsigned maskA = __ballot_sync(kAll, fineA), maskB = __ballot_sync(kAll, fineB);
-    if (maskA | maskB) {
+    if ((maskA | maskB) || (THIN && !EXACT)) {
         if (!EXACT) {  // the near-ties of the band's cells only
             if (!fineA) M.thr2[lane] = -1.f;
             if (!fineB) M.thr2[32 + lane] = -1.f;
@@ -601,6 +613,22 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
         } else {
             const int t = key_tri(half ? bestB : bestA);
             int reg = 0;
+            if (THIN && !EXACT) {  // a nearer triangle without a face
+                unsigned long long d = M.d[lane + 32 * half], win = M.win[lane + 32 * half];
+                if (COOP) {
+#pragma unroll
+                    for (int k = 0; k < kWarps; ++k) {
+                        const unsigned long long d2 = all[k].d[lane + 32 * half], w2 = all[k].win[lane + 32 * half];
+                        if (d2 < d || (d2 == d && w2 < win)) { d = d2; win = w2; }
+                    }
+                }
+                const double e = __dsqrt_rn(__longlong_as_double(static_cast<long long>(d)));
+                if (e < static_cast<double>(half ? d32B : d32A) && !(g.trec[win >> 3].ok > 0.f)) {
+                    write_cell(g.o, idx, e, static_cast<int>(win >> 3), static_cast<int>(win & 7u));
+                    if (g.o.errbound) g.o.errbound[idx] = half ? ebB : ebA;
+                    continue;
+                }
+            }
             if (g.o.near_reg && t != INT_MAX) {
                 // the region of the nearest triangle: its distance again, recentred exactly
                 // as before (the same value, now with the region)
@@ -637,7 +665,7 @@ __device__ __forceinline__ void sub_brick(const Args& g, const int64_t item, War
 // pairs for FP64 by 32 pairs, whichever warp found them: with parts of 128 entries and
 // everybody's own pairs, half of a shared sub-brick's time was waiting for the last warp (63^3:
 // 0.19 -> 0.17 ms, 35^3 around 320 triangles: 0.11 -> 0.075 ms).
-template <int PREC>
+template <int PREC, bool THIN>
 __global__ void __launch_bounds__(32 * kWarps, 5)
 k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restrict__ st) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -664,7 +692,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
             break;
         }
         for (int k = 0; k < g.grab_n && item + k < g.nwork; ++k)
-            sub_brick<PREC, true>(g, item + k, M, S, all);
+            sub_brick<PREC, THIN, true>(g, item + k, M, S, all);
     }
     for (;;) {
         if (!own) {
@@ -675,7 +703,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
         own = false;
         if (item >= g.nwork) break;
         for (int k = 0; k < g.grab_n && item + k < g.nwork; ++k)
-            sub_brick<PREC, false>(g, item + k, M, S, all);
+            sub_brick<PREC, THIN, false>(g, item + k, M, S, all);
     }
     if (lane == 0) {
         if (M.evals) atomicAdd(&st->evaluations, M.evals);
@@ -688,7 +716,7 @@ k_sdf_near(const Args g, unsigned long long* __restrict__ queue, Stats* __restri
 template <int PREC>
 int near_grid() {
     int per = 0;
-    CMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sdf_near<PREC>, 32 * kWarps,
+    CMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sdf_near<PREC, false>, 32 * kWarps,
                                                            kWarps * sizeof(WarpMem)));
     return device_sms() * (per > 0 ? per : 1);
 }
@@ -699,7 +727,7 @@ int sdf_near_grid(int precision) {
     return precision == kPrecMixed ? near_grid<kPrecMixed>() : near_grid<kPrecExact>();
 }
 
-void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, int nseg,
+void launch_sdf_near(int precision, bool thin, int grab, int probe, const MeshSeg* segs, int nseg,
                      const uint32_t* work, int64_t nwork, unsigned long long* queue,
                      const double* soup, const float4* tinfo, const float4* tinfo_lo,
                      const void* trec, const int64_t* cand_rng, const int* cand, const float4* cand_c,
@@ -716,8 +744,8 @@ void launch_sdf_near(int precision, int grab, int probe, const MeshSeg* segs, in
     auto go = [&](auto kernel) {
         kernel<<<blocks, 32 * kWarps, kWarps * sizeof(WarpMem), st>>>(g, queue, stats);
     };
-    if (precision == kPrecMixed) go(k_sdf_near<kPrecMixed>);
-    else go(k_sdf_near<kPrecExact>);
+    if (precision == kPrecMixed) thin ? go(k_sdf_near<kPrecMixed, true>) : go(k_sdf_near<kPrecMixed, false>);
+    else thin ? go(k_sdf_near<kPrecExact, true>) : go(k_sdf_near<kPrecExact, false>);
     CMG_LAUNCH();
 }
 
